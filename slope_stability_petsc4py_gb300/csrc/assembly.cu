@@ -17,6 +17,7 @@
 // the reference's C layout and makes each element's data one contiguous block.
 #include <type_traits>
 
+#include "fixed.cuh"
 #include "ssp_internal.cuh"
 
 namespace ssp {
@@ -1096,53 +1097,32 @@ __global__ void fill_elastic_ds_kernel(const int8_t *__restrict__ branch, const 
 //   K_e[(a,c),(b,d)] = sum_{x,y = 1,2} c_ax c_by R_(m_ax m_by)[(k_ax, c), (k_by, d)],   R_mn = beta^T M_mn beta,
 // four terms per entry for every node pair, so the lanes of a warp do equal work.  Only the ten
 // pairs m <= n < 4 are formed from the points; since the coordinates sum to one,
-// R_m4 = sum_n R_mn and R_44 = sum_m R_m4.  FP64 operations per element: 21 n_pl (DS - D_el),
-// 30 n_pl (weighted coordinate products), 210 n_pl (moments), 2,160 (beta^T M), 2,340 (R),
-// 1,170 (the sums), 1,860 (K): about 7,500 + 260 n_pl against about 1,935 n_pl point by point,
-// fewer from five plastic points up.  Elements with fewer plastic points keep the point-by-point
-// kernel (the element lists are split by ssp_plastic_elements_split).  The result is the
-// reference's contraction (assemble_tangent_values_3d.c:135-214) regrouped: equal to rounding.
+// R_m4 = sum_n R_mn and R_44 = sum_m R_m4.  The result is the reference's contraction
+// (assemble_tangent_values_3d.c:135-214) regrouped: equal to rounding.
+//
+// Arithmetic: 58-bit fixed point on the integer pipe (fixed.cuh).  In FP64 the same stages are about
+// 7,500 + 260 n_pl multiply-adds an element, at 1.6 a clock and SM the whole time of the kernel
+// (0.92 of the FP64 rate).  In fixed point the products are 3 x (210 n_pl + 54 x 40 + 30 x 90) IMADs and
+// the sums and the K entries integer additions.  One exponent per element for each of the tangents, the
+// weights and the gradients; DS and D_el are subtracted as 60-bit integers; dD, the gradients and M are
+// brought to 57 or 58 bits by the element's largest.  The element matrix is within 2 to 6 x 10^-16 of its
+// largest entry (a model of these integers against 80-bit sums), as the FP64 form is.
+// Stage by stage, one warp per element:
+//   inputs   lane = entry, point by point: DS to integers, minus D_el, split into limbs
+//   M        lanes over 5 pairs of pairs x 6 groups of 4 entries: 3 16-byte loads for 24 IMADs
+//   T, R     lane (pair p, component c) holds three rows of M_p and forms rows (k, c) of R_p
+//   sums, K  integer additions; each K entry becomes FP64 once and is scattered to its two places
+// Bound by issue and latency at 16 warps an SM (registers and 13 KB of shared memory a warp): 3,900
+// instructions an element, 29 % of them in T and R, 24 % in K.  On 27,283 plastic elements of a
+// 100,800-element mesh 219 us by ncu where the FP64 form took 434 with its split (264 + 169 us).
 constexpr int kMaxQ = 11;
-constexpr int kMomWarps = 4;  // warps per CTA (one element per warp)
-constexpr int kMomEntries = 465;  // alpha <= beta of the 30 x 30 element matrix
-
-struct MomentWarp {
-    union {
-        struct {
-            double M[10][21];  // moments of the pairs m <= n < 4, packed upper triangle of 6 x 6
-            double v[4][3];    // grad lambda_0..3
-            union {
-                struct {
-                    double dD[kMaxQ][21];  // DS - D_el of the plastic points, packed upper triangle
-                    double ll[kMaxQ][10];  // w s lambda_m lambda_n of the plastic points, pair order
-                } in;
-                double T[10][12][6];  // (beta_(k,c)^T M_p)[t]
-            } t;
-        } a;
-        double ke[30][31];  // the element's correction, padded rows
-    } x;
-    double R[15][78];  // R over the pairs m <= n of five coordinates, packed upper triangle of 12 x 12
-    int8_t qidx[16];   // the plastic points of the element, in order
-};
-
-struct MomentTables {
-    unsigned long long k_terms[kMomEntries];  // four (R offset | coefficient code << 11) fields of 16 bits
-    uint16_t k_pos[kMomEntries];              // alpha << 5 | beta
-    uint16_t r_pos[78];                       // (k,c) << 8 | (l,d), packed upper triangle of 12 x 12
-    uint8_t s_pos[21];                        // r << 4 | c, packed upper triangle of 6 x 6
-};
 
 // packed upper-triangle index of (i, j) in an n x n symmetric matrix (row-major upper)
-__device__ __forceinline__ int sym_index(int i, int j, int n) {
-    if (i > j) {
-        const int t = i;
-        i = j;
-        j = t;
-    }
-    return i * n - (i * (i - 1)) / 2 + (j - i);
+__host__ __device__ constexpr int sym_index(int i, int j, int n) {
+    return i <= j ? i * n - (i * (i - 1)) / 2 + (j - i) : j * n - (j * (j - 1)) / 2 + (i - j);
 }
 // (i, j), i <= j, of the packed upper-triangle index p of an n x n matrix
-__device__ __forceinline__ void sym_pair(int p, int n, int &i, int &j) {
+__host__ __device__ constexpr void sym_pair(int p, int n, int &i, int &j) {
     i = 0;
     while (p >= n - i) {
         p -= n - i;
@@ -1160,7 +1140,7 @@ __device__ __forceinline__ void beta_rows(int c, int *srow, int *gcomp) {
 
 // term t (0, 1) of node a's gradient: coordinate m (0..4), coefficient 4 or -1, gradient k (0..3).
 // Nodes 4..9 are the mid-edge nodes of edges 01, 12, 02, 13, 23, 03.
-__device__ __forceinline__ void node_term(int a, int t, int &m, int &coef, int &k) {
+__host__ __device__ constexpr void node_term(int a, int t, int &m, int &coef, int &k) {
     if (a < 4) {
         m = t == 0 ? a : 4;
         coef = t == 0 ? 4 : -1;
@@ -1174,57 +1154,187 @@ __device__ __forceinline__ void node_term(int a, int t, int &m, int &coef, int &
     coef = 4;
 }
 
-__device__ void build_moment_tables(MomentTables &tb) {
-    for (int i = threadIdx.x; i < kMomEntries; i += blockDim.x) {
-        int al, be;
-        sym_pair(i, 30, al, be);
-        const int a = al / 3, c = al - 3 * a, b = be / 3, d = be - 3 * b;
-        unsigned long long packed = 0;
-        for (int x = 0; x < 2; ++x)
-            for (int y = 0; y < 2; ++y) {
-                int mx, cx, kx, my, cy, ky;
-                node_term(a, x, mx, cx, kx);
-                node_term(b, y, my, cy, ky);
-                const int cc = cx * cy;  // 16, -4 or 1
-                const unsigned code = cc == 16 ? 0u : (cc == -4 ? 1u : 2u);
-                const unsigned off = static_cast<unsigned>(sym_index(mx, my, 5) * 78 + sym_index(3 * kx + c, 3 * ky + d, 12));
-                packed |= static_cast<unsigned long long>(off | (code << 11)) << (16 * (2 * x + y));
-            }
-        tb.k_terms[i] = packed;
-        tb.k_pos[i] = static_cast<uint16_t>(al << 5 | be);
+// The K entries (alpha <= beta) grouped by node-pair type, so that a group's coefficients are constants:
+// slots of vertex-vertex 78 -> 96, vertex-edge 216 -> 224, edge-edge 171 -> 192 entries.  (al, be) of slot i,
+// or al = -1 for a slot that pads its group.
+constexpr int kKSlots = 512;
+constexpr int kVertexVertexIters = 3, kVertexEdgeIters = 7;
+__host__ __device__ constexpr void k_slot_entry(int i, int &al, int &be) {
+    al = be = -1;
+    if (i < 32 * kVertexVertexIters) {
+        if (i < 78) sym_pair(i, 12, al, be);
+    } else if (i < 32 * (kVertexVertexIters + kVertexEdgeIters)) {
+        const int j = i - 32 * kVertexVertexIters;
+        if (j < 216) {
+            al = j / 18;
+            be = 12 + j % 18;
+        }
+    } else {
+        const int j = i - 32 * (kVertexVertexIters + kVertexEdgeIters);
+        if (j < 171) {
+            sym_pair(j, 18, al, be);
+            al += 12;
+            be += 12;
+        }
     }
-    for (int i = threadIdx.x; i < 78; i += blockDim.x) {
-        int kc, ld;
-        sym_pair(i, 12, kc, ld);
-        tb.r_pos[i] = static_cast<uint16_t>(kc << 8 | ld);
-    }
-    for (int i = threadIdx.x; i < 21; i += blockDim.x) {
-        int r, c;
-        sym_pair(i, 6, r, c);
-        tb.s_pos[i] = static_cast<uint8_t>(r << 4 | c);
-    }
+}
+// the four R offsets of slot i's entry, term order (x, y), as 16-bit fields (0 for padding)
+__host__ __device__ constexpr unsigned long long k_slot_terms(int i) {
+    int al = 0, be = 0;
+    k_slot_entry(i, al, be);
+    if (al < 0) return 0ull;
+    const int a = al / 3, c = al - 3 * a, b = be / 3, d = be - 3 * b;
+    unsigned long long packed = 0;
+    for (int x = 0; x < 2; ++x)
+        for (int y = 0; y < 2; ++y) {
+            int mx = 0, cx = 0, kx = 0, my = 0, cy = 0, ky = 0;
+            node_term(a, x, mx, cx, kx);
+            node_term(b, y, my, cy, ky);
+            const unsigned off = static_cast<unsigned>(sym_index(mx, my, 5) * 78 + sym_index(3 * kx + c, 3 * ky + d, 12));
+            packed |= static_cast<unsigned long long>(off) << (16 * (2 * x + y));
+        }
+    return packed;
 }
 
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-__device__ __forceinline__ double moment_coef(unsigned code) { return code == 0u ? 16.0 : (code == 1u ? -4.0 : 1.0); }
+// Constant tables, filled by the compiler and copied to shared memory by each CTA (building them in the
+// kernel cost every CTA several microseconds).
+struct MomentTables {
+    unsigned long long k_terms[kKSlots];
+    uint16_t k_slot[900];  // slot of entry (alpha, beta), either order, times 8
+    uint32_t m_at[24];     // r 6 + c | (c 6 + r) << 16 of the packed upper triangle of 6 x 6, -1: none
+};
+constexpr MomentTables make_moment_tables() {
+    MomentTables t{};
+    for (int i = 0; i < kKSlots; ++i) {
+        t.k_terms[i] = 8 * k_slot_terms(i);  // byte offsets: every 16-bit field below 2^13
+        int al = 0, be = 0;
+        k_slot_entry(i, al, be);
+        if (al >= 0) t.k_slot[al * 30 + be] = t.k_slot[be * 30 + al] = static_cast<uint16_t>(8 * i);
+    }
+    for (int i = 0; i < 21; ++i) {
+        int r = 0, c = 0;
+        sym_pair(i, 6, r, c);
+        t.m_at[i] = static_cast<uint32_t>((r * 6 + c) | (c * 6 + r) << 16);
+    }
+    for (int i = 21; i < 24; ++i) t.m_at[i] = 0xFFFFFFFFu;
+    return t;
+}
+__device__ const MomentTables g_moment_tables = make_moment_tables();
+static_assert(sizeof(MomentTables) % 8 == 0, "copied by 8-byte words");
 
-__global__ void __launch_bounds__(32 * kMomWarps) correction_p2_moment_kernel(
+constexpr int kMomWarps = 8;  // warps per CTA (one element per warp), two CTAs per SM
+struct alignas(16) MomentWarp {
+    union {
+        struct {
+            int2 dD[kMaxQ][24];  // DS - D_el of the plastic points, packed upper triangle (21 used)
+            int2 ll[kMaxQ][10];  // w s lambda_m lambda_n of the plastic points, pair order
+            int2 w[12];
+        } in;
+        int2 M[10][36];      // moments, full 6 x 6
+        double ke[kKSlots];  // the element's correction, by slot
+    } x;
+    long long R[14][78];  // R over the pairs m <= n of five coordinates but (4, 4), packed upper triangle of 12 x 12
+    int2 v[4][3];         // grad lambda_0..3
+    int8_t qidx[16];
+};
+struct MomentShared {
+    MomentTables tb;
+    alignas(16) int2 lam[kMaxQ][10];  // scale lambda_m lambda_n of the quadrature points, pair order
+    int e_lam;                        // their exponent
+};
+
+// An element whose inputs are not all finite: the point-by-point contraction in FP64, entry by entry, so
+// that infinities and nans reach the entries they reach there.
+__device__ __noinline__ void correction_p2_nonfinite(const double *jinv, const double *bary, const double *DS,
+                                                     const double *w, const double *shear, const double *lame,
+                                                     const int32_t *em, long long g0, unsigned qmask, long long nnz,
+                                                     double scale, double *values) {
+    const int lane = threadIdx.x & 31;
+    for (int idx = lane; idx < 900; idx += 32) {
+        const int32_t pos = em[idx];
+        if (pos < 0) continue;
+        if (pos >= nnz) {
+            flag(SSP_DEV_BAD_INDEX);
+            continue;
+        }
+        double acc = 0.0;
+        for (unsigned m = qmask; m; m &= m - 1u) {
+            const int q = __ffs(m) - 1;
+            const long long g = g0 + q;
+            double grad[2][3];
+            int comp[2];
+            for (int side = 0; side < 2; ++side) {
+                const int al = side == 0 ? idx / 30 : idx % 30, a = al / 3;
+                comp[side] = al - 3 * a;
+                for (int z = 0; z < 3; ++z) grad[side][z] = 0.0;
+                for (int t = 0; t < 2; ++t) {
+                    int mm, coef, k;
+                    node_term(a, t, mm, coef, k);
+                    const double f = coef * (mm == 4 ? 1.0 : bary[4 * q + mm]);
+                    for (int z = 0; z < 3; ++z)
+                        grad[side][z] += f * (k == 0 ? -(jinv[z] + jinv[3 + z] + jinv[6 + z]) : jinv[3 * (k - 1) + z]);
+                }
+            }
+            double sum = 0.0;
+            for (int x = 0; x < 3; ++x)
+                for (int y = 0; y < 3; ++y) {
+                    const int r = bt_row3(comp[0], x), c = bt_row3(comp[1], y);
+                    sum += grad[0][x] * (DS[36 * g + r + 6 * c] - elastic_d<3>(r, c, shear[g], lame[g])) * grad[1][y];
+                }
+            acc += scale * w[g] * sum;
+        }
+        red_add(values + pos, acc);
+    }
+}
+
+__global__ void __launch_bounds__(32 * kMomWarps, 2) correction_p2_moment_kernel(
     const double *__restrict__ jinv, const double *__restrict__ bary, const double *__restrict__ DS,
     const double *__restrict__ w, const int8_t *__restrict__ branch, const double *__restrict__ shear,
     const double *__restrict__ lame, const int32_t *__restrict__ emap, int n_elem, int n_q, long long nnz,
     double scale, double *__restrict__ values, const int32_t *__restrict__ elist, const int32_t *__restrict__ elist_count) {
     constexpr int kWarps = kMomWarps;
+    constexpr int kBits = 58, kBitsRoom = 60;  // room for D - D_el and for grad lambda_0
+    // |R| <= 9 x 2^57 in units that leave the largest 55 to 57 bits as a rule; above 57 R is shifted, so that the
+    // 64-fold sums of K stay below 2^63
+    constexpr int kBitsM = 57, kBitsV = 58, kBitsR = 57;
     extern __shared__ __align__(16) unsigned char mom_raw[];
-    MomentTables &tb = *reinterpret_cast<MomentTables *>(mom_raw);
+    MomentShared &sh = *reinterpret_cast<MomentShared *>(mom_raw);
+    const MomentTables &tb = sh.tb;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    MomentWarp &W = reinterpret_cast<MomentWarp *>(mom_raw + sizeof(MomentTables))[wid];
-    build_moment_tables(tb);
-    __syncthreads();
+    MomentWarp &W = reinterpret_cast<MomentWarp *>(mom_raw + sizeof(MomentShared))[wid];
     const long long n_iter = *elist_count;
     const long long stride = (long long)gridDim.x * kWarps;
-    constexpr int kInBatch = (kMaxQ * 21 + 31) / 32;  // DS entries a lane loads at a time
+    if ((long long)blockIdx.x * kWarps >= n_iter) return;  // uniform: no element for this CTA
+    for (int i = threadIdx.x; i < (int)(sizeof(MomentTables) / 8); i += 32 * kWarps)
+        reinterpret_cast<unsigned long long *>(&sh.tb)[i] = reinterpret_cast<const unsigned long long *>(&g_moment_tables)[i];
+    if (threadIdx.x == 0) sh.e_lam = 0;
+    __syncthreads();
+    double lam = 0.0;
+    if (threadIdx.x < 10 * n_q) {
+        int m = 0, n = 0;
+        sym_pair(threadIdx.x % 10, 4, m, n);
+        const double *b = bary + 4 * (threadIdx.x / 10);
+        lam = scale * (b[m] * b[n]);
+        atomicMax(&sh.e_lam, fx_exponent(lam));
+    }
+    __syncthreads();
+    const int e_lam = sh.e_lam;
+    if (threadIdx.x < 10 * n_q && e_lam < 2047) (&sh.lam[0][0])[threadIdx.x] = fx_split(fx_from_f64(lam, e_lam, kBits));
+    __syncthreads();
     constexpr int kMapBatch = 8;                        // map entries a lane loads at a time
+    const unsigned nnz32 = static_cast<unsigned>(nnz < 0x7FFFFFFFll ? nnz : 0x7FFFFFFFll);
+    const int pair = lane / 3, comp = lane - 3 * pair;   // T, R: pair < 10
+    int pm = 0, pn = 0, er = 0, ec = 0;                  // inputs: entry (er, ec) of the tangents
+    if (lane < 30) sym_pair(pair, 4, pm, pn);
+    if (lane < 21) sym_pair(lane, 6, er, ec);
+    const int r_row = sym_index(pm, pn, 5);
+    // D_el's entry: lambda (normal block) plus 2 G or G (diagonal)
+    const long long el_l = lane < 21 && ec < 3 ? -1ll : 0ll;
+    const int el_g = lane < 21 && er == ec ? (er < 3 ? 2 : 1) : 0;
+    const double *ds_lane = DS + er + 6 * ec;
+    const int pg = lane / 6, eg = lane - 6 * pg;  // M: pairs 2 pg, 2 pg + 1, entries 4 eg .. 4 eg + 3
     for (long long it = (long long)blockIdx.x * kWarps + wid; it < n_iter; it += stride) {
         const int32_t e32 = elist[it];
         if (e32 < 0 || e32 >= n_elem) {  // warp-uniform
@@ -1243,144 +1353,221 @@ __global__ void __launch_bounds__(32 * kMomWarps) correction_p2_moment_kernel(
         }
         const bool pl = lane < n_q && branch[g0 + lane] != 0;
         const unsigned qmask = __ballot_sync(0xffffffffu, pl);
-        const int nq = __popc(qmask);
-        __syncwarp();  // the previous element of this warp is done with its shared slice
-        if (pl) W.qidx[__popc(qmask & ((1u << lane) - 1u))] = static_cast<int8_t>(lane);
-        if (lane < 9) W.x.a.v[1 + lane / 3][lane % 3] = jinv[e * 9 + lane];
-        __syncwarp();
-        if (lane < 3) W.x.a.v[0][lane] = -(W.x.a.v[1][lane] + W.x.a.v[2][lane] + W.x.a.v[3][lane]);
-        // inputs: DS - D_el of the plastic points (every load of a lane issued before its first use)
-        // and their weighted coordinate products
-        const int n_in = nq * 21;
-        for (int base = 0; base < n_in; base += 32 * kInBatch) {
-            double dsv[kInBatch], gv[kInBatch], lv[kInBatch];
+        const int nq = __popc(qmask), kk_own = __popc(qmask & ((1u << lane) - 1u));
+        if (nq == 0) continue;
+        double g_pt = 0.0, l_pt = 0.0, w_pt = 0.0;
+        if (pl) {
+            g_pt = shear[g0 + lane];
+            l_pt = lame[g0 + lane];
+            w_pt = w[g0 + lane];
+        }
+        const double v_pt = lane < 9 ? jinv[e * 9 + lane] : 0.0;
+        double dsv[kMaxQ];  // entry (er, ec) of the plastic points, in order
+        int ex_d = max(fx_exponent(g_pt), fx_exponent(l_pt));
+        unsigned qm = qmask;
 #pragma unroll
-            for (int u = 0; u < kInBatch; ++u) {
-                const int i = base + lane + 32 * u;
-                if (i < n_in) {
-                    const int kk = i / 21, ee = i - 21 * kk, rc = tb.s_pos[ee];
-                    const long long g = g0 + W.qidx[kk];
-                    dsv[u] = DS[g * 36 + (rc >> 4) + 6 * (rc & 15)];
-                    gv[u] = shear[g];
-                    lv[u] = lame[g];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kInBatch; ++u) {
-                const int i = base + lane + 32 * u;
-                if (i < n_in) {
-                    const int kk = i / 21, ee = i - 21 * kk, rc = tb.s_pos[ee];
-                    W.x.a.t.in.dD[kk][ee] = dsv[u] - elastic_d<3>(rc >> 4, rc & 15, gv[u], lv[u]);
-                }
+        for (int kk = 0; kk < kMaxQ; ++kk) {
+            dsv[kk] = 0.0;
+            if (qm) {  // warp-uniform
+                if (lane < 21) dsv[kk] = ds_lane[(g0 + __ffs(qm) - 1) * 36];
+                qm &= qm - 1u;
             }
         }
-        for (int i = lane; i < nq * 10; i += 32) {
-            const int kk = i / 10, pp = i - 10 * kk, q = W.qidx[kk];
-            int m, n;
-            sym_pair(pp, 4, m, n);
-            W.x.a.t.in.ll[kk][pp] = (scale * w[g0 + q]) * (bary[q * 4 + m] * bary[q * 4 + n]);
-        }
-        __syncwarp();
-        // moments M_p = sum_q (w s lambda_qm lambda_qn) dD_q, two entries per lane at a time
-        for (int i0 = lane; i0 < 210; i0 += 64) {
-            const int i1 = i0 + 32 < 210 ? i0 + 32 : i0;
-            const int p0 = i0 / 21, e0 = i0 - 21 * p0, p1 = i1 / 21, e1 = i1 - 21 * p1;
-            double a0 = 0.0, a1 = 0.0;
-            for (int kk = 0; kk < nq; ++kk) {
-                a0 = fma(W.x.a.t.in.ll[kk][p0], W.x.a.t.in.dD[kk][e0], a0);
-                a1 = fma(W.x.a.t.in.ll[kk][p1], W.x.a.t.in.dD[kk][e1], a1);
-            }
-            W.x.a.M[p0][e0] = a0;
-            W.x.a.M[p1][e1] = a1;
-        }
-        __syncwarp();
-        // T_p[(k,c)][t] = sum over beta_(k,c)'s nonzeros of grad lambda_k[comp] M_p[s][t]
-        for (int i0 = lane; i0 < 720; i0 += 64) {
-            double acc[2];
-            int idx[2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = i0 + 32 * h < 720 ? i0 + 32 * h : i0;
-                const int pp = i / 72, rr = i - 72 * pp, kc = rr / 6, t = rr - 6 * kc, k = kc / 3, c = kc - 3 * k;
-                int sr[3], gc[3];
-                beta_rows(c, sr, gc);
-                double a = 0.0;
-#pragma unroll
-                for (int z = 0; z < 3; ++z) a = fma(W.x.a.v[k][gc[z]], W.x.a.M[pp][sym_index(sr[z], t, 6)], a);
-                acc[h] = a;
-                idx[h] = i;
-            }
-            (&W.x.a.t.T[0][0][0])[idx[0]] = acc[0];
-            (&W.x.a.t.T[0][0][0])[idx[1]] = acc[1];
-        }
-        __syncwarp();
-        // R_p[(k,c),(l,d)] = sum over beta_(l,d)'s nonzeros of T_p[(k,c)][s] grad lambda_l[comp]
-        for (int i0 = lane; i0 < 780; i0 += 64) {
-            double acc[2];
-            int dst[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = i0 + 32 * h < 780 ? i0 + 32 * h : i0;
-                const int pp = i / 78, ee = i - 78 * pp;
-                const int kc = tb.r_pos[ee] >> 8, ld = tb.r_pos[ee] & 0xff, l = ld / 3, d = ld - 3 * l;
-                int m, n;
-                sym_pair(pp, 4, m, n);
-                int sr[3], gc[3];
-                beta_rows(d, sr, gc);
-                double a = 0.0;
-#pragma unroll
-                for (int z = 0; z < 3; ++z) a = fma(W.x.a.t.T[pp][kc][sr[z]], W.x.a.v[l][gc[z]], a);
-                acc[h] = a;
-                dst[h] = sym_index(m, n, 5) * 78 + ee;
-            }
-            (&W.R[0][0])[dst[0]] = acc[0];
-            (&W.R[0][0])[dst[1]] = acc[1];
-        }
-        __syncwarp();
-        // R_m4 = sum_n R_mn, then R_44 = sum_m R_m4
-        for (int i = lane; i < 4 * 78; i += 32) {
-            const int m = i / 78, ee = i - 78 * m;
-            W.R[sym_index(m, 4, 5)][ee] = (W.R[sym_index(m, 0, 5)][ee] + W.R[sym_index(m, 1, 5)][ee]) +
-                                         (W.R[sym_index(m, 2, 5)][ee] + W.R[sym_index(m, 3, 5)][ee]);
-        }
-        __syncwarp();
-        for (int ee = lane; ee < 78; ee += 32)
-            W.R[14][ee] = (W.R[4][ee] + W.R[8][ee]) + (W.R[11][ee] + W.R[13][ee]);
-        // the first batch of the element -> CSR map, in flight during K
+        for (int kk = 0; kk < kMaxQ; ++kk) ex_d = max(ex_d, fx_exponent(dsv[kk]));
+        const int e_d = __reduce_max_sync(0xffffffffu, ex_d), e_w = __reduce_max_sync(0xffffffffu, fx_exponent(w_pt)),
+                  e_v = __reduce_max_sync(0xffffffffu, fx_exponent(v_pt));
         const int32_t *em = emap + e * 900;
+        if (max(max(e_d, e_w), max(e_v, e_lam)) == 2047) {  // an infinity or a nan
+            correction_p2_nonfinite(jinv + e * 9, bary, DS, w, shear, lame, em, g0, qmask, nnz, scale, values);
+            continue;
+        }
+        __syncwarp();  // the previous element of this warp is done with its shared slice
+        if (pl) {
+            W.qidx[kk_own] = static_cast<int8_t>(lane);
+            W.x.in.w[kk_own] = fx_split(fx_from_f64(w_pt, e_w, kBits));
+        }
+        const long long vi = fx_from_f64(v_pt, e_v, kBitsRoom);  // 0 beyond lane 8
+        long long v0 = -(vi + __shfl_down_sync(0xffffffffu, vi, 3) + __shfl_down_sync(0xffffffffu, vi, 6));
+        if (lane >= 3) v0 = 0;
+        const unsigned room_v = fx_room(fx_warp_bits(fx_mag(vi) | fx_mag(v0)));
+        if (lane < 9) W.v[1 + lane / 3][lane % 3] = fx_split_top<kBitsV>(fx_scale(vi, room_v));
+        if (lane < 3) W.v[0][lane] = fx_split_top<kBitsV>(fx_scale(v0, room_v));
+        // D_el's entry, formed once where the element has one material
+        const long long g_fx = fx_from_f64(g_pt, e_d, kBitsRoom), l_fx = fx_from_f64(l_pt, e_d, kBitsRoom);
+        const int q0 = __ffs(qmask) - 1;
+        const long long g_0 = __shfl_sync(0xffffffffu, g_fx, q0), l_0 = __shfl_sync(0xffffffffu, l_fx, q0);
+        const bool one_material = __all_sync(0xffffffffu, !pl || (g_fx == g_0 && l_fx == l_0));
+        auto elastic = [&](long long G, long long L) { return (L & el_l) + G * el_g; };
+        long long el = elastic(g_0, l_0);
+        long long dd[kMaxQ];
+        unsigned long long mag_d = 0;
+        qm = qmask;
+#pragma unroll
+        for (int kk = 0; kk < kMaxQ; ++kk) {
+            dd[kk] = 0;
+            if (kk < nq) {  // warp-uniform
+                if (!one_material) {
+                    const int q = __ffs(qm) - 1;
+                    qm &= qm - 1u;
+                    el = elastic(__shfl_sync(0xffffffffu, g_fx, q), __shfl_sync(0xffffffffu, l_fx, q));
+                }
+                if (lane < 21) dd[kk] = fx_from_f64(dsv[kk], e_d, kBitsRoom) - el;
+                mag_d |= fx_mag(dd[kk]);
+            }
+        }
+        const unsigned room_d = fx_room(fx_warp_bits(mag_d));
+        if (lane < 24) {
+#pragma unroll
+            for (int kk = 0; kk < kMaxQ; ++kk)
+                if (kk < nq) W.x.in.dD[kk][lane] = fx_split_top<kBits>(fx_scale(dd[kk], room_d));
+        }
+        __syncwarp();
+        if (lane < 30) {  // three points at a time, lane = pair
+            for (int kk = lane / 10; kk < nq; kk += 3) {
+                W.x.in.ll[kk][lane % 10] = fx_split(FxSum(W.x.in.w[kk], sh.lam[W.qidx[kk]][lane % 10]).value());
+            }
+        }
+        __syncwarp();
+        // moments
+        FxSum m[2][4];
+        if (lane < 30) {
+            for (int kk = 0; kk < nq; ++kk) {
+                const int4 a = *reinterpret_cast<const int4 *>(&W.x.in.ll[kk][2 * pg]);
+                const int4 b0 = *reinterpret_cast<const int4 *>(&W.x.in.dD[kk][4 * eg]),
+                           b1 = *reinterpret_cast<const int4 *>(&W.x.in.dD[kk][4 * eg + 2]);
+                const int2 av[2] = {{a.x, a.y}, {a.z, a.w}}, bv[4] = {{b0.x, b0.y}, {b0.z, b0.w}, {b1.x, b1.y}, {b1.z, b1.w}};
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) m[x][y].add_prod(av[x], bv[y]);
+            }
+        }
+        unsigned long long mag_m = 0;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+                if (lane < 30 && 4 * eg + y < 21) mag_m |= fx_mag(m[x][y].value());
+        const unsigned room_m = fx_room(fx_warp_bits(mag_m));
+        __syncwarp();  // the inputs are dead: their storage becomes the moments
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            if (lane < 30 && 4 * eg + y < 21) {
+                const unsigned at = tb.m_at[4 * eg + y];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int2 v = fx_split_top<kBitsM>(fx_scale(m[x][y].value(), room_m));
+                    W.x.M[2 * pg + x][at & 0xFFFFu] = v;
+                    W.x.M[2 * pg + x][at >> 16] = v;
+                }
+            }
+        }
+        __syncwarp();
+        // lane (p, c): T[k][t] = sum_z grad lambda_k[z] M_p[s_z(c)][t] and the rows (k, c) of R_p,
+        // R[(k,c),(l,d)] = sum_z T[k][s_z(d)] grad lambda_l[z]
+        int mag_r = 0;  // high words' magnitudes
+        if (lane < 30) {
+            int sr[3], gc[3];
+            beta_rows(comp, sr, gc);  // gc = (0, 1, 2) for every component
+            int2 v[4][3];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int z = 0; z < 3; ++z) v[k][z] = W.v[k][z];
+            const int2 *m0 = &W.x.M[pair][sr[0] * 6], *m1 = &W.x.M[pair][sr[1] * 6], *m2 = &W.x.M[pair][sr[2] * 6];
+            long long *Rp = &W.R[r_row][0];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                int2 T[6];  // (the rows of M are read again for each k: kept, they cost 36 registers)
+#pragma unroll
+                for (int t = 0; t < 6; t += 2) {
+                    const int4 a0 = *reinterpret_cast<const int4 *>(m0 + t), a1 = *reinterpret_cast<const int4 *>(m1 + t),
+                               a2 = *reinterpret_cast<const int4 *>(m2 + t);
+                    FxSum s(v[k][0], {a0.x, a0.y}), u(v[k][0], {a0.z, a0.w});
+                    s.add_prod(v[k][1], {a1.x, a1.y});
+                    u.add_prod(v[k][1], {a1.z, a1.w});
+                    s.add_prod(v[k][2], {a2.x, a2.y});
+                    u.add_prod(v[k][2], {a2.z, a2.w});
+                    T[t] = fx_split(s.value());
+                    T[t + 1] = fx_split(u.value());
+                }
+                // row i = 3k + c of the packed upper triangle starts at i * 12 - i (i - 1) / 2 - i; the
+                // entries j = 3l + d >= i are stored (l > k always, l == k when d >= c)
+                const int i = 3 * k + comp;
+                long long *row = Rp + (i * 11 - (i * (i - 1)) / 2);
+#pragma unroll
+                for (int l = k; l < 4; ++l)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        int sd[3], gd[3];
+                        beta_rows(d, sd, gd);
+                        FxSum s(T[sd[0]], v[l][0]);
+                        s.add_prod(T[sd[1]], v[l][1]);
+                        s.add_prod(T[sd[2]], v[l][2]);
+                        const long long rv = s.value();
+                        const int rh = static_cast<int>(rv >> 32);
+                        mag_r |= rh ^ (rh >> 31);
+                        if (l > k || d >= comp) row[3 * l + d] = rv;
+                    }
+            }
+        }
+        // the first batch of the element -> CSR map, in flight during the sums and K
         int32_t pos[kMapBatch];
 #pragma unroll
         for (int u = 0; u < kMapBatch; ++u) {
             const int i = lane + 32 * u;
             pos[u] = i < 900 ? em[i] : -1;
         }
-        __syncwarp();  // M, T and grad lambda are dead: their storage becomes the element matrix
-        const double *Rf = &W.R[0][0];
-        for (int i0 = lane; i0 < kMomEntries; i0 += 96) {
-            double acc[3];
-            int at[3];
-#pragma unroll
-            for (int h = 0; h < 3; ++h) {
-                const int i = i0 + 32 * h < kMomEntries ? i0 + 32 * h : i0;
-                const unsigned long long tm = tb.k_terms[i];
-                double a = 0.0;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const unsigned f = static_cast<unsigned>(tm >> (16 * t)) & 0xffffu;
-                    a = fma(moment_coef(f >> 11), Rf[f & 0x7ffu], a);
-                }
-                acc[h] = a;
-                at[h] = tb.k_pos[i];
-            }
-#pragma unroll
-            for (int h = 0; h < 3; ++h) {
-                const int al = at[h] >> 5, be = at[h] & 31;
-                W.x.ke[al][be] = acc[h];
-                W.x.ke[be][al] = acc[h];
+        const int shift_r = max(0, 64 - __clz(__reduce_or_sync(0xffffffffu, mag_r)) - kBitsR);
+        if (shift_r) {  // warp-uniform
+            __syncwarp();
+            for (int i = lane; i < 10 * 78; i += 32) {
+                const int p = i / 78;
+                W.R[p + (p > 3) + (p > 6) + (p > 8)][i - 78 * p] >>= shift_r;
             }
         }
         __syncwarp();
-        // scatter through the element -> CSR map (both mirror positions were written)
+        // R_m4 = sum_n R_mn
+        for (int ee = lane; ee < 78; ee += 32) {
+            const long long r01 = W.R[1][ee], r02 = W.R[2][ee], r03 = W.R[3][ee];
+            const long long r12 = W.R[6][ee], r13 = W.R[7][ee], r23 = W.R[10][ee];
+            W.R[4][ee] = W.R[0][ee] + r01 + r02 + r03;
+            W.R[8][ee] = r01 + W.R[5][ee] + r12 + r13;
+            W.R[11][ee] = r02 + r12 + W.R[9][ee] + r23;
+            W.R[13][ee] = r03 + r13 + r23 + W.R[12][ee];
+        }
+        __syncwarp();  // and the moments are dead: their storage becomes the element matrix
+        const int unit_m = fx_unit(e_w, kBits) + fx_unit(e_lam, kBits) + kFxDrop + fx_unit(e_d, kBitsRoom) +
+                           fx_top_unit<kBits>(room_d) + kFxDrop + fx_top_unit<kBitsM>(room_m);
+        const int unit_k = unit_m + 2 * (fx_unit(e_v, kBitsRoom) + fx_top_unit<kBitsV>(room_v) + kFxDrop) + shift_r;
+        const char *Rf = reinterpret_cast<const char *>(&W.R[0][0]);
+        auto R_at = [&](unsigned offset) { return *reinterpret_cast<const long long *>(Rf + offset); };
+        auto k_group = [&](auto kind, int first, int last) {
+#pragma unroll 2
+            for (int k0 = first; k0 < last; ++k0) {
+                const int i = 32 * k0 + lane;
+                const uint2 tm = *reinterpret_cast<const uint2 *>(&tb.k_terms[i]);
+                const unsigned o0 = tm.x & 0xFFFFu, o1 = tm.x >> 16, o2 = tm.y & 0xFFFFu, o3 = tm.y >> 16;
+                long long kv;
+                if constexpr (decltype(kind)::value == 0) {  // (4, -1) x (4, -1); R_44 = sum_m R_m4
+                    const unsigned ee = o3 < 8 * 14 * 78 ? 0 : o3 - 8 * 14 * 78;
+                    kv = (R_at(o0) << 4) - ((R_at(o1) + R_at(o2)) << 2) + R_at(8 * 4 * 78 + ee) + R_at(8 * 8 * 78 + ee) +
+                         R_at(8 * 11 * 78 + ee) + R_at(8 * 13 * 78 + ee);
+                } else if constexpr (decltype(kind)::value == 1) {  // (4, -1) x (4, 4)
+                    kv = ((R_at(o0) + R_at(o1)) << 2) - (R_at(o2) + R_at(o3));  // / 4
+                } else {  // (4, 4) x (4, 4)
+                    kv = R_at(o0) + R_at(o1) + R_at(o2) + R_at(o3);  // / 16
+                }
+                W.x.ke[i] = fx_to_f64(kv, unit_k + 2 * decltype(kind)::value);
+            }
+        };
+        k_group(std::integral_constant<int, 0>{}, 0, kVertexVertexIters);
+        k_group(std::integral_constant<int, 1>{}, kVertexVertexIters, kVertexVertexIters + kVertexEdgeIters);
+        k_group(std::integral_constant<int, 2>{}, kVertexVertexIters + kVertexEdgeIters, kKSlots / 32);
+        __syncwarp();
+        // scatter through the element -> CSR map
+        const char *ke = reinterpret_cast<const char *>(W.x.ke);
         for (int base = 0; base < 900; base += 32 * kMapBatch) {
             if (base > 0) {
 #pragma unroll
@@ -1392,12 +1579,10 @@ __global__ void __launch_bounds__(32 * kMomWarps) correction_p2_moment_kernel(
 #pragma unroll
             for (int u = 0; u < kMapBatch; ++u) {
                 const int i = base + lane + 32 * u;
-                if (pos[u] < 0) continue;
-                if (pos[u] >= nnz) {
+                if (static_cast<unsigned>(pos[u]) < nnz32)
+                    red_add(values + pos[u], *reinterpret_cast<const double *>(ke + tb.k_slot[i]));
+                else if (pos[u] >= 0)
                     flag(SSP_DEV_BAD_INDEX);
-                    continue;
-                }
-                red_add(values + pos[u], W.x.ke[i / 30][i % 30]);
             }
         }
     }
@@ -1414,12 +1599,9 @@ __global__ void __launch_bounds__(32 * kMomWarps) correction_p2_moment_kernel(
 // grouped by node-pair type so each group's four coefficients are constants, the element matrix
 // unpadded.  8.4 KB of shared memory per warp: three 8-warp CTAs per SM.
 constexpr int kF32Warps = 8;
-constexpr int kF32KEntries = 512;        // vertex-vertex 78 -> 96, vertex-edge 216 -> 224, edge-edge 171 -> 192
-constexpr int kF32VertexVertexIters = 3, kF32VertexEdgeIters = 7;
-
 struct MomentF32Tables {
-    unsigned long long k_terms[kF32KEntries];  // four packed R offsets (16-bit fields), term order (x, y)
-    uint16_t k_pos[kF32KEntries];             // alpha << 5 | beta; 0xFFFF pads a type group
+    unsigned long long k_terms[kKSlots];  // four packed R offsets (16-bit fields), term order (x, y)
+    uint16_t k_pos[kKSlots];             // alpha << 5 | beta; 0xFFFF pads a type group
     float lam[kMaxQ][4];                      // the points' barycentric coordinates, rounded to FP32
     uint8_t s_pos[21];                        // r << 4 | c of the packed upper triangle of 6 x 6
     uint8_t pair_mn[10];                      // m << 4 | n of the pairs m <= n < 4
@@ -1458,37 +1640,10 @@ __device__ __forceinline__ float f64_to_f32_bits(double x) {
 }
 
 __device__ void build_moment_f32_tables(MomentF32Tables &tb, const double *bary, int n_q) {
-    for (int i = threadIdx.x; i < kF32KEntries; i += blockDim.x) {
-        int al = -1, be = -1;
-        if (i < 32 * kF32VertexVertexIters) {
-            if (i < 78) sym_pair(i, 12, al, be);
-        } else if (i < 32 * (kF32VertexVertexIters + kF32VertexEdgeIters)) {
-            const int j = i - 32 * kF32VertexVertexIters;
-            if (j < 216) {
-                al = j / 18;
-                be = 12 + j % 18;
-            }
-        } else {
-            const int j = i - 32 * (kF32VertexVertexIters + kF32VertexEdgeIters);
-            if (j < 171) {
-                sym_pair(j, 18, al, be);
-                al += 12;
-                be += 12;
-            }
-        }
-        unsigned long long packed = 0;
-        if (al >= 0) {
-            const int a = al / 3, c = al - 3 * a, b = be / 3, d = be - 3 * b;
-            for (int x = 0; x < 2; ++x)
-                for (int y = 0; y < 2; ++y) {
-                    int mx, cx, kx, my, cy, ky;
-                    node_term(a, x, mx, cx, kx);
-                    node_term(b, y, my, cy, ky);
-                    const unsigned off = static_cast<unsigned>(sym_index(mx, my, 5) * 78 + sym_index(3 * kx + c, 3 * ky + d, 12));
-                    packed |= static_cast<unsigned long long>(off) << (16 * (2 * x + y));
-                }
-        }
-        tb.k_terms[i] = packed;
+    for (int i = threadIdx.x; i < kKSlots; i += blockDim.x) {
+        int al, be;
+        k_slot_entry(i, al, be);
+        tb.k_terms[i] = k_slot_terms(i);
         tb.k_pos[i] = al >= 0 ? static_cast<uint16_t>(al << 5 | be) : static_cast<uint16_t>(0xFFFFu);
     }
     for (int i = threadIdx.x; i < n_q * 4; i += blockDim.x) tb.lam[i >> 2][i & 3] = f64_to_f32_bits(bary[i]);
@@ -1655,15 +1810,15 @@ __global__ void __launch_bounds__(32 * kF32Warps, 3) correction_p2_moment_f32_ke
         __syncwarp();  // the moments and inputs are dead: their storage becomes the element matrix
         const float *Rf = &W.R[0][0];
 #pragma unroll 1
-        for (int k0 = 0; k0 < kF32KEntries / 32; ++k0) {
+        for (int k0 = 0; k0 < kKSlots / 32; ++k0) {
             const int i = 32 * k0 + lane;
             const unsigned long long tm = tb.k_terms[i];
             const float r0 = Rf[tm & 0xFFFu], r1 = Rf[(tm >> 16) & 0xFFFu], r2 = Rf[(tm >> 32) & 0xFFFu],
                         r3 = Rf[(tm >> 48) & 0xFFFu];
             float kv;
-            if (k0 < kF32VertexVertexIters)  // (4, -1) x (4, -1)
+            if (k0 < kVertexVertexIters)  // (4, -1) x (4, -1)
                 kv = __fmaf_rn(16.0f, r0, __fmaf_rn(-4.0f, r1 + r2, r3));
-            else if (k0 < kF32VertexVertexIters + kF32VertexEdgeIters)  // (4, -1) x (4, 4)
+            else if (k0 < kVertexVertexIters + kVertexEdgeIters)  // (4, -1) x (4, 4)
                 kv = __fmaf_rn(16.0f, r0 + r1, -4.0f * (r2 + r3));
             else  // (4, 4) x (4, 4)
                 kv = 16.0f * ((r0 + r1) + (r2 + r3));
@@ -2153,7 +2308,7 @@ int ssp_tangent_plastic_correction_p2_moments(const double *jinv, const double *
     if (!jinv || !bary || !ds || !weight || !branch || !shear || !lame || !scatter_map || !elem_list || !elem_count ||
         (nnz_out > 0 && !out_values))
         return SSP_ERR_INVALID;
-    return launch_p2_moments(correction_p2_moment_kernel, kMomWarps, sizeof(MomentTables) + sizeof(MomentWarp) * kMomWarps,
+    return launch_p2_moments(correction_p2_moment_kernel, kMomWarps, sizeof(MomentShared) + sizeof(MomentWarp) * kMomWarps,
                              jinv, bary, ds, weight, branch, shear, lame, scatter_map, n_elem, n_q, nnz_out, scale,
                              out_values, elem_list, elem_count, as_stream(stream));
 }

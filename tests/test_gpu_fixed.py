@@ -1,0 +1,101 @@
+"""The fixed-point kernels of the plain form (csrc/fixed.cuh) against the oracle, at the sizes and
+magnitudes where they can go wrong.
+
+Tolerance: 1e-13 of the largest value.  The fixed-point sums are within 2^-53 of it; the oracle's FP64
+sums of some hundred terms, of either sign and up to an order above the result, are within about
+100 x 10 x 2^-53 = 1e-13 of theirs."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-13
+
+
+@pytest.fixture(autouse=True)
+def _clean_status(cuda_device):
+    from slope_stability_petsc4py_gb300 import _lib
+
+    _lib.device_status(clear=True)
+    yield
+    assert _lib.device_status(clear=True) == 0
+
+
+def _pattern(et, dims, dim=3):
+    from slope_stability_petsc4py_gb300 import ConstitutiveOperator, synthetic
+
+    mats = synthetic.MaterialSet.layered(4, seed=1)
+    mesh = (synthetic.slope_mesh_3d(*dims, elem_type=et, n_layers=4) if dim == 3 else
+            synthetic.slope_mesh_2d(*dims, elem_type=et, n_layers=4))
+    specs = [dict(c0=float(mats.c0[i]), phi=float(mats.phi[i]), psi=float(mats.psi[i]), young=float(mats.young[i]),
+                  poisson=float(mats.poisson[i]), gamma_sat=20.0, gamma_unsat=20.0) for i in range(mats.c0.size)]
+    op = ConstitutiveOperator.from_mesh(mesh.coord, mesh.elem, mesh.q_mask, mesh.material_id, specs, elem_type=et)
+    return op, op.owned_tangent_pattern
+
+
+def _plastic_state(op, pat, n_plastic, magnitude, seed):
+    """Branch codes with n_plastic points in every element but the first (which has none), moduli and
+    symmetric tangents of the given magnitude that differ from the elastic ones at those points."""
+    rng = np.random.default_rng(seed)
+    n_el, n_q, ns = int(pat.overlap_elements.size), pat.n_q, pat.n_strain
+    branch = np.zeros((n_el, n_q), dtype=np.int8)
+    for e in range(1, n_el):
+        branch[e, rng.choice(n_q, n_plastic, replace=False)] = rng.integers(1, 5, n_plastic)
+    idx = pat.local_int_indices
+    shear, lame = magnitude * op.shear[idx], magnitude * op.lame[idx]
+    nn = 3 if pat.dim == 3 else 2
+    D = np.zeros((n_el * n_q, ns, ns))
+    D[:, :nn, :nn] = lame[:, None, None]
+    for i in range(ns):
+        D[:, i, i] += 2.0 * shear if i < nn else shear
+    A = rng.standard_normal(D.shape)
+    dD = (A + A.transpose(0, 2, 1)) * (shear * 10.0 ** rng.uniform(-3.0, 0.3, shear.size))[:, None, None]
+    dD[branch.reshape(-1) == 0] = 0.0
+    return branch.reshape(-1), shear, lame, D + dD, dD
+
+
+@pytest.mark.parametrize("n_plastic,magnitude", [(1, 1.0), (2, 1e-150), (4, 1e150), (5, 1.0), (8, 1e-9), (11, 1e6)])
+def test_p2_moment_correction(oracle, n_plastic, magnitude):
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.distributed_tangent import _p2_affine_inputs
+
+    op, pat = _pattern("P2", (5, 2, 3))
+    d = _p2_affine_inputs(pat)
+    branch, shear, lame, DS, dD = _plastic_state(op, pat, n_plastic, magnitude, n_plastic)
+    n_el, scale = int(pat.overlap_elements.size), 0.7
+    rows = np.ascontiguousarray(DS.transpose(0, 2, 1).reshape(-1, 36))
+    dev = {k: torch.as_tensor(v, device="cuda") for k, v in dict(branch=branch, shear=shear, lame=lame, ds=rows).items()}
+
+    def run(ds):
+        vals = torch.zeros(pat.nnz, dtype=torch.float64, device="cuda")
+        elist = torch.arange(n_el, dtype=torch.int32, device="cuda")
+        count = torch.tensor([n_el], dtype=torch.int32, device="cuda")
+        _lib.call("ssp_tangent_plastic_correction_p2_moments", _lib.ptr(d["jinv"]), _lib.ptr(d["bary"]), _lib.ptr(ds),
+                  _lib.ptr(d["weight"]), _lib.ptr(dev["branch"]), _lib.ptr(dev["shear"]), _lib.ptr(dev["lame"]),
+                  _lib.ptr(d["scatter_map"]), n_el, pat.n_q, pat.nnz, scale, _lib.ptr(vals), _lib.ptr(elist),
+                  _lib.ptr(count), _lib.stream_handle())
+        return vals.cpu().numpy()
+
+    want = oracle.tangent_scatter(3, pat.dphi1, pat.dphi2, pat.dphi3,
+                                  np.ascontiguousarray(scale * dD.transpose(0, 2, 1).reshape(-1, 36)),
+                                  pat.overlap_assembly_weight, d["scatter_map"].cpu().numpy(), pat.n_q, pat.nnz)
+    got = run(dev["ds"])
+    assert rel_err(got, want) <= TOL
+    # an infinity and a nan stay in their element, in the entries the contraction takes them to
+    bad = int(np.flatnonzero(branch)[0])
+    ds = dev["ds"].clone()
+    ds[bad, 0] = float("inf")
+    ds[bad, 21] = float("nan")  # (3, 3)
+    out = run(ds)
+    smap = d["scatter_map"].cpu().numpy()[bad // pat.n_q]
+    assert not np.isfinite(out[smap[smap >= 0]]).all() and np.isnan(out).any()
+    others = np.ones(pat.nnz, dtype=bool)
+    others[smap[smap >= 0]] = False
+    assert np.array_equal(out[others], got[others]) or rel_err(out[others], got[others]) <= TOL
