@@ -226,74 +226,192 @@ __device__ __forceinline__ void sym_matvec(const double *M, const double *v, dou
     out[2] = M[5] * v[0] + M[4] * v[1] + M[2] * v[2];
 }
 
-// One thread per element: bary is [n_q][4] (λ0..λ3 of each point).
-__global__ void __launch_bounds__(64) strain3_p2_affine_kernel(const double *__restrict__ jinv,
-                                                               const double *__restrict__ bary,
-                                                               const double *__restrict__ u,
-                                                               const int32_t *__restrict__ dof, long long n_u,
-                                                               int n_elem, int n_q, double *__restrict__ E) {
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= n_elem) return;
+// Both kernels: one thread per element, one warp per CTA, in 58-bit fixed point (fixed.cuh; one exponent per
+// element for the displacement differences, the gradients, the stresses, ...).  In FP64 they were bound by
+// that pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 48 and 71, bound by the
+// latency of 10 to 12 warps an SM of 160 registers and some 4,200 integer instructions an element).  E and the stresses pass
+// through shared memory, so that a warp's 32 elements are one contiguous block of global memory; elements
+// with an input that is not finite take the FP64 form of the same sums.
+constexpr int kP2StageMaxQ = 30;  // points per element up to which a warp's block is staged (46 KiB)
+
+__device__ __noinline__ void strain3_p2_nonfinite(const double *jinv, const double *bary, const double *u,
+                                                  const int32_t *dl, long long n_u, int n_q, double *out) {
+    for (int q = 0; q < n_q; ++q) {
+        double G[3][3] = {};
+        for (int a = 0; a < 10; ++a) {
+            double g[3];
+            for (int z = 0; z < 3; ++z) {
+                const double g0 = -(jinv[z] + jinv[3 + z] + jinv[6 + z]);
+                if (a < 4) {
+                    g[z] = (4.0 * bary[4 * q + a] - 1.0) * (a == 0 ? g0 : jinv[3 * (a - 1) + z]);
+                } else {
+                    const int i = (a == 5 || a == 7) ? 1 : (a == 8 ? 2 : 0), j = a == 4 ? 1 : (a == 5 || a == 6) ? 2 : 3;
+                    g[z] = 4.0 * (bary[4 * q + i] * jinv[3 * (j - 1) + z] + bary[4 * q + j] * (i == 0 ? g0 : jinv[3 * (i - 1) + z]));
+                }
+            }
+            for (int c = 0; c < 3; ++c) {
+                const int32_t i = dl[3 * a + c];
+                const double v = i < 0 || i >= n_u ? 0.0 : u[i];
+                for (int z = 0; z < 3; ++z) G[c][z] += v * g[z];
+            }
+        }
+        out[6 * q] = G[0][0];
+        out[6 * q + 1] = G[1][1];
+        out[6 * q + 2] = G[2][2];
+        out[6 * q + 3] = G[0][1] + G[1][0];
+        out[6 * q + 4] = G[1][2] + G[2][1];
+        out[6 * q + 5] = G[0][2] + G[2][0];
+    }
+}
+
+// the points' lambda_1..3 as limbs in shared memory, in units of 2^(*e - 1080); *e >= 1022 (values below 1)
+template <int LIMB>
+__device__ __forceinline__ void p2_lambda_table(const double *bary, int n_q, int2 *table, int *e_out) {
+    const int lane = threadIdx.x;
+    int e = 1022;
+    for (int i = lane; i < 3 * n_q; i += 32) e = max(e, fx_exponent(bary[4 * (i / 3) + 1 + i % 3]));
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (e < 2047)
+        for (int i = lane; i < 3 * n_q; i += 32) table[i] = fx_split<LIMB>(fx_from_f64(bary[4 * (i / 3) + 1 + i % 3], e, 58));
+    *e_out = e;
+}
+
+// Strain.  bary is [n_q][4] (λ0..λ3 of each point).  With d_a = u_a - u_0 every A_im - A_0m is a sum of at
+// most nine d's, so the differences are taken first, exactly, and brought to 58 bits by their largest.
+template <bool STAGED>
+__global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double *__restrict__ jinv,
+                                                                   const double *__restrict__ bary,
+                                                                   const double *__restrict__ u,
+                                                                   const int32_t *__restrict__ dof, long long n_u,
+                                                                   int n_elem, int n_q, double *__restrict__ E) {
+    constexpr int kLambdaLimb = 30;  // S has up to 61 bits: limbs of 30 bits, lambda's too
+    extern __shared__ __align__(16) unsigned char p2_raw[];
+    int2 *s_lam = reinterpret_cast<int2 *>(p2_raw);  // [n_q][3]
+    double *stage = reinterpret_cast<double *>(p2_raw + ((24 * n_q + 15) & ~15));
+    const int lane = threadIdx.x;
+    const long long e0 = blockIdx.x * 32ll, e = e0 + lane;
+    int e_lam;
+    p2_lambda_table<kLambdaLimb>(bary, n_q, s_lam, &e_lam);
+    // the warp's dof lids, through the staging area
+    const int n_here = static_cast<int>(n_elem - e0 < 32 ? n_elem - e0 : 32);
+    int32_t *s_dof = reinterpret_cast<int32_t *>(stage);
+    if (STAGED) {
+        for (int i = lane; i < 30 * n_here; i += 32) s_dof[i] = dof[e0 * 30 + i];
+    }
+    __syncwarp();
+    const int32_t *dl = STAGED ? s_dof + 30 * lane : dof + e * 30;
+    const bool valid = e < n_elem;
+    double *out = STAGED ? stage + 6 * n_q * lane : E + 6 * n_q * e;
     double un[10][3];
-    const int32_t *dl = dof + e * 30;
+    int e_u = 0;
+    bool bad = false;
 #pragma unroll
     for (int a = 0; a < 10; ++a) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const int32_t i = dl[3 * a + c];
-            if (i < 0 || i >= n_u) {
-                flag(SSP_DEV_BAD_INDEX);
-                un[a][c] = 0.0;
-            } else {
-                un[a][c] = u[i];
-            }
+            const int32_t i = valid ? dl[3 * a + c] : 0;
+            un[a][c] = 0.0;
+            if (i < 0 || i >= n_u) bad = true;
+            else if (valid) un[a][c] = u[i];
+            e_u = max(e_u, fx_exponent(un[a][c]));
         }
     }
-    double gl[3][3];  // ∇λ_1..3
+    if (bad && valid) flag(SSP_DEV_BAD_INDEX);
+    double jv[9];
+    int e_j = 0;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) gl[k / 3][k % 3] = jinv[e * 9 + k];
-    // ∇u = Σ_m λ_m G_m, G_m = Σ_{i=1..3} (A_im − A_0m) ⊗ ∇λ_i, A_ii = 3u_i, A_im = 4u_(edge im) − u_i
-    double S[4][6];
+    for (int k = 0; k < 9; ++k) {
+        jv[k] = valid ? jinv[e * 9 + k] : 0.0;
+        e_j = max(e_j, fx_exponent(jv[k]));
+    }
+    const bool finite = e_u < 2047 && e_j < 2047 && e_lam < 2047;
+    if (STAGED) __syncwarp();  // every lane has its lids: the area may become the strains
+    if (valid && !finite) strain3_p2_nonfinite(jinv + e * 9, bary, u, dof + e * 30, n_u, n_q, out);
+    if (valid && finite) {
+        long long d[10][3];  // u_a - u_0, then times 2^(s - 4): 58 bits
+        unsigned long long mag = 0;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        double A0[3], G[3][3];
+        for (int c = 0; c < 3; ++c) {
+            const long long u0 = fx_from_f64(un[0][c], e_u, 60);
+            d[0][c] = 0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) A0[c] = m == 0 ? 3.0 * un[0][c] : 4.0 * un[p2_edge_node(0, m)][c] - un[0][c];
+            for (int a = 1; a < 10; ++a) {
+                d[a][c] = fx_from_f64(un[a][c], e_u, 60) - u0;
+                mag |= fx_mag(d[a][c]);
+            }
+        }
+        const int s = min(__clzll(static_cast<long long>(mag)) - 2, 58);  // to 62 bits
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+        for (int a = 1; a < 10; ++a)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) G[c][k] = 0.0;
+            for (int c = 0; c < 3; ++c) d[a][c] = (d[a][c] << s) >> 4;
+        int2 gl[3][3];  // ∇λ_1..3
 #pragma unroll
-        for (int i = 1; i < 4; ++i) {
+        for (int k = 0; k < 9; ++k) gl[k / 3][k % 3] = fx_split(fx_from_f64(jv[k], e_j, 58));
+        // ∇u = Σ_m λ_m G_m, G_m = Σ_{i=1..3} (A_im − A_0m) ⊗ ∇λ_i, A_ii = 3u_i, A_im = 4u_(edge im) − u_i
+        long long S0[6];
+        int2 dS[3][6];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            int2 b[3][3];  // (A_im - A_0m) / 16, at most 9 x 2^54
+#pragma unroll
+            for (int i = 1; i < 4; ++i)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const long long A0 = m == 0 ? 0ll : 4 * d[p2_edge_node(0, m)][c];
+                    const long long Ai = i == m ? 3 * d[i][c] : 4 * d[p2_edge_node(i, m)][c] - d[i][c];
+                    b[i - 1][c] = fx_split_top<58>(Ai - A0);
+                }
+            long long Sm[6];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const double Ai = i == m ? 3.0 * un[i][c] : 4.0 * un[p2_edge_node(i, m)][c] - un[i][c];
-                const double b = Ai - A0[c];
+                FxSum n(b[0][c], gl[0][c]);  // G_cc
+                n.add_prod(b[1][c], gl[1][c]);
+                n.add_prod(b[2][c], gl[2][c]);
+                Sm[c] = n.value();
+                const int x = c == 2 ? 0 : c, y = c == 0 ? 1 : 2;  // (0,1), (1,2), (0,2)
+                FxSum t(b[0][x], gl[0][y]);  // G_xy + G_yx
+                t.add_prod(b[0][y], gl[0][x]);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) G[c][k] += b * gl[i - 1][k];
+                for (int i = 1; i < 3; ++i) {
+                    t.add_prod(b[i][x], gl[i][y]);
+                    t.add_prod(b[i][y], gl[i][x]);
+                }
+                Sm[3 + c] = t.value();
+            }
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                if (m == 0) S0[c] = Sm[c];
+                else dS[m - 1][c] = fx_split<kLambdaLimb>(Sm[c] - S0[c]);
             }
         }
-        S[m][0] = G[0][0];
-        S[m][1] = G[1][1];
-        S[m][2] = G[2][2];
-        S[m][3] = G[0][1] + G[1][0];
-        S[m][4] = G[1][2] + G[2][1];
-        S[m][5] = G[0][2] + G[2][0];
+        // the coordinates sum to one: E(q) = S_0 + sum_{m>=1} lambda_qm (S_m - S_0)
+        const int unit_S = fx_unit(e_u, 60) - s + 8 + fx_unit(e_j, 58) + kFxDrop, shift_0 = fx_unit(e_lam, 58) + 2 * kLambdaLimb;
+        const int unit_E = unit_S + shift_0;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) S0[c] >>= min(shift_0, 63);
+#pragma unroll 1
+        for (int q = 0; q < n_q; ++q) {
+            const int2 l1 = s_lam[3 * q], l2 = s_lam[3 * q + 1], l3 = s_lam[3 * q + 2];
+            double v[6];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                FxSum t(dS[0][c], l1);
+                t.add_prod(dS[1][c], l2);
+                t.add_prod(dS[2][c], l3);
+                v[c] = fx_to_f64(t.value<kLambdaLimb>() + S0[c], unit_E);
+            }
+            double2 *o = reinterpret_cast<double2 *>(out + 6 * q);
+            o[0] = make_double2(v[0], v[1]);
+            o[1] = make_double2(v[2], v[3]);
+            o[2] = make_double2(v[4], v[5]);
+        }
     }
-    // the coordinates sum to one: E(q) = S_0 + sum_{m>=1} lambda_qm (S_m - S_0), 18 FMA per point
-#pragma unroll
-    for (int m = 1; m < 4; ++m)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) S[m][c] -= S[0][c];
-    for (int q = 0; q < n_q; ++q) {
-        const double l1 = bary[4 * q + 1], l2 = bary[4 * q + 2], l3 = bary[4 * q + 3];
-        double v[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) v[c] = fma(l3, S[3][c], fma(l2, S[2][c], fma(l1, S[1][c], S[0][c])));
-        double2 *o = reinterpret_cast<double2 *>(E + 6 * (e * n_q + q));
-        o[0] = make_double2(v[0], v[1]);
-        o[1] = make_double2(v[2], v[3]);
-        o[2] = make_double2(v[4], v[5]);
+    if (STAGED) {
+        __syncwarp();
+        const double2 *src = reinterpret_cast<const double2 *>(stage);
+        double2 *dst = reinterpret_cast<double2 *>(E + 6 * n_q * e0);
+        for (int i = lane; i < 3 * n_q * n_here; i += 32) dst[i] = src[i];
     }
 }
 
@@ -439,68 +557,185 @@ __global__ void __launch_bounds__(kAffineThreads) force3_affine_kernel(const dou
     if (r2 >= 0) red_add(F + r2, a2);
 }
 
-// One thread per element; elem_row as in force_element_kernel; atomics into F.
-__global__ void __launch_bounds__(64) force3_p2_affine_kernel(const double *__restrict__ jinv,
-                                                              const double *__restrict__ bary,
-                                                              const double *__restrict__ S,
-                                                              const double *__restrict__ w,
-                                                              const int32_t *__restrict__ elem_row, int n_rows,
-                                                              int n_elem, int n_q, double *__restrict__ F) {
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= n_elem) return;
-    double M[4][6];
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) M[m][c] = 0.0;
-    for (int q = 0; q < n_q; ++q) {
-        const long long g = e * n_q + q;
-        const double2 *s2 = reinterpret_cast<const double2 *>(S + 6 * g);
-        const double2 a = s2[0], b = s2[1], c2 = s2[2];
-        const double wq = w[g];
-        const double T[6] = {wq * a.x, wq * a.y, wq * b.x, wq * b.y, wq * c2.x, wq * c2.y};
-        const double l[4] = {bary[4 * q], bary[4 * q + 1], bary[4 * q + 2], bary[4 * q + 3]};
-#pragma unroll
+__device__ __noinline__ void force3_p2_nonfinite(const double *jinv, const double *bary, const double *S, const double *w,
+                                                 const int32_t *er, int n_rows, int n_q, double *F) {
+    double M[4][6] = {}, gl[4][3];
+    for (int q = 0; q < n_q; ++q)
         for (int m = 0; m < 4; ++m)
-#pragma unroll
-            for (int c = 0; c < 6; ++c) M[m][c] += l[m] * T[c];
+            for (int c = 0; c < 6; ++c) M[m][c] += bary[4 * q + m] * (w[q] * S[6 * q + c]);
+    for (int k = 0; k < 3; ++k) {
+        for (int i = 0; i < 3; ++i) gl[1 + i][k] = jinv[3 * i + k];
+        gl[0][k] = -(gl[1][k] + gl[2][k] + gl[3][k]);
     }
-    double gl[4][3];
+    for (int a = 0; a < 10; ++a) {
+        double f[3];
+        if (a < 4) {
+            double V[6];
+            for (int c = 0; c < 6; ++c) V[c] = 4.0 * M[a][c] - (M[0][c] + M[1][c] + M[2][c] + M[3][c]);
+            sym_matvec(V, gl[a], f);
+        } else {
+            const int i = (a == 5 || a == 7) ? 1 : (a == 8 ? 2 : 0), j = a == 4 ? 1 : (a == 5 || a == 6) ? 2 : 3;
+            double x[3], y[3];
+            sym_matvec(M[i], gl[j], x);
+            sym_matvec(M[j], gl[i], y);
+            for (int c = 0; c < 3; ++c) f[c] = 4.0 * (x[c] + y[c]);
+        }
+        for (int c = 0; c < 3; ++c) {
+            const int row = er[3 * a + c];
+            if (row >= 0 && row < n_rows) red_add(F + row, f[c]);
+        }
+    }
+}
+
+// (M v)[c] for M symmetric as [11,22,33,12,23,13], added to a sum
+__device__ __forceinline__ void fx_sym_row(FxSum &s, const int2 *M, const int2 *v, int c) {
+    constexpr int kRow[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
 #pragma unroll
-    for (int k = 0; k < 9; ++k) gl[1 + k / 3][k % 3] = jinv[e * 9 + k];
+    for (int z = 0; z < 3; ++z) s.add_prod(M[kRow[c][z]], v[z]);
+}
+
+// Force; elem_row as in force_element_kernel; reductions into F.  The moment of lambda_0 is the sum of w sigma
+// less the other three.
+template <bool STAGED>
+__global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *__restrict__ jinv,
+                                                                  const double *__restrict__ bary,
+                                                                  const double *__restrict__ S,
+                                                                  const double *__restrict__ w,
+                                                                  const int32_t *__restrict__ elem_row, int n_rows,
+                                                                  int n_elem, int n_q, double *__restrict__ F) {
+    extern __shared__ __align__(16) unsigned char p2_raw[];
+    int2 *s_lam = reinterpret_cast<int2 *>(p2_raw);  // [n_q][3]
+    double *stage = reinterpret_cast<double *>(p2_raw + ((24 * n_q + 15) & ~15));
+    const int lane = threadIdx.x;
+    const long long e0 = blockIdx.x * 32ll, e = e0 + lane;
+    const int n_here = static_cast<int>(n_elem - e0 < 32 ? n_elem - e0 : 32);
+    if (STAGED) {
+        const char *src = reinterpret_cast<const char *>(S + 6 * n_q * e0);
+        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(stage));
+        for (int i = lane; i < 3 * n_q * n_here; i += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
+    }
+    int e_lam;
+    p2_lambda_table<kFxLimb>(bary, n_q, s_lam, &e_lam);
+    if (STAGED) asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncwarp();
+    if (e >= n_elem) return;
+    const double *Se = STAGED ? stage + 6 * n_q * lane : S + 6 * n_q * e;
+    const double *we = w + e * n_q;
+    int e_s = 0, e_w = 0, e_j = 0;
+#pragma unroll 1
+    for (int q = 0; q < n_q; ++q) {
+        e_w = max(e_w, fx_exponent(we[q]));
+        const double2 *s2 = reinterpret_cast<const double2 *>(Se + 6 * q);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) gl[0][k] = -(gl[1][k] + gl[2][k] + gl[3][k]);
-    double f[10][3];
+        for (int k = 0; k < 3; ++k) e_s = max(e_s, max(fx_exponent(s2[k].x), fx_exponent(s2[k].y)));
+    }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {  // vertices: (4 M_i − Σ_m M_m) ∇λ_i
-        double V[6];
+    for (int k = 0; k < 9; ++k) e_j = max(e_j, fx_exponent(jinv[e * 9 + k]));
+    const int32_t *er = elem_row + e * 30;
+    if (max(max(e_s, e_w), max(e_j, e_lam)) == 2047) {
+        force3_p2_nonfinite(jinv + e * 9, bary, Se, we, er, n_rows, n_q, F);
+        return;
+    }
+    // the sums of n_q products, and of four moments, stay below 2^63
+    const int bits_s = 57 - (n_q <= 15 ? 0 : 28 - __clz(n_q));
+    long long Mt[6];  // sum of w sigma
+    FxSum Ms[3][6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) V[c] = 4.0 * M[i][c] - (M[0][c] + M[1][c] + M[2][c] + M[3][c]);
-        sym_matvec(V, gl[i], f[i]);
+    for (int c = 0; c < 6; ++c) Mt[c] = 0;
+#pragma unroll 1
+    for (int q = 0; q < n_q; ++q) {
+        const int2 wq = fx_split(fx_from_f64(we[q], e_w, 58));
+        const int2 l[3] = {s_lam[3 * q], s_lam[3 * q + 1], s_lam[3 * q + 2]};
+        const double2 *s2 = reinterpret_cast<const double2 *>(Se + 6 * q);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double2 sv = s2[k];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = 2 * k + h;
+                const long long T = FxSum(wq, fx_split(fx_from_f64(h == 0 ? sv.x : sv.y, e_s, bits_s))).value();
+                Mt[c] += T;
+                const int2 Tl = fx_split(T);
+#pragma unroll
+                for (int m = 0; m < 3; ++m) Ms[m][c].add_prod(l[m], Tl);
+            }
+        }
+    }
+    // all in units of Mt's, brought to 58 bits by the largest
+    const int shift_l = min(e_lam - 1022, 63);
+    long long M[4][6];
+    unsigned long long mag = 0;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        const long long sum = Mt[c] >> shift_l;
+        M[0][c] = sum;
+#pragma unroll
+        for (int m = 1; m < 4; ++m) {
+            M[m][c] = Ms[m - 1][c].value();
+            M[0][c] -= M[m][c];
+            mag |= fx_mag(M[m][c]);
+        }
+        Mt[c] = sum;
+        mag |= fx_mag(M[0][c]) | fx_mag(sum);
+    }
+    const int lz = min(__clzll(static_cast<long long>(mag)), 63) - 6;  // to 58 bits (the sums may have 62)
+    const int up = max(lz, 0), down = max(-lz, 0);
+    int2 Ml[4][6], v[4][3];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        Mt[c] = (Mt[c] << up) >> down;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            M[m][c] = (M[m][c] << up) >> down;
+            Ml[m][c] = fx_split(M[m][c]);
+        }
+    }
+    // grad lambda_0..3: the high limb of grad lambda_0 has up to 31 bits
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        long long v0 = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const long long x = fx_from_f64(jinv[e * 9 + 3 * i + k], e_j, 58);
+            v0 -= x;
+            v[1 + i][k] = fx_split(x);
+        }
+        v[0][k] = fx_split(v0);
+    }
+    const int unit_M = fx_unit(e_s, bits_s) + fx_unit(e_w, 58) + kFxDrop + shift_l - up + down;
+    const int unit_f = unit_M + fx_unit(e_j, 58) + kFxDrop;
+    auto emit = [&](int a, int c, const FxSum &f, int unit) {
+        const int row = er[3 * a + c];
+        if (row < 0) return;
+        if (row >= n_rows) {
+            flag(SSP_DEV_BAD_INDEX);
+            return;
+        }
+        red_add(F + row, fx_to_f64(f.value(), unit));
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // vertices: (4 M_i − Σ_m M_m) ∇λ_i, the bracket below 2^61, by 8
+        int2 V[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) V[c] = fx_split((4 * M[i][c] - Mt[c]) >> 3);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            FxSum f;
+            fx_sym_row(f, V, v[i], c);
+            emit(i, c, f, unit_f + 3);
+        }
     }
     constexpr int kEi[6] = {0, 1, 0, 1, 2, 0}, kEj[6] = {1, 2, 2, 3, 3, 3};
 #pragma unroll
     for (int k = 0; k < 6; ++k) {  // edges: 4 (M_i ∇λ_j + M_j ∇λ_i)
         const int i = kEi[k], j = kEj[k];
-        double x[3], y[3];
-        sym_matvec(M[i], gl[j], x);
-        sym_matvec(M[j], gl[i], y);
-        const int a = p2_edge_node(i, j);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[a][c] = 4.0 * (x[c] + y[c]);
-    }
-    const int32_t *er = elem_row + e * 30;
-#pragma unroll
-    for (int a = 0; a < 10; ++a) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const int row = er[3 * a + c];
-            if (row < 0) continue;
-            if (row >= n_rows) {
-                flag(SSP_DEV_BAD_INDEX);
-                continue;
-            }
-            red_add(F + row, f[a][c]);
+            FxSum f;
+            fx_sym_row(f, Ml[i], v[j], c);
+            fx_sym_row(f, Ml[j], v[i], c);
+            emit(p2_edge_node(i, j), c, f, unit_f + 2);
         }
     }
 }
@@ -2144,8 +2379,13 @@ int ssp_assemble_overlap_strain_3d_p2_affine(const double *jinv, const double *b
     if ((long long)n_elem * n_q != n_int) return SSP_ERR_INVALID;
     if (n_elem == 0) return SSP_OK;
     if (!jinv || !bary || !u_overlap || !elem_dof_lids || !out_values) return SSP_ERR_INVALID;
-    strain3_p2_affine_kernel<<<grid_for(n_elem, 64), 64, 0, as_stream(stream)>>>(jinv, bary, u_overlap, elem_dof_lids,
-                                                                                 n_u, n_elem, n_q, out_values);
+    const size_t table = (24 * (size_t)n_q + 15) & ~size_t(15);
+    if (n_q <= kP2StageMaxQ && table + 32 * 48 * (size_t)n_q >= 3840 + table)
+        strain3_p2_affine_kernel<true><<<grid_for(n_elem, 32), 32, table + 32 * 48 * (size_t)n_q, as_stream(stream)>>>(
+            jinv, bary, u_overlap, elem_dof_lids, n_u, n_elem, n_q, out_values);
+    else
+        strain3_p2_affine_kernel<false><<<grid_for(n_elem, 32), 32, table, as_stream(stream)>>>(
+            jinv, bary, u_overlap, elem_dof_lids, n_u, n_elem, n_q, out_values);
     return launch_status();
 }
 
@@ -2158,8 +2398,13 @@ int ssp_assemble_force_element_p2_affine(const double *jinv, const double *bary,
     if (n_rows > 0 && cudaMemsetAsync(out_values, 0, sizeof(double) * n_rows, st) != cudaSuccess) return SSP_ERR_CUDA;
     if (n_elem == 0) return SSP_OK;
     if (!jinv || !bary || !stress || !weight || !elem_row) return SSP_ERR_INVALID;
-    force3_p2_affine_kernel<<<grid_for(n_elem, 64), 64, 0, st>>>(jinv, bary, stress, weight, elem_row, n_rows, n_elem,
-                                                                 n_q, out_values);
+    const size_t table = (24 * (size_t)n_q + 15) & ~size_t(15);
+    if (n_q <= kP2StageMaxQ && (reinterpret_cast<uintptr_t>(stress) & 15u) == 0)
+        force3_p2_affine_kernel<true><<<grid_for(n_elem, 32), 32, table + 32 * 48 * (size_t)n_q, st>>>(
+            jinv, bary, stress, weight, elem_row, n_rows, n_elem, n_q, out_values);
+    else
+        force3_p2_affine_kernel<false><<<grid_for(n_elem, 32), 32, table, st>>>(jinv, bary, stress, weight, elem_row, n_rows,
+                                                                                n_elem, n_q, out_values);
     return launch_status();
 }
 

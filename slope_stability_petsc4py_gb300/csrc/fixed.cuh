@@ -61,8 +61,9 @@ __device__ __forceinline__ double fx_to_f64(long long x, int unit) {
     return hi == 0u ? 0.0 : __hiloint2double(static_cast<int>(oh), static_cast<int>(m));
 }
 
+template <int LIMB = kFxLimb>
 __device__ __forceinline__ int2 fx_split(long long x) {
-    return make_int2(static_cast<int>(x >> kFxLimb), static_cast<int>(x) & ((1 << kFxLimb) - 1));
+    return make_int2(static_cast<int>(x >> LIMB), static_cast<int>(x) & ((1 << LIMB) - 1));
 }
 
 // Bits of the largest magnitude of a block: the magnitudes' bits (one's complement of negative values) are
@@ -110,7 +111,8 @@ struct FxSum {
         hh = fx_mad(a.x, b.x, hh);
         mid = fx_mad(a.y, b.x, fx_mad(a.x, b.y, mid));
     }
-    __device__ __forceinline__ long long value() const { return hh + (mid >> kFxLimb); }
+    template <int LIMB = kFxLimb>
+    __device__ __forceinline__ long long value() const { return hh + (mid >> LIMB); }
 };
 
 }  // namespace ssp

@@ -99,3 +99,75 @@ def test_p2_moment_correction(oracle, n_plastic, magnitude):
     others = np.ones(pat.nnz, dtype=bool)
     others[smap[smap >= 0]] = False
     assert np.array_equal(out[others], got[others]) or rel_err(out[others], got[others]) <= TOL
+
+
+@pytest.mark.parametrize("dims,magnitude,n_q", [((5, 2, 3), 1.0, 11), ((4, 3, 1), 1e-140, 11), ((7, 1, 1), 1e140, 11),
+                                                ((4, 2, 2), 1.0, 1), ((4, 2, 2), 1.0, 2), ((4, 2, 2), 1e5, 31), ((4, 2, 2), 1.0, 64)])
+def test_p2_strain_and_force(oracle, dims, magnitude, n_q):
+    """Element counts that are no multiple of a warp, other point counts (staged and not), magnitudes near
+    the ends of FP64's range, and inputs that are not finite."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.distributed_tangent import _p2_affine_inputs
+
+    op, pat = _pattern("P2", dims)
+    d = _p2_affine_inputs(pat)
+    rng = np.random.default_rng(n_q)
+    n_el = int(pat.overlap_elements.size)
+    lam = rng.dirichlet(np.ones(4), n_q) if n_q != 11 else d["bary"].cpu().numpy()
+    jinv = d["jinv"].cpu().numpy().reshape(n_el, 3, 3)
+    gl = np.concatenate([-jinv.sum(axis=1, keepdims=True), jinv], axis=1)  # (n_el, 4, 3)
+    g = np.empty((n_el, n_q, 10, 3))
+    for a in range(4):
+        g[:, :, a] = (4.0 * lam[None, :, a, None] - 1.0) * gl[:, None, a]
+    for a, (i, j) in zip(range(4, 10), ((0, 1), (1, 2), (0, 2), (1, 3), (2, 3), (0, 3))):
+        g[:, :, a] = 4.0 * (lam[None, :, i, None] * gl[:, None, j] + lam[None, :, j, None] * gl[:, None, i])
+    dphi = [np.ascontiguousarray(g[..., z].reshape(-1, 10)) for z in range(3)]
+    u = magnitude * rng.standard_normal(int(pat.overlap_global_dofs.size)) * 10.0 ** rng.uniform(-3.0, 0.0)
+    dof = pat.overlap_element_dof_lids
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a), device="cuda")  # noqa: E731
+    bary = dev(lam)
+
+    def strain(u):
+        E = torch.full((n_el * n_q, 6), -7.0, dtype=torch.float64, device="cuda")
+        ud = dev(u)
+        _lib.call("ssp_assemble_overlap_strain_3d_p2_affine", _lib.ptr(d["jinv"]), _lib.ptr(bary), _lib.ptr(ud), u.size,
+                  _lib.ptr(d["dof_lids"]), n_el * n_q, n_el, n_q, _lib.ptr(E), _lib.stream_handle())
+        return E.cpu().numpy()
+
+    E = strain(u)
+    assert rel_err(E, oracle.strain_3d(*dphi, u, dof, n_q)) <= TOL
+    S = magnitude * rng.standard_normal((n_el * n_q, 6)) * 10.0 ** rng.uniform(-2.0, 0.0, (n_el * n_q, 1))
+    w = rng.uniform(-0.2, 1.0, n_el * n_q)
+    rows = d["elem_row"].cpu().numpy()
+    n_rows = int(pat.local_matrix_pattern.shape[0])
+
+    def force(S):
+        F = torch.full((n_rows,), -7.0, dtype=torch.float64, device="cuda")
+        Sd, wd = dev(S), dev(w)
+        _lib.call("ssp_assemble_force_element_p2_affine", _lib.ptr(d["jinv"]), _lib.ptr(bary), _lib.ptr(Sd), _lib.ptr(wd),
+                  _lib.ptr(d["elem_row"]), n_el, n_q, n_rows, _lib.ptr(F), _lib.stream_handle())
+        return F.cpu().numpy()
+
+    bt = ((0, 3, 5), (3, 1, 4), (5, 4, 2))
+    want = np.zeros(n_rows)
+    ws = (w[:, None] * S).reshape(n_el, n_q, 6)
+    for c in range(3):
+        f = sum(np.einsum("eqa,eq->ea", g[..., z], ws[..., bt[c][z]]) for z in range(3))
+        r = rows.reshape(n_el, 10, 3)[:, :, c]
+        np.add.at(want, r[r >= 0], f[r >= 0])
+    F = force(S)
+    assert rel_err(F, want) <= TOL
+    # not finite: the elements of one dof, the rows of one element
+    u2 = u.copy()
+    u2[dof[0, 4]] = float("nan")
+    hit = (dof == dof[0, 4]).any(axis=1).repeat(n_q)
+    E2 = strain(u2)
+    assert np.isnan(E2[hit]).any() and np.array_equal(E2[~hit], E[~hit])
+    S2 = S.copy()
+    S2[0, 1] = float("inf")
+    F2 = force(S2)
+    touched = np.zeros(n_rows, dtype=bool)
+    touched[rows[0][rows[0] >= 0]] = True
+    assert not np.isfinite(F2[touched]).all() and rel_err(F2[~touched], F[~touched]) <= TOL
