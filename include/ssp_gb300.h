@@ -51,6 +51,12 @@ enum ssp_status {
 int ssp_constitutive_3d_s(const double *E, const double *c_bar, const double *sin_phi, const double *shear,
                           const double *bulk, const double *lame, int n_int, double *S_out, void *stream);
 
+/* The same stresses in two passes: the elastic screen of ssp_constitutive_3d_sds_binned finishes the points it
+ * proves elastic, the others are decided and finished as a dense list.  scratch: n_int + 4 int32 (device,
+ * overwritten). */
+int ssp_constitutive_3d_s_screened(const double *E, const double *c_bar, const double *sin_phi, const double *shear,
+                                   const double *lame, int n_int, double *S_out, int32_t *scratch, void *stream);
+
 /* Replaces constitutive_problem_3d_sds_batch_c (src/slope_stability/cython/constitutive_3d_batch.h:15-25).
  * S and the consistent tangent DS; DS is symmetric (associated flow, sin(psi) = sin(phi)). */
 int ssp_constitutive_3d_sds(const double *E, const double *c_bar, const double *sin_phi, const double *shear,
@@ -380,6 +386,12 @@ int ssp_finish_values(double *values, long long nnz, const int32_t *constrained_
 
 /* dst[i] = src[idx[i]] (owned free rows of a force vector, problem.py:1008-1015). */
 int ssp_gather(const double *src, const int32_t *idx, int n, double *dst, void *stream);
+
+/* No reference counterpart.  branch_out[i] = branch[positions[i]] for i < n, and ds_out row i = ds row
+ * positions[i] (n_entries doubles) where that branch is not 0; the other rows of ds_out are not written.
+ * positions lie in [0, n_src).  The state of a subdomain's points from the owned evaluation. */
+int ssp_gather_plastic_rows(const int8_t *branch, const double *ds, const int32_t *positions, int n, int n_src,
+                            int n_entries, int8_t *branch_out, double *ds_out, void *stream);
 
 /* 1 if host_ptr is pinned, device-mapped host memory (cudaHostAlloc / cudaMallocHost memory, or
  * registered memory, under unified addressing) that kernels can store to, else 0.  The copy entry

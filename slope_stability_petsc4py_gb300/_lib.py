@@ -29,6 +29,7 @@ STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA error", 3: "unsupported eleme
 
 _SIGS = {
     "ssp_constitutive_3d_s": [_vp] * 6 + [_c_int, _vp, _vp],
+    "ssp_constitutive_3d_s_screened": [_vp] * 5 + [_c_int, _vp, _vp, _vp],
     "ssp_constitutive_3d_sds": [_vp] * 6 + [_c_int, _vp, _vp, _vp],
     "ssp_constitutive_3d_branch": [_vp] * 5 + [_c_int, _vp, _vp, _vp],
     "ssp_constitutive_2d": [_vp] * 6 + [_c_int, _vp, _vp, _vp],
@@ -81,6 +82,7 @@ _SIGS = {
     "ssp_tangent_element": [_c_int, _c_int] + [_vp] * 6 + [_c_int, _c_int, _c_int, _c_ll, _vp, _c_int, _vp],
     "ssp_finish_values": [_vp, _c_ll, _vp, _c_int, _vp, _c_dbl, _vp],
     "ssp_gather": [_vp, _vp, _c_int, _vp, _vp],
+    "ssp_gather_plastic_rows": [_vp] * 3 + [_c_int] * 3 + [_vp] * 3,
     "ssp_device_status": [ctypes.POINTER(_c_int), _c_int],
     "ssp_branch_features": [_vp] * 5 + [_c_int, _vp, _vp],
     "ssp_mlp_predict": [_vp, _vp, _c_int, _c_int, _vp, _vp],
@@ -138,11 +140,11 @@ def check(status: int, what: str) -> None:
 
 # kernels each entry point launches per call (for launch accounting); callables take the args
 _KERNELS_PER_CALL = {
-    "ssp_constitutive_3d_s": 1, "ssp_constitutive_3d_sds": 1, "ssp_constitutive_3d_branch": 1,
+    "ssp_constitutive_3d_s": 1, "ssp_constitutive_3d_s_screened": 2, "ssp_constitutive_3d_sds": 1, "ssp_constitutive_3d_branch": 1,
     "ssp_constitutive_2d": 1, "ssp_reduction": 1, "ssp_geometry": 1, "ssp_assemble_overlap_strain_3d": 1,
     "ssp_assemble_overlap_strain_2d": 1, "ssp_assemble_force_3d_rows": 1, "ssp_assemble_force_element": 1,
     "ssp_assemble_tangent_values_3d_rows": 1, "ssp_assemble_tangent_values_3d_p2": 1, "ssp_tangent_element": 1,
-    "ssp_gather": 1, "ssp_tc_tf32_probe": 1, "ssp_tc_wait_probe": 1, "ssp_constitutive_sds_branch": 1,
+    "ssp_gather": 1, "ssp_gather_plastic_rows": 1, "ssp_tc_tf32_probe": 1, "ssp_tc_wait_probe": 1, "ssp_constitutive_sds_branch": 1,
     "ssp_copy_out": 1, "ssp_copy_device": 1, "ssp_copy_rows_device": 1, "ssp_copy_rows_device_share": 1, "ssp_host_writable": 0, "ssp_plastic_elements": 1, "ssp_mark_element_rows": 1,
     "ssp_copy_rows_out": 1, "ssp_copy_rows_out_share": 1,
     "ssp_assemble_overlap_strain_3d_mixed": 1, "ssp_assemble_force_element_mixed": 1, "ssp_split_f64": 1,

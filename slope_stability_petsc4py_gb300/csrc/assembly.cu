@@ -2218,6 +2218,30 @@ __global__ void gather_rows_kernel(const double *__restrict__ src, const int32_t
     if (i < n) dst[i] = src[idx[i]];
 }
 
+// branch_out[i] = branch[pos[i]], and the tangent rows of the points whose branch is not 0: one warp for 32
+// points, whose plastic rows it copies one after the other as 8-byte words.  (Gathering every row moved nine
+// tenths elastic ones that the corrections never read: 233 us for 457k points, 12 % of them plastic.)
+__global__ void gather_plastic_rows_kernel(const int8_t *__restrict__ branch, const double *__restrict__ ds,
+                                           const int32_t *__restrict__ pos, int n, int n_src, int ns2,
+                                           int8_t *__restrict__ branch_out, double *__restrict__ ds_out) {
+    const int lane = threadIdx.x & 31;
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x, i0 = i - lane;
+    int p = -1;
+    int8_t b = 0;
+    if (i < n) {
+        p = pos[i];
+        if (p < 0 || p >= n_src) flag(SSP_DEV_BAD_INDEX);
+        else b = branch[p];
+        branch_out[i] = b;
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, b != 0); m; m &= m - 1u) {
+        const int k = __ffs(m) - 1;
+        const double *src = ds + (long long)__shfl_sync(0xffffffffu, p, k) * ns2;
+        double *dst = ds_out + (i0 + k) * ns2;
+        for (int c = lane; c < ns2; c += 32) dst[c] = src[c];
+    }
+}
+
 // ---------------------------------------------------------------------------- dispatch
 
 template <int DIM, int NP, int NQ, int THREADS, bool SYM, bool CORR>
@@ -2641,6 +2665,16 @@ int ssp_gather(const double *src, const int32_t *idx, int n, double *dst, void *
 }
 
 }  // extern "C"
+
+extern "C" int ssp_gather_plastic_rows(const int8_t *branch, const double *ds, const int32_t *positions, int n, int n_src,
+                                       int n_entries, int8_t *branch_out, double *ds_out, void *stream) {
+    if (n < 0 || n_src < 0 || n_entries <= 0) return SSP_ERR_INVALID;
+    if (n == 0) return SSP_OK;
+    if (!branch || !ds || !positions || !branch_out || !ds_out) return SSP_ERR_INVALID;
+    gather_plastic_rows_kernel<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(branch, ds, positions, n, n_src, n_entries,
+                                                                               branch_out, ds_out);
+    return launch_status();
+}
 
 // The device address of pinned, device-mapped host memory (nullptr if the pointer is not such memory).
 static void *mapped_device_pointer(const void *host_ptr) {

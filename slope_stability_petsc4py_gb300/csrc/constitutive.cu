@@ -15,7 +15,7 @@
 
 #include <mutex>
 
-#include "ssp_internal.cuh"
+#include "mohr_coulomb.cuh"
 
 namespace ssp {
 
@@ -33,33 +33,6 @@ struct Principal3 {
     double t[6], sq[6];
     double I1, e1, e2, e3;
 };
-
-// sin and cos of a Lode angle theta in [0, pi/3] from their Taylor series, Horner in theta^2: the
-// first omitted terms, theta^19 / 19! and theta^20 / 20!, are below 2e-17 there, and without a
-// branch every lane of a warp runs the same instructions (a general sincos reduces its argument by
-// quadrants, and pi/4 < pi/3).  Within one ulp of the correctly rounded values on [0, pi/3].
-__device__ __forceinline__ void sincos_lode(double theta, double &s, double &c) {
-    const double z = theta * theta;
-    double ps = 1.0 / 355687428096000.0;  // 1/17!
-    ps = fma(ps, z, -1.0 / 1307674368000.0);
-    ps = fma(ps, z, 1.0 / 6227020800.0);
-    ps = fma(ps, z, -1.0 / 39916800.0);
-    ps = fma(ps, z, 1.0 / 362880.0);
-    ps = fma(ps, z, -1.0 / 5040.0);
-    ps = fma(ps, z, 1.0 / 120.0);
-    ps = fma(ps, z, -1.0 / 6.0);
-    s = fma(theta * z, ps, theta);
-    double pc = -1.0 / 6402373705728000.0;  // -1/18!
-    pc = fma(pc, z, 1.0 / 20922789888000.0);
-    pc = fma(pc, z, -1.0 / 87178291200.0);
-    pc = fma(pc, z, 1.0 / 479001600.0);
-    pc = fma(pc, z, -1.0 / 3628800.0);
-    pc = fma(pc, z, 1.0 / 40320.0);
-    pc = fma(pc, z, -1.0 / 720.0);
-    pc = fma(pc, z, 1.0 / 24.0);
-    pc = fma(pc, z, -0.5);
-    c = fma(z, pc, 1.0);
-}
 
 __device__ __forceinline__ void principal3(const double *E, Principal3 &p) {
 #pragma unroll
@@ -137,10 +110,6 @@ struct Decision3 {
     double den;  // its denominator
 };
 
-struct Mat3 {
-    double c_bar, sin_phi, shear, lame;
-};
-
 // Plastic multipliers of the three return branches (constitutive_3D_kernel.h:144-147, 213-215, 277-279).
 __device__ __forceinline__ void smooth_lam(const Principal3 &p, const Mat3 &m, double f_tr, double &lam, double &den) {
     const double sp = m.sin_phi;
@@ -208,35 +177,6 @@ __device__ __forceinline__ void finish_elastic(const double *t, double I1, const
     }
 }
 
-// Elastic screen from invariants, before any eigen-decomposition, in FP32.  With principal trial
-// strains e1 >= e2 >= e3, Q = J2/3 and Lode angle a, the trial yield function is
-//   f = 2G[(e1 - e3) + s(e1 + e3)] + 2 lambda s I1 - c_bar,
-//   (e1 - e3) + s(e1 + e3) = 2 sqrt(Q) (sqrt(3) sin a + s cos a) + 2 s I1 / 3,
-// and sqrt(3) sin a + s cos a <= sqrt(3 + s^2) for every a (Cauchy-Schwarz), so
-//   f <= bound = 2G[2 sqrt(Q) sqrt(3 + s^2) + 2 s I1 / 3] + 2 lambda s I1 - c_bar.
-// The bound is evaluated in FP32 from inputs truncated to 24 bits (J2 from differences of the
-// normal components, so no cancellation against I1): its absolute error stays below ~4e-6 of
-//   size = 2|G| (2 sqrt(Q) sqrt(3 + s^2) + 3 max|t_i|) + 2|lambda s I1| + |c_bar|.
-// A point with bound <= -1e-4 size is therefore elastic however the FP64 eigenvalues of the full
-// path round (their error is at most ~1e-8 sqrt(Q), near repeated roots): the full path's branch
-// test would say elastic too.  Such a point is finished from t and I1 in FP64 with the elastic
-// branch's own arithmetic, so S and DS are bitwise those of the full path, and it costs about a
-// dozen FP64 instructions instead of an eigen-decomposition.
-__device__ __forceinline__ bool screen_elastic(const double *E, const Mat3 &m) {
-    float t[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) t[i] = df_from_f64(E[i]).hi * (i < 3 ? 1.0f : 0.5f);
-    const float G = df_from_f64(m.shear).hi, L = df_from_f64(m.lame).hi;
-    const float s = df_from_f64(m.sin_phi).hi, c = df_from_f64(m.c_bar).hi;
-    const float d01 = t[0] - t[1], d12 = t[1] - t[2], d20 = t[2] - t[0];
-    const float J2 = (d01 * d01 + d12 * d12 + d20 * d20) * (1.0f / 6.0f) + t[3] * t[3] + t[4] * t[4] + t[5] * t[5];
-    const float I1 = t[0] + t[1] + t[2];
-    const float dev = 2.0f * sqrtf(J2 * (1.0f / 3.0f)) * sqrtf(3.0f + s * s);
-    const float bound = 2.0f * G * (dev + (2.0f / 3.0f) * s * I1) + 2.0f * L * s * I1 - c;
-    const float tmax = fmaxf(fmaxf(fabsf(t[0]), fabsf(t[1])), fmaxf(fabsf(t[2]), fmaxf(fabsf(t[3]), fmaxf(fabsf(t[4]), fabsf(t[5])))));
-    const float size = 2.0f * fabsf(G) * (dev + 3.0f * tmax) + 2.0f * fabsf(L * s * I1) + fabsf(c);
-    return bound <= -1e-4f * size;
-}
 // t (shears halved) and I1 of the trial strain, in FP64, as principal3 forms them.
 __device__ __forceinline__ void elastic_trial(const double *E, double *t, double &I1) {
 #pragma unroll
@@ -775,7 +715,7 @@ __global__ void __launch_bounds__(128) mc3d_bin_kernel(const double *__restrict_
 #pragma unroll
                 for (int k = 0; k < 36; ++k) w[lane * kDsStride + k] = ds[k];
             }
-            branch[p] = static_cast<int8_t>(kElastic);
+            if (branch) branch[p] = static_cast<int8_t>(kElastic);
         } else {
             listed = true;
         }
@@ -846,6 +786,32 @@ __global__ void __launch_bounds__(128, 5) mc3d_decide_kernel(const double *__res
         if (b == kLeft) edges[jl] = p;
         const int jr = warp_append(b == kRight, scratch + 3);
         if (b == kRight) edges[n - 1 - jr] = p;
+    }
+}
+
+// Stress only: the listed points decided and finished (the single pass paid an eigen-decomposition in nearly
+// every warp for the tenth of the points that need one: 296 us for 1.1 M points; screen and list 37 + 100).
+__global__ void __launch_bounds__(128, 5) mc3d_stress_list_kernel(const double *__restrict__ E,
+                                                                  const double *__restrict__ c_bar,
+                                                                  const double *__restrict__ sin_phi,
+                                                                  const double *__restrict__ shear,
+                                                                  const double *__restrict__ lame, int n,
+                                                                  double *__restrict__ S,
+                                                                  const int32_t *__restrict__ scratch) {
+    const int cnt = scratch[0];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
+        const int p = scratch[4 + i];
+        if (p < 0 || p >= n) {
+            flag(SSP_DEV_BAD_INDEX);
+            continue;
+        }
+        double e[6], s[6];
+        load6(E, p, e);
+        const Mat3 m{c_bar[p], sin_phi[p], shear[p], lame[p]};
+        Principal3 pr;
+        principal3(e, pr);
+        finish3<false>(pr, decide3(pr, m), m, s, nullptr);
+        store6(S, p, s);
     }
 }
 
@@ -1268,6 +1234,23 @@ int ssp_constitutive_3d_s(const double *E, const double *c_bar, const double *si
     if (!E || !c_bar || !sin_phi || !shear || !lame || !S_out) return SSP_ERR_INVALID;
     mc3d_kernel<false><<<grid_for(n_int, 128), 128, 0, as_stream(stream)>>>(E, c_bar, sin_phi, shear, lame, n_int, S_out,
                                                                              nullptr, nullptr);
+    return launch_status();
+}
+
+int ssp_constitutive_3d_s_screened(const double *E, const double *c_bar, const double *sin_phi, const double *shear,
+                                   const double *lame, int n_int, double *S_out, int32_t *scratch, void *stream) {
+    if (n_int < 0) return SSP_ERR_INVALID;
+    if (n_int == 0) return SSP_OK;
+    if (!E || !c_bar || !sin_phi || !shear || !lame || !S_out || !scratch) return SSP_ERR_INVALID;
+    const int rc = binned_screen(E, c_bar, sin_phi, shear, lame, n_int, S_out, nullptr, nullptr, scratch, as_stream(stream),
+                                 false);
+    if (rc != SSP_OK) return rc;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long need = (n_int + 127ll) / 128, full = (long long)sms * 5;
+    mc3d_stress_list_kernel<<<static_cast<unsigned>(need < full ? need : full), 128, 0, as_stream(stream)>>>(
+        E, c_bar, sin_phi, shear, lame, n_int, S_out, scratch);
     return launch_status();
 }
 

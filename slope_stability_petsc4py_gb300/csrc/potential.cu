@@ -15,11 +15,15 @@
 // The sum is deterministic: a fixed grid of at most SSP_POTENTIAL_PARTIALS blocks writes one
 // partial each (in-block tree), and one block adds the partials in a fixed tree.
 
-#include "ssp_internal.cuh"
+#include "mohr_coulomb.cuh"
 
 namespace {
 
-constexpr int kBlock = 256;
+constexpr int kBlock = 128;
+// five blocks on each of 152 SMs: long enough runs of points that a warp's queue mostly empties as full warps
+// (1,024 blocks of 256 threads left 18 of 32 lanes on average in a pass of their own: 196 us against 164)
+constexpr int kMaxBlocks = 760;
+static_assert(kMaxBlocks <= SSP_POTENTIAL_PARTIALS, "one partial sum a block");
 
 __device__ __forceinline__ double np_maximum(double floor_value, double x) {
     // np.maximum(floor, x): NaN propagates
@@ -41,15 +45,14 @@ __device__ __forceinline__ double safe_denominator(double d) {
 __device__ __forceinline__ int mc_potential(double e1, double e2, double e3, double tr, double c, double s, double G,
                                             double K, double L, double d_s, double d_l, double d_r, double &psi) {
     const double f_tr = 2.0 * G * ((1.0 + s) * e1 - (1.0 - s) * e3) + 2.0 * (L * s) * tr - c;
-    const double g_sl = (e1 - e2) / np_maximum(1.0e-15, 1.0 + s);
-    const double g_sr = (e2 - e3) / np_maximum(1.0e-15, 1.0 - s);
-    const double g_la = (e1 + e2 - 2.0 * e3) / np_maximum(1.0e-15, 3.0 - s);
-    const double g_ra = (2.0 * e1 - e2 - e3) / np_maximum(1.0e-15, 3.0 + s);
     const double vol = 0.5 * L * tr * tr;
     if (f_tr <= 0.0) {
         psi = vol + G * (e1 * e1 + e2 * e2 + e3 * e3);
         return 0;
     }
+    // each bound where its branch is tested: an FP64 division costs as much as five multiply-adds here
+    const double g_sl = (e1 - e2) / np_maximum(1.0e-15, 1.0 + s);
+    const double g_sr = (e2 - e3) / np_maximum(1.0e-15, 1.0 - s);
     const double l_s = f_tr / safe_denominator(d_s);
     if (l_s <= g_sl && l_s <= g_sr) {  // lambda_s <= np.minimum(g_sl, g_sr), NaN-failing
         psi = vol + G * (e1 * e1 + e2 * e2 + e3 * e3) - 0.5 * d_s * (l_s * l_s);
@@ -58,7 +61,7 @@ __device__ __forceinline__ int mc_potential(double e1, double e2, double e3, dou
     const double lin = 2.0 * L * s * tr - c;
     if (g_sl < g_sr) {
         const double l_l = (G * ((1.0 + s) * (e1 + e2) - 2.0 * (1.0 - s) * e3) + lin) / safe_denominator(d_l);
-        if (l_l >= g_sl && l_l <= g_la) {
+        if (l_l >= g_sl && l_l <= (e1 + e2 - 2.0 * e3) / np_maximum(1.0e-15, 3.0 - s)) {
             const double h = e1 + e2;
             psi = vol + G * (e3 * e3 + 0.5 * (h * h)) - 0.5 * d_l * (l_l * l_l);
             return 2;
@@ -66,7 +69,7 @@ __device__ __forceinline__ int mc_potential(double e1, double e2, double e3, dou
     }
     if (g_sl > g_sr) {
         const double l_r = (G * (2.0 * (1.0 + s) * e1 - (1.0 - s) * (e2 + e3)) + lin) / safe_denominator(d_r);
-        if (l_r >= g_sr && l_r <= g_ra) {
+        if (l_r >= g_sr && l_r <= (2.0 * e1 - e2 - e3) / np_maximum(1.0e-15, 3.0 + s)) {
             const double h = e2 + e3;
             psi = vol + G * (e1 * e1 + 0.5 * (h * h)) - 0.5 * d_r * (l_r * l_r);
             return 3;
@@ -87,20 +90,24 @@ __device__ __forceinline__ int point_potential(const double *__restrict__ E, dou
         const double I1 = e11 + e22 + e33;
         const double I2 = e11 * e22 + e11 * e33 + e22 * e33 - r3 * r3 - r4 * r4 - r5 * r5;
         const double I3 = e11 * e22 * e33 - e33 * r3 * r3 - e22 * r4 * r4 - e11 * r5 * r5 + 2.0 * r3 * r4 * r5;
-        const double Q = np_maximum(0.0, (I1 * I1 - 3.0 * I2) / 9.0);
-        const double R = (-2.0 * (I1 * I1 * I1) + 9.0 * I1 * I2 - 27.0 * I3) / 54.0;
+        // divisions by constants as products with the rounded reciprocals, sqrt(Q^3) as sqrt(Q) Q (an ulp)
+        const double Q = np_maximum(0.0, (I1 * I1 - 3.0 * I2) * (1.0 / 9.0));
+        const double R = (-2.0 * (I1 * I1 * I1) + 9.0 * I1 * I2 - 27.0 * I3) * (1.0 / 54.0);
+        const double rq = sqrt(Q);
         double theta = 0.0;
         if (Q > 0.0) {
-            double t = R / np_maximum(1.0e-15, sqrt(Q * Q * Q));
+            double t = R / np_maximum(1.0e-15, rq * Q);
             t = t < -1.0 ? -1.0 : (t > 1.0 ? 1.0 : t);
-            theta = acos(t) / 3.0;
+            theta = acos(t) * (1.0 / 3.0);
         }
-        const double rq = sqrt(Q);
-        const double third = I1 / 3.0;
-        const double two_pi_3 = 2.0 * 3.14159265358979323846 / 3.0;
-        const double e1 = -2.0 * rq * cos(theta + two_pi_3) + third;
-        const double e2 = -2.0 * rq * cos(theta - two_pi_3) + third;
-        const double e3 = -2.0 * rq * cos(theta) + third;
+        const double third = I1 * (1.0 / 3.0);
+        // cos(theta +- 2 pi / 3) from one sine and cosine
+        double st, ct;
+        ssp::sincos_lode(theta, st, ct);
+        const double rs = 1.7320508075688772 * st;
+        const double e1 = rq * (ct + rs) + third;
+        const double e2 = rq * (ct - rs) + third;
+        const double e3 = -2.0 * rq * ct + third;
         const double d_s = 4.0 * L * s2 + 4.0 * G * (1.0 + s2);
         const double d_l = 4.0 * L * s2 + G * (1.0 + s) * (1.0 + s) + 2.0 * G * (1.0 - s) * (1.0 - s);
         const double d_r = 4.0 * L * s2 + 2.0 * G * (1.0 + s) * (1.0 + s) + G * (1.0 - s) * (1.0 - s);
@@ -138,27 +145,99 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
     return v;  // valid in thread 0
 }
 
+// 3D: the FP32 elastic screen of the return mapping (screen_elastic, whose bound holds for every Lode angle)
+// settles the points it proves elastic from two invariants: e1^2 + e2^2 + e3^2 = I1^2 - 2 I2, the sum of the
+// squared tensor entries.  The others queue up in shared memory, 32 to a warp, and take the eigenvalues'
+// acos and square root as full warps: with a tenth of the points listed nearly every warp paid for them
+// (613 us for 1.1 M points, now 160).  A warp's queue fills in point order, so the sums are the same in
+// every run.
 template <int DIM>
-__global__ void __launch_bounds__(kBlock) potential_kernel(const double *__restrict__ E, const double *__restrict__ c_bar,
+__global__ void __launch_bounds__(kBlock, 5) potential_kernel(const double *__restrict__ E, const double *__restrict__ c_bar,
                                                            const double *__restrict__ sin_phi,
                                                            const double *__restrict__ shear,
                                                            const double *__restrict__ bulk,
                                                            const double *__restrict__ lame,
                                                            const double *__restrict__ weight, int n, double *psi_out,
-                                                           int8_t *branch_out, double *partial) {
+                                                           int8_t *branch_out, double *partial, int vec) {
     __shared__ double red[kBlock / 32];
+    __shared__ int queue[kBlock / 32][64], left[kBlock / 32];
+    int mine = -1;
     constexpr int NS = DIM == 3 ? 6 : 3;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double acc = 0.0;
-    for (long long p = (long long)blockIdx.x * kBlock + threadIdx.x; p < n; p += (long long)gridDim.x * kBlock) {
-        double e[NS];
+    auto load = [&](long long p, double *e) {
+        if (DIM == 3 && vec) {  // 16-byte loads where E is aligned
+            const double2 *e2 = reinterpret_cast<const double2 *>(E + 6 * p);
 #pragma unroll
-        for (int k = 0; k < NS; ++k) e[k] = E[p * NS + k];
-        double psi;
-        const int b = point_potential<DIM>(e, c_bar[p], sin_phi[p], shear[p], bulk[p], lame[p], psi);
+            for (int k = 0; k < 3; ++k) {
+                const double2 v = e2[k];
+                e[2 * k] = v.x;
+                e[2 * k + 1] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NS; ++k) e[k] = E[p * NS + k];
+        }
+    };
+    auto settle = [&](long long p, double psi, int b) {
         if (psi_out) psi_out[p] = psi;
         if (branch_out) branch_out[p] = (int8_t)b;
         if (weight) acc += weight[p] * psi;
+    };
+    auto full = [&](long long p) {
+        double e[NS], psi;
+        load(p, e);
+        const int b = point_potential<DIM>(e, c_bar[p], sin_phi[p], shear[p], bulk[p], lame[p], psi);
+        settle(p, psi, b);
+    };
+    int queued = 0;  // the same in every lane
+    for (long long p0 = (long long)blockIdx.x * kBlock + 32 * warp; p0 < n; p0 += (long long)gridDim.x * kBlock) {
+        const long long p = p0 + lane;
+        if (DIM == 2) {
+            if (p < n) full(p);
+            continue;
+        }
+        bool listed = false;
+        if (p < n) {
+            double e[6];
+            load(p, e);
+            const ssp::Mat3 m{c_bar[p], sin_phi[p], shear[p], lame[p]};
+            const double t[6] = {e[0], e[1], e[2], 2.0 * e[3], 2.0 * e[4], 2.0 * e[5]};  // halved by the screen
+            if (ssp::screen_elastic(t, m)) {
+                const double tr = e[0] + e[1] + e[2];
+                const double sq = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + 2.0 * (e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
+                settle(p, 0.5 * m.lame * tr * tr + m.shear * sq, 0);
+            } else {
+                listed = true;
+            }
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, listed);
+        if (listed) queue[warp][queued + __popc(mask & ((1u << lane) - 1u))] = static_cast<int>(p);
+        queued += __popc(mask);
+        __syncwarp();
+        if (queued >= 32) {
+            const int q = queue[warp][lane];
+            const int rest = lane + 32 < queued ? queue[warp][lane + 32] : 0;
+            __syncwarp();
+            queue[warp][lane] = rest;
+            queued -= 32;
+            __syncwarp();
+            full(q);
+        }
     }
+    // what the block's warps have left, in warp order, again as full warps
+    if (lane == 0) left[warp] = queued;
+    __syncthreads();
+    int k = threadIdx.x;
+#pragma unroll 1
+    for (int v = 0; v < kBlock / 32; ++v) {
+        if (k >= 0 && k < left[v]) {
+            mine = queue[v][k];
+            break;
+        }
+        k -= left[v];
+    }
+    if (mine >= 0) full(mine);
     if (!partial) return;
     acc = block_sum(acc, red);
     if (threadIdx.x == 0) partial[blockIdx.x] = acc;
@@ -186,19 +265,18 @@ int ssp_potential_energy(int dim, const double *E, const double *c_bar, const do
     if (n_int < 0) return SSP_ERR_INVALID;
     if (total_out && (!weight || !partial)) return SSP_ERR_INVALID;
     cudaStream_t st = as_stream(stream);
-    const int blocks = n_int == 0 ? 0 : (int)((n_int + kBlock - 1) / kBlock < SSP_POTENTIAL_PARTIALS
-                                                  ? (n_int + kBlock - 1) / kBlock
-                                                  : SSP_POTENTIAL_PARTIALS);
+    const int blocks = n_int == 0 ? 0 : (int)((n_int + kBlock - 1) / kBlock < kMaxBlocks ? (n_int + kBlock - 1) / kBlock : kMaxBlocks);
     if (blocks > 0) {
         if (!E || !c_bar || !sin_phi || !shear || !bulk || !lame) return SSP_ERR_INVALID;
         const double *w = total_out ? weight : nullptr;
         double *part = total_out ? partial : nullptr;
+        const int vec = (reinterpret_cast<uintptr_t>(E) & 15u) == 0;
         if (dim == 3)
             potential_kernel<3><<<blocks, kBlock, 0, st>>>(E, c_bar, sin_phi, shear, bulk, lame, w, n_int, psi_out,
-                                                           branch_out, part);
+                                                           branch_out, part, vec);
         else
             potential_kernel<2><<<blocks, kBlock, 0, st>>>(E, c_bar, sin_phi, shear, bulk, lame, w, n_int, psi_out,
-                                                           branch_out, part);
+                                                           branch_out, part, vec);
     }
     if (total_out) potential_total_kernel<<<1, 1024, 0, st>>>(partial, blocks, total_out);
     return launch_status();

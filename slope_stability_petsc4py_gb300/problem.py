@@ -52,6 +52,9 @@ except Exception:  # pragma: no cover
 _OWNED_MODES = {"overlap", "unique_exchange", "unique", "unique_gather", "no_overlap", "partitioned"}
 # (dim, nodes per element) with a mixed-precision plastic-correction kernel (CUDA-core warp kernel
 # for the triangles and P1/P2 tets, tcgen05 tensor-core kernel for P4 tets)
+# points from which stress-only evaluations screen first and decide a dense list (two launches and a memset
+# more; one pass below, where a launch costs more than the eigen-decompositions it saves)
+SCREENED_STRESS_POINTS = 16384
 MIXED_TANGENT_ELEMENTS = {(2, 3), (2, 6), (2, 15), (3, 4), (3, 10), (3, 35)}
 
 
@@ -516,6 +519,12 @@ class ConstitutiveOperator:
             _lib.call("ssp_constitutive_sds_branch", pat.dim, _lib.ptr(E), _lib.ptr(self._owned_overlap_c_bar),
                       _lib.ptr(self._owned_overlap_sin_phi), _lib.ptr(d["shear"]), _lib.ptr(d["lame"]), n, _lib.ptr(S),
                       _lib.ptr(DS), _lib.ptr(branch), st)
+        elif pat.dim == 3 and n >= SCREENED_STRESS_POINTS:
+            if self._scratch is None or self._scratch.numel() < n + 4:
+                self._scratch = t.empty(3 * n + 12, dtype=t.int32, device="cuda")
+            _lib.call("ssp_constitutive_3d_s_screened", _lib.ptr(E), _lib.ptr(self._owned_overlap_c_bar),
+                      _lib.ptr(self._owned_overlap_sin_phi), _lib.ptr(d["shear"]), _lib.ptr(d["lame"]), n, _lib.ptr(S),
+                      _lib.ptr(self._scratch), st)
         elif pat.dim == 3:
             _lib.call("ssp_constitutive_3d_s", *args, _lib.ptr(S), st)
         else:
@@ -879,23 +888,29 @@ class ConstitutiveOperator:
             raise ValueError("BDDC subdomain pattern not configured")
         return pattern
 
-    def _bddc_local_DS(self, complete: bool = True):
+    def _bddc_positions(self, pattern):
+        """The subdomain's points in the owned evaluation (int64 and int32, device), or None where the
+        pattern was prepared without them."""
+        if int(pattern.overlap_local_positions.size) != int(pattern.local_int_indices.size):
+            return None
+        d = pattern.device
+        if "overlap_positions" not in d:
+            t = _lib.torch()
+            d["overlap_positions"] = t.as_tensor(pattern.overlap_local_positions.astype(np.int64), device="cuda")
+            d["overlap_positions32"] = d["overlap_positions"].to(t.int32)
+        return d["overlap_positions"], d["overlap_positions32"]
+
+    def _bddc_local_DS(self):
         """DS rows of the subdomain's points as an AoS CUDA tensor (n_local, n_strain^2): gathered
-        from the owned (overlap) evaluation, else taken from a global ``DS`` (problem.py:1646-1656).
-        complete=False: the elastic points' rows may be left as the return mapping left them (the
-        plastic corrections read only the plastic points' rows)."""
-        t = _lib.require_cuda()
+        from the owned (overlap) evaluation, else taken from a global ``DS`` (problem.py:1646-1656)."""
+        t = _lib.torch()
         pattern = self._bddc_pattern()
         if self._DS_aos is not None:
-            if complete:
-                self._complete_ds()
-            if int(pattern.overlap_local_positions.size) != int(pattern.local_int_indices.size):
-                raise RuntimeError("BDDC overlap-local integration-point map is incomplete")
-            pos = pattern.device.get("overlap_positions")
+            self._complete_ds()
+            pos = self._bddc_positions(pattern)
             if pos is None:
-                pos = pattern.device["overlap_positions"] = t.as_tensor(
-                    pattern.overlap_local_positions.astype(np.int64), device="cuda")
-            return self._DS_aos.index_select(0, pos)
+                raise RuntimeError("BDDC overlap-local integration-point map is incomplete")
+            return self._DS_aos.index_select(0, pos[0])
         if self.DS is None:
             raise ValueError("Tangent DS not computed")
         ds = np.asarray(self.DS, dtype=np.float64)[:, pattern.local_int_indices]
@@ -960,46 +975,72 @@ class ConstitutiveOperator:
             return False
         if "predictor_ok" not in self._bddc:
             t = _lib.torch()
-            d, pos = pattern.device, pattern.device.get("overlap_positions")
+            d, pos = pattern.device, self._bddc_positions(pattern)
             ok = pos is not None and "shear" in d and "lame" in d
             if ok:
-                ok = bool(t.equal(self._dev["shear"].index_select(0, pos), d["shear"])) and bool(
-                    t.equal(self._dev["lame"].index_select(0, pos), d["lame"]))
+                ok = bool(t.equal(self._dev["shear"].index_select(0, pos[0]), d["shear"])) and bool(
+                    t.equal(self._dev["lame"].index_select(0, pos[0]), d["lame"]))
             self._bddc["predictor_ok"] = ok
         return self._bddc["predictor_ok"]
+
+    def _bddc_jinv(self, pattern):
+        """J^{-1} of the subdomain's elements where its corrections may take the moment form: straight-sided
+        P2 tetrahedra, the subdomain's elements whole elements of the owned pattern with the same
+        gradients (checked once per pattern); else None."""
+        if "jinv" not in self._bddc:
+            t = _lib.torch()
+            own, d, jinv = self._require_pattern(), pattern.device, None
+            if pattern.dim == 3 and pattern.n_p == 10 and _p2_affine_inputs(own) is not None:
+                pos = self._bddc_positions(pattern)[0].reshape(-1, pattern.n_q)
+                el = pos[:, 0] // pattern.n_q
+                whole = el[:, None] * pattern.n_q + t.arange(pattern.n_q, device="cuda")
+                if t.equal(pos, whole) and all(t.equal(own.device[k].index_select(0, pos.reshape(-1)), d[k])
+                                               for k in ("dphi1", "dphi2", "dphi3")):
+                    jinv = own.device["jinv"].index_select(0, el)
+            self._bddc["jinv"] = jinv
+        return self._bddc["jinv"]
 
     def _bddc_tangent_into(self, values, r=None):
         """Subdomain tangent values into ``values``; with r, the regularised (1-r) K + r K_el.
 
         When the elastic predictor applies (_bddc_predictor_ok), the elastic subdomain values plus
-        the plastic elements' corrections B^T w (DS - D_el) B scaled by (1-r) -- the owned path's
-        assembly, FP64 or mixed-precision by ``tangent_form``; otherwise the full element contraction
-        of every subdomain point (problem.py:1710-1857)."""
+        the plastic elements' corrections B^T w (DS - D_el) B scaled by (1-r), in the plain form's
+        arithmetic whatever ``tangent_form``; otherwise the full element contraction of every
+        subdomain point (problem.py:1710-1857)."""
         from .bddc import bddc_tangent_values_device
 
         pattern = self._bddc_pattern()
         d, st = pattern.device, _lib.stream_handle()
         n_el = int(pattern.local_elements.size)
-        predictor = bool(n_el) and self._bddc_predictor_ok(pattern)
-        ds = self._bddc_local_DS(complete=not predictor)
-        if predictor:
+        if bool(n_el) and self._bddc_predictor_ok(pattern):
             t = _lib.torch()
-            branch = self._branch.index_select(0, d["overlap_positions"])
+            n = int(pattern.n_local_int)
+            branch = t.empty(n, dtype=t.int8, device="cuda")
+            ds = t.empty((n, pattern.n_strain ** 2), dtype=t.float64, device="cuda")  # plastic rows only
             if "plastic_list" not in self._bddc:
                 self._bddc["plastic_list"] = (t.empty(n_el, dtype=t.int32, device="cuda"),
                                               t.empty(1, dtype=t.int32, device="cuda"))
             elist, ecount = self._bddc["plastic_list"]
-            values.copy_(d["elastic_values"])
+            _lib.call("ssp_gather_plastic_rows", _lib.ptr(self._branch), _lib.ptr(self._DS_aos),
+                      _lib.ptr(d["overlap_positions32"]), n, int(self._branch.numel()), pattern.n_strain ** 2,
+                      _lib.ptr(branch), _lib.ptr(ds), st)
+            _lib.call("ssp_copy_device", _lib.ptr(d["elastic_values"]), int(values.numel()), _lib.ptr(values), st)
             _lib.call("ssp_plastic_elements", _lib.ptr(branch), n_el, pattern.n_q, _lib.ptr(elist), _lib.ptr(ecount), st)
-            mixed = self.tangent_form == "mixed" and (pattern.dim, pattern.n_p) in MIXED_TANGENT_ELEMENTS
-            entry = "ssp_tangent_plastic_correction_mixed" if mixed else "ssp_tangent_plastic_correction"
-            _lib.call(entry, pattern.dim, _lib.ptr(d["dphi1"]), _lib.ptr(d["dphi2"]),
-                      _lib.ptr(d["dphi3"]) if pattern.dim == 3 else None, _lib.ptr(ds), _lib.ptr(d["weight"]),
-                      _lib.ptr(branch), _lib.ptr(d["shear"]), _lib.ptr(d["lame"]), _lib.ptr(d["scatter_map"]), n_el,
-                      pattern.n_p, pattern.n_q, pattern.nnz, 1.0 if r is None else 1.0 - float(r), _lib.ptr(values),
-                      _lib.ptr(elist), _lib.ptr(ecount), st)
+            scale = 1.0 if r is None else 1.0 - float(r)
+            jinv = self._bddc_jinv(pattern)
+            if jinv is not None:
+                _lib.call("ssp_tangent_plastic_correction_p2_moments", _lib.ptr(jinv),
+                          _lib.ptr(self._require_pattern().device["bary"]), _lib.ptr(ds), _lib.ptr(d["weight"]),
+                          _lib.ptr(branch), _lib.ptr(d["shear"]), _lib.ptr(d["lame"]), _lib.ptr(d["scatter_map"]), n_el,
+                          pattern.n_q, pattern.nnz, scale, _lib.ptr(values), _lib.ptr(elist), _lib.ptr(ecount), st)
+            else:
+                _lib.call("ssp_tangent_plastic_correction", pattern.dim, _lib.ptr(d["dphi1"]), _lib.ptr(d["dphi2"]),
+                          _lib.ptr(d["dphi3"]) if pattern.dim == 3 else None, _lib.ptr(ds), _lib.ptr(d["weight"]),
+                          _lib.ptr(branch), _lib.ptr(d["shear"]), _lib.ptr(d["lame"]), _lib.ptr(d["scatter_map"]), n_el,
+                          pattern.n_p, pattern.n_q, pattern.nnz, scale, _lib.ptr(values), _lib.ptr(elist),
+                          _lib.ptr(ecount), st)
             return values
-        bddc_tangent_values_device(pattern, ds, out=values)
+        bddc_tangent_values_device(pattern, self._bddc_local_DS(), out=values)
         if r is not None and pattern.nnz:
             _lib.call("ssp_finish_values", _lib.ptr(values), pattern.nnz, None, 0, _lib.ptr(d["elastic_values"]),
                       float(r), st)
