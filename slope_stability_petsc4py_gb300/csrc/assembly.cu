@@ -1337,7 +1337,7 @@ __global__ void fill_elastic_ds_kernel(const int8_t *__restrict__ branch, const 
 //
 // Arithmetic: 58-bit fixed point on the integer pipe (fixed.cuh).  In FP64 the same stages are about
 // 7,500 + 260 n_pl multiply-adds an element, at 1.6 a clock and SM the whole time of the kernel
-// (0.92 of the FP64 rate).  In fixed point the products are 3 x (210 n_pl + 54 x 40 + 30 x 90) IMADs and
+// (0.92 of the FP64 rate).  In fixed point the products are 3 x (210 n_pl + 3 x 24 x 30 + 3 x 30 x 30) IMADs and
 // the sums and the K entries integer additions.  One exponent per element for each of the tangents, the
 // weights and the gradients; DS and D_el are subtracted as 60-bit integers; dD, the gradients and M are
 // brought to 57 or 58 bits by the element's largest.  The element matrix is within 2 to 6 x 10^-16 of its
@@ -2286,8 +2286,9 @@ int launch_element_warp(const ElemArgs &a, cudaStream_t st) {
 
 template <bool SYM, bool CORR>
 int dispatch_element(int dim, int n_p, int n_q, const ElemArgs &a, cudaStream_t st) {
-    if (dim == 3 && n_p == 10 && n_q == 11) return launch_element_warp<3, 10, 11, SYM, CORR>(a, st);
-    if (dim == 3 && n_p == 35 && n_q == 24) return launch_element<3, 35, 24, 256, SYM, CORR>(a, st);
+    if (dim == 3 && ((n_p == 10 && n_q == 11) || (n_p == 35 && n_q == 24)))
+        return tangent_fixed(n_p, SYM, CORR, a.d1, a.d2, a.d3, a.DS, a.w, a.emap, a.n_elem, a.nnz, a.values, a.branch,
+                             a.shear, a.lame, a.scale, a.elist, a.elist_count, st);
     if (dim == 3 && n_p == 4 && n_q == 1) return launch_element<3, 4, 1, 32, SYM, CORR>(a, st);
     if (dim == 2 && n_p == 6 && n_q == 7) return launch_element<2, 6, 7, 32, SYM, CORR>(a, st);
     if (dim == 2 && n_p == 3 && n_q == 1) return launch_element<2, 3, 1, 32, SYM, CORR>(a, st);

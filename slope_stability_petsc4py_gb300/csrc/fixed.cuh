@@ -1,9 +1,8 @@
 // 58-bit fixed-point arithmetic on the integer pipe (not part of the public C ABI).
 //
-// GB300 issues FP64 at 1.6 operations per clock and SM and 32 x 32 -> 64-bit integer multiply-adds
-// (one IMAD.WIDE each) at 57 (measured, both with eight independent chains per thread).  A sum of
-// products of about 58 significant bits takes three of the latter per term, so it runs about twelve
-// times faster there than as FP64 multiply-adds, and more exactly: FP64 rounds every step to 53 bits.
+// GB300 issues FP64 at 1.6 multiply-adds per clock and SM.  A sum of products of about 58 significant bits
+// takes three 32 x 32 -> 64-bit integer multiply-adds per term here, 22 to 29 per clock and SM (measured): five
+// times the rate, beside an idle FP64 pipe, and more exact: FP64 rounds every step to 53 bits.
 //
 // A block of values that belong together (an element's tangents, its gradients) shares one exponent, that
 // of its largest; a value is a 64-bit integer in units of the block's last place.  Operands of a product

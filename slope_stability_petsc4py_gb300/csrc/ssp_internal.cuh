@@ -68,6 +68,13 @@ int binned_decide_finish(const double *E, const double *c_bar, const double *sin
                          int32_t *scratch, const int32_t *lists, const int32_t *counts, int n_lists,
                          long long list_stride, bool compensated_ds, cudaStream_t st);
 
+// Element tangents of P2 (n_p = 10, n_q = 11) and P4 (35, 24) tetrahedra in fixed point (tangent_fixed.cu):
+// full (symmetric: every D is), or with corr the plastic correction of symmetric tangents.
+int tangent_fixed(int n_p, bool sym, bool corr, const double *d1, const double *d2, const double *d3, const double *DS,
+                  const double *w, const int32_t *emap, int n_elem, long long nnz, double *values, const int8_t *branch,
+                  const double *shear, const double *lame, double scale, const int32_t *elist,
+                  const int32_t *elist_count, cudaStream_t st);
+
 // Mixed-precision plastic-correction tangent of 3D P4 elements on the tensor cores (tangent_tc.cu).
 int correction_tc_p4(const double *d1, const double *d2, const double *d3, const double *DS, const double *w,
                      const int8_t *branch, const double *shear, const double *lame, const int32_t *emap, int n_elem,

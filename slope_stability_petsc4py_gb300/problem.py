@@ -270,12 +270,11 @@ class ConstitutiveOperator:
         self._energy_scratch = None  # block partials + total of potential_energy
         # plain form on straight-sided P2 tetrahedra: elements with at least this many plastic points
         # get their correction in moment form (ssp_tangent_plastic_correction_p2_moments), the others
-        # point by point; 0 disables it.  In fixed point the moment form is the cheaper one from two
-        # points up, and about equal at one (100,800 tetrahedra, 27 thousand of them plastic: a step of
-        # 724, 736, 735, 751, 767 us with 1 to 5).  The mixed form's moment kernel (FP32 after the FP64
-        # DS - D_el) costs less than its point-by-point kernel from one plastic point up: every plastic
-        # element by default.
-        self.moment_min_points = 2
+        # point by point (ssp_tangent_plastic_correction); 0 disables it.  100,800 tetrahedra, 27 thousand
+        # of them plastic: both kernels take 252 us with 2, 248 with 3, 356 with 0.  The mixed form's
+        # moment kernel (FP32 after the FP64 DS - D_el) costs less than its point-by-point kernel from
+        # one plastic point up: every plastic element by default.
+        self.moment_min_points = 3
         self.moment_min_points_mixed = 1
         # "plain": FP64 throughout (the drop-in, parity 1e-12 with the reference);
         # "mixed": the plastic-point tangent products in FP32 (CUDA cores for P1/P2, tensor cores

@@ -171,3 +171,52 @@ def test_p2_strain_and_force(oracle, dims, magnitude, n_q):
     touched = np.zeros(n_rows, dtype=bool)
     touched[rows[0][rows[0] >= 0]] = True
     assert not np.isfinite(F2[touched]).all() and rel_err(F2[~touched], F[~touched]) <= TOL
+
+
+@pytest.mark.parametrize("et,dims,kind,n_plastic,magnitude", [
+    ("P2", (4, 2, 2), "full", 0, 1.0), ("P2", (4, 2, 2), "symmetric", 0, 1e-150), ("P2", (4, 2, 2), "correction", 1, 1.0),
+    ("P2", (4, 2, 2), "correction", 11, 1e150), ("P4", (2, 1, 1), "full", 0, 1e6), ("P4", (2, 1, 1), "symmetric", 0, 1.0),
+    ("P4", (2, 2, 1), "correction", 1, 1e-9), ("P4", (2, 2, 1), "correction", 13, 1.0), ("P4", (2, 1, 1), "correction", 24, 1.0)])
+def test_element_tangents(oracle, et, dims, kind, n_plastic, magnitude):
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+
+    op, pat = _pattern(et, dims)
+    d, n_el, scale = pat.device, int(pat.overlap_elements.size), 0.7
+    branch, shear, lame, DS, dD = _plastic_state(op, pat, n_plastic, magnitude, n_plastic)
+    if kind == "full":
+        rng = np.random.default_rng(1)
+        DS = DS + 0.5 * shear[:, None, None] * rng.standard_normal(DS.shape)
+    dev = {k: torch.as_tensor(np.ascontiguousarray(v), device="cuda") for k, v in dict(
+        branch=branch, shear=shear, lame=lame, ds=DS.transpose(0, 2, 1).reshape(-1, 36)).items()}
+    geo = [_lib.ptr(d[k]) for k in ("dphi1", "dphi2", "dphi3")]
+
+    def run(ds):
+        vals = torch.zeros(pat.nnz, dtype=torch.float64, device="cuda")
+        if kind == "correction":
+            elist = torch.arange(n_el, dtype=torch.int32, device="cuda")
+            count = torch.tensor([n_el], dtype=torch.int32, device="cuda")
+            _lib.call("ssp_tangent_plastic_correction", 3, *geo, _lib.ptr(ds), _lib.ptr(d["weight"]), _lib.ptr(dev["branch"]),
+                      _lib.ptr(dev["shear"]), _lib.ptr(dev["lame"]), _lib.ptr(d["scatter_map"]), n_el, pat.n_p, pat.n_q,
+                      pat.nnz, scale, _lib.ptr(vals), _lib.ptr(elist), _lib.ptr(count), _lib.stream_handle())
+        else:
+            _lib.call("ssp_tangent_element", 3, int(kind == "symmetric"), *geo, _lib.ptr(ds), _lib.ptr(d["weight"]),
+                      _lib.ptr(d["scatter_map"]), n_el, pat.n_p, pat.n_q, pat.nnz, _lib.ptr(vals), 0, _lib.stream_handle())
+        return vals.cpu().numpy()
+
+    rows = scale * dD if kind == "correction" else DS
+    smap = d["scatter_map"].cpu().numpy()
+    want = oracle.tangent_scatter(3, pat.dphi1, pat.dphi2, pat.dphi3, np.ascontiguousarray(rows.transpose(0, 2, 1).reshape(-1, 36)),
+                                  pat.overlap_assembly_weight, smap, pat.n_q, pat.nnz)
+    got = run(dev["ds"])
+    assert rel_err(got, want) <= TOL
+    bad = int(np.flatnonzero(branch)[0]) if n_plastic else 3
+    ds = dev["ds"].clone()
+    ds[bad, 0] = float("inf")
+    ds[bad, 21] = float("nan")
+    out = run(ds)
+    mine = smap[bad // pat.n_q]
+    others = np.ones(pat.nnz, dtype=bool)
+    others[mine[mine >= 0]] = False
+    assert np.isnan(out[mine[mine >= 0]]).any() and rel_err(out[others], got[others]) <= TOL
