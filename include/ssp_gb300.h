@@ -261,6 +261,13 @@ int ssp_assemble_force_element(int dim, const double *dphi1, const double *dphi2
                                const double *stress, const double *weight, const int32_t *elem_row, int n_elem,
                                int n_p, int n_q, int n_rows, double *out_values, void *stream);
 
+/* The same with the stresses of a point stress_stride doubles apart (the return mappings of plane strain write
+ * four a point, of which the force takes three). */
+int ssp_assemble_force_element_strided(int dim, const double *dphi1, const double *dphi2, const double *dphi3,
+                                       const double *stress, int stress_stride, const double *weight,
+                                       const int32_t *elem_row, int n_elem, int n_p, int n_q, int n_rows,
+                                       double *out_values, void *stream);
+
 /* ------------------------------------------------------------------ tangent CSR values */
 
 /* Replaces assemble_tangent_values_3d_rows_c (src/slope_stability/cython/assemble_tangent_values_3d.h:21-38).
@@ -413,6 +420,12 @@ int ssp_copy_rows_device(const double *src, const int32_t *indptr, const uint8_t
  * with a small share it runs beside them rather than ahead of them, at a lower rate of its own. */
 int ssp_copy_rows_device_share(const double *src, const int32_t *indptr, const uint8_t *row_mark, int n_rows,
                                long long nnz, double *dst, int blocks_per_sm, void *stream);
+
+/* No reference counterpart.  The rows that a plastic correction of the listed elements writes, copied from src
+ * to dst (both device): row_mark [n_rows] zeroed, ssp_mark_element_rows, ssp_copy_rows_device_share. */
+int ssp_restore_element_rows(const double *src, const int32_t *indptr, const int32_t *elem_row, int n_elem, int n_ld,
+                             const int32_t *elem_list, const int32_t *elem_count, int n_rows, long long nnz,
+                             uint8_t *row_mark, double *dst, int blocks_per_sm, void *stream);
 
 /* dst_host[0..n) = src[0..n) written by the SMs into pinned, device-mapped host memory
  * (ssp_host_writable(dst_host) must hold, else SSP_ERR_INVALID); asynchronous on the stream.

@@ -82,6 +82,8 @@ _SIGS = {
     "ssp_tangent_element": [_c_int, _c_int] + [_vp] * 6 + [_c_int, _c_int, _c_int, _c_ll, _vp, _c_int, _vp],
     "ssp_finish_values": [_vp, _c_ll, _vp, _c_int, _vp, _c_dbl, _vp],
     "ssp_gather": [_vp, _vp, _c_int, _vp, _vp],
+    "ssp_restore_element_rows": [_vp, _vp, _vp, _c_int, _c_int, _vp, _vp, _c_int, _c_ll, _vp, _vp, _c_int, _vp],
+    "ssp_assemble_force_element_strided": [_c_int] + [_vp] * 4 + [_c_int] + [_vp] * 2 + [_c_int] * 4 + [_vp, _vp],
     "ssp_gather_plastic_rows": [_vp] * 3 + [_c_int] * 3 + [_vp] * 3,
     "ssp_device_status": [ctypes.POINTER(_c_int), _c_int],
     "ssp_branch_features": [_vp] * 5 + [_c_int, _vp, _vp],
@@ -144,7 +146,8 @@ _KERNELS_PER_CALL = {
     "ssp_constitutive_2d": 1, "ssp_reduction": 1, "ssp_geometry": 1, "ssp_assemble_overlap_strain_3d": 1,
     "ssp_assemble_overlap_strain_2d": 1, "ssp_assemble_force_3d_rows": 1, "ssp_assemble_force_element": 1,
     "ssp_assemble_tangent_values_3d_rows": 1, "ssp_assemble_tangent_values_3d_p2": 1, "ssp_tangent_element": 1,
-    "ssp_gather": 1, "ssp_gather_plastic_rows": 1, "ssp_tc_tf32_probe": 1, "ssp_tc_wait_probe": 1, "ssp_constitutive_sds_branch": 1,
+    "ssp_gather": 1, "ssp_gather_plastic_rows": 1, "ssp_restore_element_rows": 2,
+    "ssp_assemble_force_element_strided": 1, "ssp_tc_tf32_probe": 1, "ssp_tc_wait_probe": 1, "ssp_constitutive_sds_branch": 1,
     "ssp_copy_out": 1, "ssp_copy_device": 1, "ssp_copy_rows_device": 1, "ssp_copy_rows_device_share": 1, "ssp_host_writable": 0, "ssp_plastic_elements": 1, "ssp_mark_element_rows": 1,
     "ssp_copy_rows_out": 1, "ssp_copy_rows_out_share": 1,
     "ssp_assemble_overlap_strain_3d_mixed": 1, "ssp_assemble_force_element_mixed": 1, "ssp_split_f64": 1,
@@ -172,18 +175,26 @@ LAUNCHES = {"count": 0}
 TRACE = None
 
 
+_ENTRIES = {}  # name -> (ctypes function, kernels per call), looked up once
+
+
 def call(name: str, *args) -> None:
-    k = _KERNELS_PER_CALL.get(name, 0)
-    n_k = k(args) if callable(k) else k
+    entry = _ENTRIES.get(name)
+    if entry is None:
+        entry = _ENTRIES[name] = (getattr(load(), name), _KERNELS_PER_CALL.get(name, 0))
+    fn, k = entry
+    n_k = k if type(k) is int else k(args)
     if TRACE is not None and n_k:
         t = torch()
         e0, e1 = t.cuda.Event(enable_timing=True), t.cuda.Event(enable_timing=True)
         e0.record()
-        check(getattr(load(), name)(*args), name)
+        check(fn(*args), name)
         e1.record()
         TRACE.append((name, e0, e1))
     else:
-        check(getattr(load(), name)(*args), name)
+        status = fn(*args)
+        if status:
+            check(status, name)
     LAUNCHES["count"] += n_k
 
 
@@ -207,10 +218,16 @@ def raise_on_device_status() -> None:
 # ----------------------------------------------------------------------------- torch helpers
 
 
-def torch():
-    import torch as _t
+_TORCH = None
 
-    return _t
+
+def torch():
+    global _TORCH
+    if _TORCH is None:
+        import torch as _t
+
+        _TORCH = _t
+    return _TORCH
 
 
 def ptr(t) -> int | None:
@@ -225,14 +242,24 @@ def ptr(t) -> int | None:
 
 
 def stream_handle() -> int:
-    return torch().cuda.current_stream().cuda_stream
+    """Raw handle of torch's current stream on the current device (without the Stream object that
+    torch.cuda.current_stream() makes: 3 us a call, ten calls a Newton iteration)."""
+    c = torch()._C
+    return c._cuda_getCurrentRawStream(c._cuda_getDevice())
+
+
+_CUDA_SEEN = False
 
 
 def require_cuda():
+    global _CUDA_SEEN
     t = torch()
-    if not t.cuda.is_available():
-        raise SSPError("no CUDA device: the GB300 hot path has no CPU fallback")
-    load()
+    if not _CUDA_SEEN:  # is_available() asks the driver library and the environment every time
+        if not t.cuda.is_available():
+            raise SSPError("no CUDA device: the GB300 hot path has no CPU fallback")
+        load()
+        t.cuda.init()
+        _CUDA_SEEN = True
     return t
 
 

@@ -175,10 +175,9 @@ __global__ void force_rows3_kernel(const double *__restrict__ d1, const double *
 // local dof alpha or -1.  One thread per (element, local dof); atomics into F.
 template <int DIM>
 __global__ void force_element_kernel(const double *__restrict__ d1, const double *__restrict__ d2,
-                                     const double *__restrict__ d3, const double *__restrict__ S,
+                                     const double *__restrict__ d3, const double *__restrict__ S, int stride,
                                      const double *__restrict__ w, const int32_t *__restrict__ elem_row, int n_rows,
                                      int n_elem, int n_p, int n_q, double *__restrict__ F) {
-    constexpr int NS = DIM == 3 ? 6 : 3;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int nld = DIM * n_p;
     if (t >= (long long)n_elem * nld) return;
@@ -194,7 +193,7 @@ __global__ void force_element_kernel(const double *__restrict__ d1, const double
     double acc = 0.0;
     for (int q = 0; q < n_q; ++q) {
         const long long g = e * n_q + q;
-        const double *s = S + NS * g;
+        const double *s = S + stride * g;
         const double gx = d1[g * n_p + node], gy = d2[g * n_p + node];
         if (DIM == 3) {
             acc += w[g] * bt3(comp, gx, gy, d3[g * n_p + node], s);
@@ -2378,10 +2377,12 @@ int ssp_assemble_force_3d_rows(const double *dphi1, const double *dphi2, const d
     return launch_status();
 }
 
-int ssp_assemble_force_element(int dim, const double *dphi1, const double *dphi2, const double *dphi3,
-                               const double *stress, const double *weight, const int32_t *elem_row, int n_elem,
-                               int n_p, int n_q, int n_rows, double *out_values, void *stream) {
-    if ((dim != 2 && dim != 3) || n_elem < 0 || n_p <= 0 || n_q <= 0 || n_rows < 0) return SSP_ERR_INVALID;
+int ssp_assemble_force_element_strided(int dim, const double *dphi1, const double *dphi2, const double *dphi3,
+                                       const double *stress, int stress_stride, const double *weight,
+                                       const int32_t *elem_row, int n_elem, int n_p, int n_q, int n_rows,
+                                       double *out_values, void *stream) {
+    if ((dim != 2 && dim != 3) || n_elem < 0 || n_p <= 0 || n_q <= 0 || n_rows < 0 || stress_stride < (dim == 3 ? 6 : 3))
+        return SSP_ERR_INVALID;
     if (!out_values && n_rows > 0) return SSP_ERR_INVALID;
     cudaStream_t st = as_stream(stream);
     if (n_rows > 0 && cudaMemsetAsync(out_values, 0, sizeof(double) * n_rows, st) != cudaSuccess) return SSP_ERR_CUDA;
@@ -2389,12 +2390,19 @@ int ssp_assemble_force_element(int dim, const double *dphi1, const double *dphi2
     if (!dphi1 || !dphi2 || (dim == 3 && !dphi3) || !stress || !weight || !elem_row) return SSP_ERR_INVALID;
     const long long n = (long long)n_elem * dim * n_p;
     if (dim == 3)
-        force_element_kernel<3><<<grid_for(n, 128), 128, 0, st>>>(dphi1, dphi2, dphi3, stress, weight, elem_row, n_rows,
-                                                                  n_elem, n_p, n_q, out_values);
+        force_element_kernel<3><<<grid_for(n, 128), 128, 0, st>>>(dphi1, dphi2, dphi3, stress, stress_stride, weight,
+                                                                  elem_row, n_rows, n_elem, n_p, n_q, out_values);
     else
-        force_element_kernel<2><<<grid_for(n, 128), 128, 0, st>>>(dphi1, dphi2, nullptr, stress, weight, elem_row, n_rows,
-                                                                  n_elem, n_p, n_q, out_values);
+        force_element_kernel<2><<<grid_for(n, 128), 128, 0, st>>>(dphi1, dphi2, nullptr, stress, stress_stride, weight,
+                                                                  elem_row, n_rows, n_elem, n_p, n_q, out_values);
     return launch_status();
+}
+
+int ssp_assemble_force_element(int dim, const double *dphi1, const double *dphi2, const double *dphi3,
+                               const double *stress, const double *weight, const int32_t *elem_row, int n_elem,
+                               int n_p, int n_q, int n_rows, double *out_values, void *stream) {
+    return ssp_assemble_force_element_strided(dim, dphi1, dphi2, dphi3, stress, dim == 3 ? 6 : 3, weight, elem_row, n_elem,
+                                              n_p, n_q, n_rows, out_values, stream);
 }
 
 int ssp_assemble_overlap_strain_3d_p2_affine(const double *jinv, const double *bary, const double *u_overlap, int n_u,
@@ -2755,6 +2763,18 @@ int ssp_copy_rows_device(const double *src, const int32_t *indptr, const uint8_t
 int ssp_copy_rows_device_share(const double *src, const int32_t *indptr, const uint8_t *row_mark, int n_rows,
                                long long nnz, double *dst, int blocks_per_sm, void *stream) {
     if (blocks_per_sm < 1 || blocks_per_sm > 8) return SSP_ERR_INVALID;
+    return copy_rows_device(src, indptr, row_mark, n_rows, nnz, dst, blocks_per_sm, stream);
+}
+
+int ssp_restore_element_rows(const double *src, const int32_t *indptr, const int32_t *elem_row, int n_elem, int n_ld,
+                             const int32_t *elem_list, const int32_t *elem_count, int n_rows, long long nnz,
+                             uint8_t *row_mark, double *dst, int blocks_per_sm, void *stream) {
+    if (blocks_per_sm < 1 || blocks_per_sm > 8 || n_rows < 0 || nnz < 0) return SSP_ERR_INVALID;
+    if (n_rows == 0 || nnz == 0) return SSP_OK;
+    if (!row_mark) return SSP_ERR_INVALID;
+    if (cudaMemsetAsync(row_mark, 0, n_rows, as_stream(stream)) != cudaSuccess) return SSP_ERR_CUDA;
+    const int rc = ssp_mark_element_rows(elem_row, n_elem, n_ld, elem_list, elem_count, n_rows, row_mark, stream);
+    if (rc != SSP_OK) return rc;
     return copy_rows_device(src, indptr, row_mark, n_rows, nnz, dst, blocks_per_sm, stream);
 }
 

@@ -632,43 +632,61 @@ def _local_field_aos(pattern, field, rows: int):
     return _lib.to_device(np.ascontiguousarray(f.T), t.float64)
 
 
-def owned_force_device(pattern, S_aos, *, mixed: bool = False):
+def _free_element_rows(pattern):
+    """elem_row with an owned row's place among the owned free rows instead of the row (every entry
+    of elem_row is a free row or -1); made once per pattern."""
+    d = pattern.device
+    if "elem_free_row" not in d:
+        t = _lib.torch()
+        n_rows = int(pattern.local_matrix_pattern.shape[0])
+        place = t.full((n_rows + 1,), -1, dtype=t.int32, device="cuda")  # the last one for -1
+        free = d["owned_free_rows"].long()
+        place[free] = t.arange(free.numel(), dtype=t.int32, device="cuda")
+        d["elem_free_row"] = place[d["elem_row"].long()]
+    return d["elem_free_row"]
+
+
+def owned_force_device(pattern, S_aos, *, mixed: bool = False, free: bool = False):
     """Owned internal force B^T (w S) on owned rows (constrained rows = 0), CUDA tensor (n_rows,);
-    mixed (3D): the compensated FP32 kernel of the mixed-precision form."""
+    with free on the owned free rows only.  S_aos: a point's stresses in a row, of which the first
+    n_strain are read.  mixed (3D): the compensated FP32 kernel of the mixed-precision form."""
     t = _lib.require_cuda()
     d = pattern.device
-    n_rows = int(pattern.local_matrix_pattern.shape[0])
+    if free:
+        rows, n_rows = _free_element_rows(pattern), int(d["owned_free_rows"].numel())
+    else:
+        rows, n_rows = d["elem_row"], int(pattern.local_matrix_pattern.shape[0])
     F = t.empty(n_rows, dtype=t.float64, device="cuda")
     if mixed and pattern.dim == 3:
         d = _mixed_inputs(pattern)
         if pattern.affine and pattern.n_p == 10:
             _lib.call("ssp_assemble_force_element_p2_affine_mixed", _lib.ptr(d["jinv_hl"]), _lib.ptr(d["bary_hl"]),
-                      _lib.ptr(d["w_hl"]), _lib.ptr(S_aos), _lib.ptr(d["elem_row"]), int(pattern.overlap_elements.size),
+                      _lib.ptr(d["w_hl"]), _lib.ptr(S_aos), _lib.ptr(rows), int(pattern.overlap_elements.size),
                       pattern.n_q, n_rows, _lib.ptr(F), _lib.stream_handle())
         elif pattern.affine:
             _lib.call("ssp_assemble_force_element_affine_mixed", _lib.ptr(d["jinv_hl"]), _lib.ptr(d["ghat_hl"]),
-                      _lib.ptr(d["w_hl"]), _lib.ptr(S_aos), _lib.ptr(d["elem_row"]), int(pattern.overlap_elements.size),
+                      _lib.ptr(d["w_hl"]), _lib.ptr(S_aos), _lib.ptr(rows), int(pattern.overlap_elements.size),
                       pattern.n_p, pattern.n_q, n_rows, _lib.ptr(F), _lib.stream_handle())
         else:
             _lib.call("ssp_assemble_force_element_mixed", _lib.ptr(d["wdphi1_hl"]), _lib.ptr(d["wdphi2_hl"]),
-                      _lib.ptr(d["wdphi3_hl"]), _lib.ptr(S_aos), _lib.ptr(d["elem_row"]),
+                      _lib.ptr(d["wdphi3_hl"]), _lib.ptr(S_aos), _lib.ptr(rows),
                       int(pattern.overlap_elements.size), pattern.n_p, pattern.n_q, n_rows, _lib.ptr(F),
                       _lib.stream_handle())
         return F
     if pattern.dim == 3 and _p2_affine_inputs(pattern) is not None:
         _lib.call("ssp_assemble_force_element_p2_affine", _lib.ptr(d["jinv"]), _lib.ptr(d["bary"]), _lib.ptr(S_aos),
-                  _lib.ptr(d["weight"]), _lib.ptr(d["elem_row"]), int(pattern.overlap_elements.size), pattern.n_q,
+                  _lib.ptr(d["weight"]), _lib.ptr(rows), int(pattern.overlap_elements.size), pattern.n_q,
                   n_rows, _lib.ptr(F), _lib.stream_handle())
         return F
     if pattern.dim == 3 and _affine_fp64_inputs(pattern) is not None:
         _lib.call("ssp_assemble_force_element_affine", _lib.ptr(d["jinv"]), _lib.ptr(d["ghat"]), _lib.ptr(S_aos),
-                  _lib.ptr(d["weight"]), _lib.ptr(d["elem_row"]), int(pattern.overlap_elements.size), pattern.n_p,
+                  _lib.ptr(d["weight"]), _lib.ptr(rows), int(pattern.overlap_elements.size), pattern.n_p,
                   pattern.n_q, n_rows, _lib.ptr(F), _lib.stream_handle())
         return F
-    _lib.call("ssp_assemble_force_element", pattern.dim, _lib.ptr(d["dphi1"]), _lib.ptr(d["dphi2"]),
-              _lib.ptr(d["dphi3"]) if pattern.dim == 3 else None, _lib.ptr(S_aos), _lib.ptr(d["weight"]),
-              _lib.ptr(d["elem_row"]), int(pattern.overlap_elements.size), pattern.n_p, pattern.n_q, n_rows,
-              _lib.ptr(F), _lib.stream_handle())
+    _lib.call("ssp_assemble_force_element_strided", pattern.dim, _lib.ptr(d["dphi1"]), _lib.ptr(d["dphi2"]),
+              _lib.ptr(d["dphi3"]) if pattern.dim == 3 else None, _lib.ptr(S_aos), int(S_aos.shape[1]),
+              _lib.ptr(d["weight"]), _lib.ptr(rows), int(pattern.overlap_elements.size), pattern.n_p, pattern.n_q,
+              n_rows, _lib.ptr(F), _lib.stream_handle())
     return F
 
 

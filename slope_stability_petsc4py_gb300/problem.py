@@ -55,6 +55,11 @@ _OWNED_MODES = {"overlap", "unique_exchange", "unique", "unique_gather", "no_ove
 # points from which stress-only evaluations screen first and decide a dense list (two launches and a memset
 # more; one pass below, where a launch costs more than the eigen-decompositions it saves)
 SCREENED_STRESS_POINTS = 16384
+# CSR values from which their starting values are staged on a second stream: its events and stream switches
+# cost the host about 40 us a step, the rows of a smaller pattern less than that to copy in line
+STAGED_NNZ = 4_000_000
+# CSR values below which the host mirror is refreshed in full on the current stream (2 MB: 12 us of the link)
+IN_LINE_HOST_VALUES = 262_144
 MIXED_TANGENT_ELEMENTS = {(2, 3), (2, 6), (2, 15), (3, 4), (3, 10), (3, 35)}
 
 
@@ -92,8 +97,17 @@ class OwnedCSRMatrix:
         """Refresh the pinned host mirror from the device values on a side stream.  rows: a device
         uint8 mark per CSR row; only the marked rows are stored (ssp_copy_rows_out), the caller
         having established that the other rows equal the mirror already.  mirror: the state the
-        mirror holds afterwards."""
+        mirror holds afterwards.  Few values are copied in full on the current stream: the side
+        stream's events and switches cost the host more than the copy takes."""
         t = _lib.torch()
+        if self.values.numel() < IN_LINE_HOST_VALUES:
+            self._host.copy_(self.values, non_blocking=True)
+            if self._copied is None:
+                self._copied = t.cuda.Event()
+            self._copied.record()
+            self.mirror = mirror
+            self._last_rows = None
+            return self
         cur = t.cuda.current_stream()
         self._copy_stream.wait_stream(cur)
         with t.cuda.stream(self._copy_stream):
@@ -551,13 +565,15 @@ class ConstitutiveOperator:
         self.time_stress_tangent.append(perf_counter() - t0)
         return self._owned_local_S
 
-    def _force_device(self):
+    def _force_device(self, free: bool = False):
         pat = self._require_pattern()
         if self._S_aos is None:
             raise ValueError("Stress tensor not computed")
         t0 = perf_counter()
-        S = self._S_aos[:, : self.n_strain].contiguous() if self._S_aos.shape[1] != self.n_strain else self._S_aos
-        F = owned_force_device(pat, S, mixed=self.tangent_form == "mixed")
+        S = self._S_aos
+        if pat.dim == 3 and S.shape[1] != self.n_strain:
+            S = S[:, : self.n_strain].contiguous()
+        F = owned_force_device(pat, S, mixed=self.tangent_form == "mixed", free=free)
         self.time_local_force_assembly.append(perf_counter() - t0)
         return F
 
@@ -572,12 +588,7 @@ class ConstitutiveOperator:
 
     def build_F_free_local(self):
         t0 = perf_counter()
-        F = self._force_device()
-        t = _lib.torch()
-        idx = self.owned_tangent_pattern.device["owned_free_rows"]
-        free = t.empty(idx.numel(), dtype=t.float64, device="cuda")
-        _lib.call("ssp_gather", _lib.ptr(F), _lib.ptr(idx), int(idx.numel()), _lib.ptr(free), _lib.stream_handle())
-        out = self._to_host(free)
+        out = self._to_host(self._force_device(free=True))
         self.time_build_F.append(perf_counter() - t0)
         return out
 
@@ -659,11 +670,8 @@ class ConstitutiveOperator:
         pat = self._require_pattern()
         dv, d = self._dev, pat.device
         n_rows, n_el = int(pat.local_matrix_pattern.shape[0]), int(pat.overlap_elements.size)
-        mark, st = dv["restore_mark"], _lib.stream_handle()  # allocated with the plastic lists
-        mark.zero_()
+        mark = dv["restore_mark"]  # allocated with the plastic lists
         elist, ecount = dv["plastic_lists"][kind][last["list"]]
-        _lib.call("ssp_mark_element_rows", _lib.ptr(d["elem_row"]), n_el, pat.dim * pat.n_p, _lib.ptr(elist),
-                  _lib.ptr(ecount), n_rows, _lib.ptr(mark), st)
         # staged beside the strain and return mapping: with many points per CSR entry (P2) those run
         # long enough to hide a slower copy on a small share of the SMs (two blocks per SM); with few
         # (P4) they are short, and shares of 4 to 8 blocks per SM measured the same, so the copy
@@ -673,8 +681,9 @@ class ConstitutiveOperator:
         share = 8
         if staged and self.return_mapping in ("binned", "previous"):
             share = self.restore_share or (2 if pat.n_local_int >= 0.01 * pat.nnz else 8)
-        _lib.call("ssp_copy_rows_device_share", _lib.ptr(start), _lib.ptr(d["indptr"]), _lib.ptr(mark), n_rows,
-                  int(values.numel()), _lib.ptr(values), int(share), st)
+        _lib.call("ssp_restore_element_rows", _lib.ptr(start), _lib.ptr(d["indptr"]), _lib.ptr(d["elem_row"]), n_el,
+                  pat.dim * pat.n_p, _lib.ptr(elist), _lib.ptr(ecount), n_rows, int(values.numel()), _lib.ptr(mark),
+                  _lib.ptr(values), int(share), _lib.stream_handle())
 
     def _stage_values(self, r):
         """Issue the copy of the regularised tangent's starting values into its values array on the
@@ -683,7 +692,7 @@ class ConstitutiveOperator:
         the tangent assembly waits for it instead of copying."""
         self._drain_staged()
         if not self.stage_values or self.owned_tangent_pattern is None or \
-                self.owned_tangent_kernel not in ("rows", "legacy"):
+                self.owned_tangent_kernel not in ("rows", "legacy") or self.owned_tangent_pattern.nnz < STAGED_NNZ:
             return
         t = _lib.require_cuda()
         pat = self.owned_tangent_pattern
@@ -841,6 +850,8 @@ class ConstitutiveOperator:
         rows of that build's and the current build's plastic elements (every other entry equals the start
         values in both).  None: refresh everything."""
         if not self.incremental_host_copy or info["prev"] is None or mat.mirror != (info["key"], info["prev_no"]):
+            return None
+        if mat.values.numel() < IN_LINE_HOST_VALUES:
             return None
         if not _lib.host_writable(mat._host.data_ptr()):
             return None
