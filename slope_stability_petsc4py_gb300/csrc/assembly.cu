@@ -422,6 +422,10 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
 // read J^{-1} once per element (72 bytes) and the table from shared memory.  Used for P1 and P4
 // (P2 has the barycentric form above).
 
+// Elements of more than four nodes take the fixed-point kernels (affine_fixed.cu) where their sums have room;
+// P1's 45 multiply-adds a point are no work to convert for.
+constexpr int kAffineSmallNodes = 4, kAffineMaxTerms = 120;
+
 // Strain: grad u = G J^{-1}, G_ik = sum_{a>=1} (u_a - u_0)_i ghat_a,k(q) (the element's rigid
 // translation removed first, as the mixed form does); E the engineering strains of grad u.
 constexpr int kAffineThreads = 128;
@@ -1758,7 +1762,8 @@ __global__ void __launch_bounds__(32 * kMomWarps, 2) correction_p2_moment_kernel
             __syncwarp();
             for (int i = lane; i < 10 * 78; i += 32) {
                 const int p = i / 78;
-                W.R[p + (p > 3) + (p > 6) + (p > 8)][i - 78 * p] >>= shift_r;
+                long long &x = W.R[p + (p > 3) + (p > 6) + (p > 8)][i - 78 * p];
+                x = (x + (1ll << (shift_r - 1))) >> shift_r;
             }
         }
         __syncwarp();
@@ -2451,6 +2456,9 @@ int ssp_assemble_overlap_strain_3d_affine(const double *jinv, const double *ghat
     // the table plus the displacements of the at most 128 / n_q + 2 elements a block's points cover
     const size_t smem = sizeof(double) * (3 * (size_t)n_p * n_q + 3 * (size_t)n_p * (kAffineThreads / n_q + 2));
     if (smem > 48 * 1024) return SSP_ERR_UNSUPPORTED;
+    if (n_p > kAffineSmallNodes && n_p <= kAffineMaxTerms)
+        return strain3_affine_fixed(jinv, ghat, u_overlap, elem_dof_lids, n_u, n_elem, n_p, n_q, out_values,
+                                    as_stream(stream));
     strain3_affine_kernel<<<grid_for(n_int, kAffineThreads), kAffineThreads, smem, as_stream(stream)>>>(
         jinv, ghat, u_overlap, elem_dof_lids, n_u, n_elem, n_p, n_q, out_values);
     return launch_status();
@@ -2468,6 +2476,8 @@ int ssp_assemble_force_element_affine(const double *jinv, const double *ghat, co
     if (n_rows > 0 && cudaMemsetAsync(out_values, 0, sizeof(double) * n_rows, st) != cudaSuccess) return SSP_ERR_CUDA;
     if (n_elem == 0) return SSP_OK;
     if (!jinv || !ghat || !stress || !weight || !elem_row) return SSP_ERR_INVALID;
+    if (n_p > kAffineSmallNodes && 3 * n_q <= kAffineMaxTerms && (reinterpret_cast<uintptr_t>(stress) & 15u) == 0)
+        return force3_affine_fixed(jinv, ghat, weight, stress, elem_row, n_rows, n_elem, n_p, n_q, out_values, st);
     const long long n = (long long)n_elem * n_p;
     force3_affine_kernel<<<grid_for(n, kAffineThreads), kAffineThreads, smem, st>>>(jinv, ghat, weight, stress,
                                                                                     elem_row, n_rows, n_elem, n_p, n_q,

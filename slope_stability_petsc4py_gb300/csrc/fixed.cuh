@@ -6,9 +6,10 @@
 //
 // A block of values that belong together (an element's tangents, its gradients) shares one exponent, that
 // of its largest; a value is a 64-bit integer in units of the block's last place.  Operands of a product
-// are split into two limbs, x = h 2^29 + l with 0 <= l < 2^29; a sum of products keeps the h h and the
-// h l + l h parts in two 64-bit accumulators and drops l l (below one unit of the result per term).  With
-// |x| < 2^58 there is room for 15 terms.  Every stage is brought back to 58 bits by the block's largest
+// are split into two limbs, x = h 2^29 + l with a signed lower limb; a sum of products keeps the h h and the
+// h l + l h parts in two 64-bit accumulators and drops l l (a quarter of a unit of the result per term, of either
+// sign, so that long sums have no bias).  With |x| < 2^58 there is room for 15 terms, with 55 bits and limbs of
+// 28 for 120, with 56 for 72.  Every stage is brought back to 58 bits by the block's largest
 // value (fx_warp_bits, fx_room): without that the losses of the stages add up (three of them left 40 bits of
 // the P2 moment form).  Errors are relative to the largest value of a block, as norms see them.
 //
@@ -27,7 +28,8 @@ constexpr int kFxDrop = 2 * kFxLimb;  // a product sum's unit is 2^58 times the 
 // biased exponent of x (2047: infinity or nan)
 __device__ __forceinline__ int fx_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
 
-// x in units of 2^(e_block - 1022 - bits), truncated: |x| < 2^(e_block - 1022) maps below 2^bits (bits <= 62).
+// x in units of 2^(e_block - 1022 - bits), truncated: |x| < 2^(e_block - 1022) maps below 2^bits (bits <= 62; at
+// 60 a value is exact down to 2^-7 of the largest).
 // x is finite with an exponent of at most e_block; subnormal values count as zero.
 __device__ __forceinline__ long long fx_from_f64(double x, int e_block, int bits) {
     const int hi = __double2hiint(x), e = (hi >> 20) & 0x7FF;
@@ -60,9 +62,11 @@ __device__ __forceinline__ double fx_to_f64(long long x, int unit) {
     return hi == 0u ? 0.0 : __hiloint2double(static_cast<int>(oh), static_cast<int>(m));
 }
 
+// x = h 2^LIMB + l, -2^(LIMB-1) <= l < 2^(LIMB-1)
 template <int LIMB = kFxLimb>
 __device__ __forceinline__ int2 fx_split(long long x) {
-    return make_int2(static_cast<int>(x >> LIMB), static_cast<int>(x) & ((1 << LIMB) - 1));
+    const int h = static_cast<int>((x + (1ll << (LIMB - 1))) >> LIMB);
+    return make_int2(h, static_cast<int>(x) - static_cast<int>(static_cast<unsigned>(h) << LIMB));
 }
 
 // Bits of the largest magnitude of a block: the magnitudes' bits (one's complement of negative values) are
@@ -79,11 +83,14 @@ __device__ __forceinline__ long long fx_scale(long long x, unsigned two_s) {
 }
 // the power of two that brings a block of `bits` bits to 62, at most 2^31
 __device__ __forceinline__ unsigned fx_room(int bits) { return 1u << min(31, 62 - bits); }
-// x of up to 62 bits as limbs of x 2^(BITS - 62), and the exponent of that unit after fx_scale by two_s
+// x 2^-s rounded: truncated operands have a bias that every product of a sum repeats (the full P2 contraction
+// with truncated 55-bit factors was 16 times as far from the exact sums as FP64; rounded to 56 it is nearer)
+template <int S>
+__device__ __forceinline__ long long fx_round(long long x) { return (x + (1ll << (S - 1))) >> S; }
+// x of up to 62 bits as limbs of x 2^(BITS - 62), rounded, and the exponent of that unit after fx_scale by two_s
 template <int BITS>
 __device__ __forceinline__ int2 fx_split_top(long long x) {
-    constexpr int kDrop = 62 - BITS;
-    return make_int2(static_cast<int>(x >> (kFxLimb + kDrop)), static_cast<int>(x >> kDrop) & ((1 << kFxLimb) - 1));
+    return fx_split(fx_round<62 - BITS>(x));
 }
 template <int BITS>
 __device__ __forceinline__ int fx_top_unit(unsigned two_s) { return (62 - BITS) - (31 - __clz(two_s)); }
@@ -111,7 +118,7 @@ struct FxSum {
         mid = fx_mad(a.y, b.x, fx_mad(a.x, b.y, mid));
     }
     template <int LIMB = kFxLimb>
-    __device__ __forceinline__ long long value() const { return hh + (mid >> LIMB); }
+    __device__ __forceinline__ long long value() const { return hh + fx_round<LIMB>(mid); }
 };
 
 }  // namespace ssp

@@ -68,6 +68,13 @@ int binned_decide_finish(const double *E, const double *c_bar, const double *sin
                          int32_t *scratch, const int32_t *lists, const int32_t *counts, int n_lists,
                          long long list_stride, bool compensated_ds, cudaStream_t st);
 
+// Strain and force of straight-sided tetrahedra through J^{-1} and the gradient table, in fixed point
+// (affine_fixed.cu); arguments as the ssp_*_affine entries, checked there.  force adds into F.
+int strain3_affine_fixed(const double *jinv, const double *ghat, const double *u, const int32_t *dof, int n_u, int n_elem,
+                         int n_p, int n_q, double *E, cudaStream_t st);
+int force3_affine_fixed(const double *jinv, const double *ghat, const double *w, const double *S, const int32_t *elem_row,
+                        int n_rows, int n_elem, int n_p, int n_q, double *F, cudaStream_t st);
+
 // Element tangents of P2 (n_p = 10, n_q = 11) and P4 (35, 24) tetrahedra in fixed point (tangent_fixed.cu):
 // full (symmetric: every D is), or with corr the plastic correction of symmetric tangents.
 int tangent_fixed(int n_p, bool sym, bool corr, const double *d1, const double *d2, const double *d3, const double *DS,

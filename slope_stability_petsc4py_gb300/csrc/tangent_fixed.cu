@@ -4,21 +4,23 @@
 //
 // In FP64 these contractions run at that pipe's 1.6 multiply-adds per clock and SM (full P2 contraction of
 // 19,200 elements 1,267 us, P4 correction of 2,150 plastic elements 1,362 us).  Here every product is three
-// 32 x 32 -> 64-bit IMADs and every sum exact until it is converted once: 456 and 425 us, the IMADs 66 and
-// 47 % of their pipe's time, then the latency of the phases between barriers.  The P2 correction of 27,283
-// plastic elements takes 356 us (641 in FP64); the moment form (assembly.cu) is faster from three points up.
+// 32 x 32 -> 64-bit IMADs and every sum exact until it is converted once: 485 and 455 us, the IMADs some 60 and
+// 45 % of their pipe's time, then the latency of the phases between barriers.  The P2 correction of 27,283
+// plastic elements takes 380 us (641 in FP64); the moment form (assembly.cu) is faster from three points up.
 //
 // One CTA per element (grid-stride), one node pair of K_e per thread: 3 x 3 entries in 18 64-bit accumulators,
 // whose loads of a point (three gradients of node a, the H column of node b in nine 16-byte loads, conflict-free
 // at its 144-byte stride) feed 81 IMADs.  Two nodes a per thread halve the loads but need 168 registers: 11
-// warps an SM instead of 20, and 520 us against 425 on the P4 correction.  Symmetric tangents take the pairs on
+// warps an SM instead of 20, and 520 us against 425 on the P4 correction (before H was rounded by its largest).  Symmetric tangents take the pairs on
 // and above the diagonal (P2: 55, two warps; P4: 630, twenty warps), others all.
-//   1. gradients to 55 bits and D (correction: w-less DS - D_el by 60-bit subtraction) to 58, by the element's
-//      largest; w D rounded to 54
+//   1. gradients to 56 or 57 bits and D (correction: w-less DS - D_el by 60-bit subtraction) to 58, by the element's
+//      largest; w D rounded to 56
 //   2. H[q][b][d][m] = sum_r D[m][row(d, r)] g_b,r for every point at once, kept as limbs
 //   3. K[(a,c),(b,d)] = sum_q sum_r g_a,r H[q][b][d][row(c, r)]; 72 terms at most: limbs of 28 bits, the lower
 //      one signed, so that the dropped products have no bias and both accumulators stay below 2^63
-//   4. the sums, at 58 bits or so, become FP64 and are reduced into the CSR values
+//   4. the sums, at 57 bits or so, become FP64 and are reduced into the CSR values
+// The entries are as near the exact sums as FP64's (a model of these integers: 3e-17 against 1.3e-16 for P2
+// in the 2-norm, P4 6e-17 against 2.4e-16).
 // An element whose inputs are not all finite takes the same sums in FP64.
 #include "fixed.cuh"
 #include "ssp_internal.cuh"
@@ -27,13 +29,8 @@ namespace ssp {
 namespace {
 
 constexpr int kLimb = 28;
-constexpr int kBitsG = 55, kBitsWD = 54;
-
-// x = h 2^28 + l, -2^27 <= l < 2^27
-__device__ __forceinline__ int2 split28(long long x) {
-    const int h = static_cast<int>((x + (1ll << (kLimb - 1))) >> kLimb);
-    return make_int2(h, static_cast<int>(x) - static_cast<int>(static_cast<unsigned>(h) << kLimb));
-}
+// Factors of 56 bits (P2's gradients 57), H's by the element's largest: 72 terms of H times g (P2 33) stay below
+// 2^63 in both accumulators.
 
 struct Args {
     const double *d1, *d2, *d3, *DS, *w;
@@ -109,6 +106,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
     tangent_fixed_kernel(Args A) {
     using Sh = Shape<NP, NQ, SYM>;
     constexpr int kThreads = Sh::kThreads, kWarps = kThreads / 32, kNld = 3 * NP;
+    constexpr int kBitsG = NQ * 3 <= 36 ? 57 : 56;
     constexpr int kGradRounds = (NQ * NP + kThreads - 1) / kThreads, kDRounds = (NQ * 36 + kThreads - 1) / kThreads;
     extern __shared__ __align__(16) unsigned char fx_raw[];
     Smem<NP, NQ> &S = *reinterpret_cast<Smem<NP, NQ> *>(fx_raw);
@@ -117,6 +115,17 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
     auto block_max = [&](int which, int v) {  // written before, read after a barrier
         v = __reduce_max_sync(0xffffffffu, v);
         if (lane == 0) S.exps[which][warp] = v;
+    };
+    auto block_or = [&](unsigned long long v) {
+        const unsigned hi = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(v >> 32)),
+                       lo = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(v));
+        if (lane == 0) S.mags[warp] = static_cast<unsigned long long>(hi) << 32 | lo;
+    };
+    auto warps_or = [&]() {
+        unsigned long long v = 0;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) v |= S.mags[i];
+        return v;
     };
     auto warps_max = [&](int which) {
         int v = 0;
@@ -197,7 +206,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
             if (i < nq * NP) {
                 const int k = i / NP;
 #pragma unroll
-                for (int r = 0; r < 3; ++r) S.g[k][i - k * NP][r] = split28(fx_from_f64(gv[u][r], e_g, kBitsG));
+                for (int r = 0; r < 3; ++r) S.g[k][i - k * NP][r] = fx_split<kLimb>(fx_round<60 - kBitsG>(fx_from_f64(gv[u][r], e_g, 60)));
             }
         }
         if (tid < nq) {
@@ -222,27 +231,21 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
                 mag |= fx_mag(dd[u]);
             }
         }
-        {
-            const unsigned hi = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(mag >> 32)),
-                           lo = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(mag));
-            if (lane == 0) S.mags[warp] = static_cast<unsigned long long>(hi) << 32 | lo;
-        }
+        block_or(mag);
         __syncthreads();
-        mag = 0;
-#pragma unroll
-        for (int i = 0; i < kWarps; ++i) mag |= S.mags[i];
-        const unsigned room = fx_room(64 - __clzll(static_cast<long long>(mag)));
+        const unsigned room = fx_room(64 - __clzll(static_cast<long long>(warps_or())));
 #pragma unroll
         for (int u = 0; u < kDRounds; ++u) {
             const int i = tid + u * kThreads;
             if (i < nq * 36) {
                 const int k = i / 36;
                 const long long v = FxSum(S.wl[k], fx_split_top<58>(fx_scale(dd[u], room))).value();
-                S.wD[k][i - 36 * k] = split28((v + 8) >> 4);
+                S.wD[k][i - 36 * k] = fx_split<kLimb>(fx_round<2>(v));
             }
         }
         __syncthreads();
         // H of every point: item (point, beta), six strain components
+        mag = 0;
         for (int i = tid; i < nq * kNld; i += kThreads) {
             const int k = i / kNld, be = i - k * kNld, n = be / 3, d = be - 3 * n;
             int2 gr[3];
@@ -260,15 +263,30 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
                 t.add_prod(gr[1], {x1.z, x1.w});
                 s.add_prod(gr[2], {x2.x, x2.y});
                 t.add_prod(gr[2], {x2.z, x2.w});
-                const int2 hs = split28(s.value<kLimb>()), ht = split28(t.value<kLimb>());
-                out[m] = make_int4(hs.x, hs.y, ht.x, ht.y);
+                const long long hs = s.value<kLimb>(), ht = t.value<kLimb>();
+                mag |= fx_mag(hs) | fx_mag(ht);  // 64-bit for now
+                out[m] = make_int4(static_cast<int>(hs), static_cast<int>(hs >> 32), static_cast<int>(ht),
+                                   static_cast<int>(ht >> 32));
             }
         }
+        block_or(mag);
         __syncthreads();
-        // total = hh 2^56 + mid 2^28, kept from 2^53 up
+        const unsigned room_h = fx_room(64 - __clzll(static_cast<long long>(warps_or())));
+        for (int i = tid; i < nq * NP * 9; i += kThreads) {
+            int4 *p = reinterpret_cast<int4 *>(&S.H[0][0][0]) + i;
+            const int4 x = *p;
+            const long long hs = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.y)) << 32 |
+                                                        static_cast<unsigned>(x.x)),
+                            ht = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.w)) << 32 |
+                                                        static_cast<unsigned>(x.z));
+            const int2 hl = fx_split<kLimb>(fx_round<6>(fx_scale(hs, room_h))), tl = fx_split<kLimb>(fx_round<6>(fx_scale(ht, room_h)));
+            *p = make_int4(hl.x, hl.y, tl.x, tl.y);
+        }
+        __syncthreads();
+        // total = hh 2^56 + mid 2^28
         const int unit_g = fx_unit(e_g, kBitsG);
-        const int unit_wd = fx_unit(e_w, 58) + fx_unit(e_d, 60) + fx_top_unit<58>(room) + kFxDrop + 4;
-        const int unit_k = unit_wd + unit_g + 2 * kLimb + unit_g + 53;
+        const int unit_wd = fx_unit(e_w, 58) + fx_unit(e_d, 60) + fx_top_unit<58>(room) + kFxDrop + 2;
+        const int unit_k = unit_wd + unit_g + 2 * kLimb + fx_top_unit<56>(room_h) + unit_g + 2 * kLimb;
         const unsigned nnz32 = static_cast<unsigned>(A.nnz < 0x7FFFFFFFll ? A.nnz : 0x7FFFFFFFll);
         auto emit = [&](int32_t p, double v) {
             if (static_cast<unsigned>(p) < nnz32) red_add(A.values + p, v);
@@ -310,7 +328,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     if (SYM && a == b && c > d) continue;
-                    const double v = fx_to_f64((acc[c][d].hh << 3) + (acc[c][d].mid >> 25), unit_k);
+                    const double v = fx_to_f64(acc[c][d].value<kLimb>(), unit_k);
                     emit(up[c * kNld + d], v);
                     if (SYM && (a != b || c != d)) emit(low[d * kNld + c], v);
                 }

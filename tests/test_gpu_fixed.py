@@ -220,3 +220,59 @@ def test_element_tangents(oracle, et, dims, kind, n_plastic, magnitude):
     others = np.ones(pat.nnz, dtype=bool)
     others[mine[mine >= 0]] = False
     assert np.isnan(out[mine[mine >= 0]]).any() and rel_err(out[others], got[others]) <= TOL
+
+
+@pytest.mark.parametrize("et,dims,magnitude", [("P4", (2, 2, 2), 1.0), ("P4", (3, 1, 1), 1e-140), ("P4", (1, 1, 1), 1e140),
+                                               ("P2", (4, 2, 3), 1.0)])
+def test_affine_strain_and_force(oracle, et, dims, magnitude):
+    """The table form (P4's; P2 takes it here for another shape): whole and partly filled groups of elements."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.fem import reference_gradients
+
+    op, pat = _pattern(et, dims)
+    d, n_el, n_q, n_p = pat.device, int(pat.overlap_elements.size), pat.n_q, pat.n_p
+    rng = np.random.default_rng(n_el)
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a), device="cuda")  # noqa: E731
+    ghat = dev(np.transpose(reference_gradients(3, et), (2, 1, 0)))
+    dof = pat.overlap_element_dof_lids
+    u = magnitude * (3.0 + rng.standard_normal(int(pat.overlap_global_dofs.size)))
+    dphi = [pat.dphi1, pat.dphi2, pat.dphi3]
+
+    def strain(u):
+        E, ud = torch.full((n_el * n_q, 6), -7.0, dtype=torch.float64, device="cuda"), dev(u)
+        _lib.call("ssp_assemble_overlap_strain_3d_affine", _lib.ptr(d["jinv"]), _lib.ptr(ghat), _lib.ptr(ud), u.size,
+                  _lib.ptr(d["dof_lids"]), n_el * n_q, n_el, n_p, n_q, _lib.ptr(E), _lib.stream_handle())
+        return E.cpu().numpy()
+
+    E = strain(u)
+    assert rel_err(E, oracle.strain_3d(*dphi, u, dof, n_q)) <= TOL
+    S = magnitude * rng.standard_normal((n_el * n_q, 6)) * 10.0 ** rng.uniform(-2.0, 0.0, (n_el * n_q, 1))
+    rows = d["elem_row"].cpu().numpy()
+    n_rows = int(pat.local_matrix_pattern.shape[0])
+
+    def force(S):
+        F, Sd = torch.full((n_rows,), -7.0, dtype=torch.float64, device="cuda"), dev(S)
+        _lib.call("ssp_assemble_force_element_affine", _lib.ptr(d["jinv"]), _lib.ptr(ghat), _lib.ptr(Sd),
+                  _lib.ptr(d["weight"]), _lib.ptr(d["elem_row"]), n_el, n_p, n_q, n_rows, _lib.ptr(F), _lib.stream_handle())
+        return F.cpu().numpy()
+
+    bt = ((0, 3, 5), (3, 1, 4), (5, 4, 2))
+    want = np.zeros(n_rows)
+    ws = (pat.overlap_assembly_weight[:, None] * S).reshape(n_el, n_q, 6)
+    for c in range(3):
+        f = sum(np.einsum("eqa,eq->ea", dphi[z].reshape(n_el, n_q, n_p), ws[..., bt[c][z]]) for z in range(3))
+        r = rows.reshape(n_el, n_p, 3)[:, :, c]
+        np.add.at(want, r[r >= 0], f[r >= 0])
+    F = force(S)
+    assert rel_err(F, want) <= TOL
+    u2, S2 = u.copy(), S.copy()
+    u2[dof[0, 4]] = float("nan")
+    S2[0, 1] = float("inf")
+    hit = (dof == dof[0, 4]).any(axis=1).repeat(n_q)
+    E2, F2 = strain(u2), force(S2)
+    touched = np.zeros(n_rows, dtype=bool)
+    touched[rows[0][rows[0] >= 0]] = True
+    assert np.isnan(E2[hit]).any() and np.array_equal(E2[~hit], E[~hit])
+    assert not np.isfinite(F2[touched]).all() and rel_err(F2[~touched], F[~touched]) <= TOL
