@@ -30,45 +30,24 @@ __device__ __forceinline__ double half_ident(int i) { return i < 3 ? 1.0 : 0.5; 
 enum Branch : int { kElastic = 0, kSmooth = 1, kLeft = 2, kRight = 3, kApex = 4 };
 
 struct Principal3 {
-    double t[6], sq[6];
+    double t[6];
     double I1, e1, e2, e3;
 };
 
+// t (shears halved) of E and its principal values, ordered.
 __device__ __forceinline__ void principal3(const double *E, Principal3 &p) {
 #pragma unroll
     for (int i = 0; i < 6; ++i) p.t[i] = half_ident(i) * E[i];
-    const double *t = p.t;
-    p.sq[0] = t[0] * t[0] + t[3] * t[3] + t[5] * t[5];
-    p.sq[1] = t[1] * t[1] + t[3] * t[3] + t[4] * t[4];
-    p.sq[2] = t[2] * t[2] + t[4] * t[4] + t[5] * t[5];
-    p.sq[3] = t[0] * t[3] + t[1] * t[3] + t[4] * t[5];
-    p.sq[4] = t[3] * t[5] + t[1] * t[4] + t[2] * t[4];
-    p.sq[5] = t[0] * t[5] + t[3] * t[4] + t[2] * t[5];
-    const double I1 = t[0] + t[1] + t[2];
-    const double I2 = t[0] * t[1] + t[0] * t[2] + t[1] * t[2] - t[3] * t[3] - t[4] * t[4] - t[5] * t[5];
-    const double I3 = t[0] * t[1] * t[2] - t[2] * t[3] * t[3] - t[1] * t[5] * t[5] - t[0] * t[4] * t[4] +
-                      2.0 * t[3] * t[4] * t[5];
-    // divisions by constants as products with the rounded reciprocals (an ulp from the quotients)
-    double Q = (I1 * I1 - 3.0 * I2) * (1.0 / 9.0);
-    if (Q < 0.0) Q = 0.0;
-    const double R = (-2.0 * I1 * I1 * I1 + 9.0 * I1 * I2 - 27.0 * I3) * (1.0 / 54.0);
-    const double rq = sqrt(Q);
-    double theta = 0.0;
-    if (!(Q < 1e-30)) {
-        double c = R / (rq * Q);
-        c = fmin(1.0, fmax(-1.0, c));
-        theta = acos(c) * (1.0 / 3.0);
+    const Deviator d = deviator_invariants(p.t);
+    double rq, v;
+    roots_newton(d.Q, rq, v);
+    p.I1 = d.I1;
+    const bool spherical = d.Q < 1e-30;
+    const int close = lode_values(spherical ? 1.0 : d.R * (v * v * v), rq, d.third, p.e1, p.e2, p.e3);
+    if (close && !spherical) {
+        if (close == 1) refine_pair(p.t, d.third, p.e3, p.e1, p.e2);
+        else refine_pair(p.t, d.third, p.e1, p.e2, p.e3);
     }
-    const double third = I1 * (1.0 / 3.0);
-    p.I1 = I1;
-    // cos(theta -+ 2 pi/3) = -cos(theta)/2 +- (sqrt(3)/2) sin(theta): one sine and cosine instead of
-    // three cosines
-    double st, ct;
-    sincos_lode(theta, st, ct);
-    const double r3 = 1.7320508075688772 * st;
-    p.e1 = rq * (ct + r3) + third;
-    p.e2 = rq * (ct - r3) + third;
-    p.e3 = -2.0 * rq * ct + third;
 }
 
 // d(t*t)_i / dE_j (symmetric), entry for i <= j only.
@@ -94,9 +73,13 @@ __device__ __forceinline__ double square_jac(const double *t, int i, int j) {
     }
 }
 
-__device__ __forceinline__ void projection(const Principal3 &p, double sum_o, double prod_o, double inv, double *P) {
+__device__ __forceinline__ void projection(const double *t, const double *sq, double sum_o, double prod_o, double inv,
+                                           double *P) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) P[i] = inv * (p.sq[i] - sum_o * p.t[i] + prod_o * vol_iota(i));
+    for (int i = 0; i < 6; ++i) {
+        const double v = fma(-sum_o, t[i], sq[i]);
+        P[i] = __dmul_rn(inv, i < 3 ? __dadd_rn(v, prod_o) : v);
+    }
 }
 
 __device__ __forceinline__ void store_sym(double *DS, int i, int j, double v) {
@@ -106,51 +89,31 @@ __device__ __forceinline__ void store_sym(double *DS, int i, int j, double v) {
 
 struct Decision3 {
     int branch;
-    double lam;  // plastic multiplier of the selected branch (elastic / apex: unused)
-    double den;  // its denominator
+    double num, den;  // the plastic multiplier of the selected branch is num / den (elastic / apex: unused)
 };
 
-// Plastic multipliers of the three return branches (constitutive_3D_kernel.h:144-147, 213-215, 277-279).
-__device__ __forceinline__ void smooth_lam(const Principal3 &p, const Mat3 &m, double f_tr, double &lam, double &den) {
-    const double sp = m.sin_phi;
-    den = 4.0 * m.lame * m.sin_phi * sp + 4.0 * m.shear * (1.0 + m.sin_phi * sp);
-    lam = f_tr / den;
-}
-__device__ __forceinline__ void left_lam(const Principal3 &p, const Mat3 &m, double &lam, double &den) {
-    const double sp = m.sin_phi, sf = m.sin_phi, G = m.shear, L = m.lame;
-    den = 4.0 * L * sf * sp + G * (1.0 + sf) * (1.0 + sp) + 2.0 * G * (1.0 - sf) * (1.0 - sp);
-    lam = (G * ((1.0 + sf) * (p.e1 + p.e2) - 2.0 * (1.0 - sf) * p.e3) + 2.0 * L * sf * p.I1 - m.c_bar) / den;
-}
-__device__ __forceinline__ void right_lam(const Principal3 &p, const Mat3 &m, double &lam, double &den) {
-    const double sp = m.sin_phi, sf = m.sin_phi, G = m.shear, L = m.lame;
-    den = 4.0 * L * sf * sp + 2.0 * G * (1.0 + sf) * (1.0 + sp) + G * (1.0 - sf) * (1.0 - sp);
-    lam = (G * (2.0 * (1.0 + sf) * p.e1 - (1.0 - sf) * (p.e2 + p.e3)) + 2.0 * L * sf * p.I1 - m.c_bar) / den;
-}
-__device__ __forceinline__ double trial_yield(const Principal3 &p, const Mat3 &m) {
-    return 2.0 * m.shear * ((1.0 + m.sin_phi) * p.e1 - (1.0 - m.sin_phi) * p.e3) + 2.0 * m.lame * m.sin_phi * p.I1 -
-           m.c_bar;
-}
-
-// Branch selection (constitutive_3D_kernel.h:114-338).
+// Branch selection (constitutive_3D_kernel.h:114-338).  The bounds g = x / d and the multipliers lam = num / den
+// (den > 0) are compared cross-multiplied, without a division; the two edges, of which a point can have one,
+// share the evaluation of theirs.
 __device__ __forceinline__ Decision3 decide3(const Principal3 &p, const Mat3 &m) {
-    const double sp = m.sin_phi;
-    const double f_tr = trial_yield(p, m);
+    const double s = m.sin_phi, G = m.shear, p1 = 1.0 + s, m1 = 1.0 - s;
+    const double ls2 = 2.0 * m.lame * s;
+    const double lin = ls2 * p.I1 - m.c_bar;
+    const double f_tr = 2.0 * G * (p1 * p.e1 - m1 * p.e3) + lin;
     if (f_tr <= 0.0) return {kElastic, 0.0, 1.0};
-    // the reference's bounds g = x / d (d = 1 +- sin phi, 3 -+ sin phi, all positive) compared as
-    // lam d against x, and g_sl against g_sr cross-multiplied: no division for the tests
-    const double a_sl = p.e1 - p.e2, d_sl = 1.0 + sp;  // g_sl = a_sl / d_sl
-    const double a_sr = p.e2 - p.e3, d_sr = 1.0 - sp;  // g_sr = a_sr / d_sr
-    double lam, den;
-    smooth_lam(p, m, f_tr, lam, den);
-    if (lam * d_sl <= a_sl && lam * d_sr <= a_sr) return {kSmooth, lam, den};
-    const double l_sl = a_sl * d_sr, l_sr = a_sr * d_sl;  // g_sl < g_sr <=> l_sl < l_sr
-    if (l_sl < l_sr) {
-        left_lam(p, m, lam, den);
-        if (lam * d_sl >= a_sl && lam * (3.0 - sp) <= p.e1 + p.e2 - 2.0 * p.e3) return {kLeft, lam, den};
-    }
-    if (l_sl > l_sr) {
-        right_lam(p, m, lam, den);
-        if (lam * d_sr >= a_sr && lam * (3.0 + sp) <= 2.0 * p.e1 - p.e2 - p.e3) return {kRight, lam, den};
+    const double a_sl = p.e1 - p.e2, a_sr = p.e2 - p.e3;  // g_sl = a_sl / p1, g_sr = a_sr / m1
+    const double l4 = 2.0 * ls2 * s;
+    const double den = l4 + 4.0 * G * (1.0 + s * s);
+    if (f_tr * p1 <= a_sl * den && f_tr * m1 <= a_sr * den) return {kSmooth, f_tr, den};
+    const double l_sl = a_sl * m1, l_sr = a_sr * p1;  // g_sl < g_sr <=> l_sl < l_sr
+    const bool left = l_sl < l_sr;
+    if (left || l_sl > l_sr) {
+        const double x = left ? p.e1 + p.e2 : 2.0 * p.e1, y = left ? 2.0 * p.e3 : p.e2 + p.e3;
+        const double pp = p1 * p1, mm = m1 * m1;
+        const double de = l4 + G * (left ? pp + 2.0 * mm : 2.0 * pp + mm);
+        const double nu = G * (p1 * x - m1 * y) + lin;
+        const double lower = left ? nu * p1 - a_sl * de : nu * m1 - a_sr * de;
+        if (lower >= 0.0 && nu * (left ? 3.0 - s : 3.0 + s) <= (x - y) * de) return {left ? kLeft : kRight, nu, de};
     }
     return {kApex, 0.0, 1.0};
 }
@@ -326,10 +289,10 @@ __device__ __forceinline__ bool edge_ds_compensated(const Principal3 &p, const M
 // points keep the entry-by-entry form.
 constexpr double kRegroupGap = 0.05;
 
+// Smooth face, in the basis (P1, P3, iota): P2 = iota - P1 - P3 and Dp = al P1 + be P3 + ga iota.
 __device__ __forceinline__ bool smooth_ds_regrouped(const Principal3 &p, const Mat3 &m, const double *P1,
-                                                    const double *P2, const double *P3, double inv1, double inv2,
-                                                    double inv3, double s1, double s2, double s3, const double *Dp,
-                                                    double inv_den, double *DS) {
+                                                    const double *P3, double inv1, double inv2, double inv3, double s1,
+                                                    double s2, double s3, double inv_den, double *DS) {
     const double e1 = p.e1, e2 = p.e2, e3 = p.e3;
     if (!(fmin(e1 - e2, e2 - e3) >= kRegroupGap * fmax(fabs(e1), fabs(e3)))) return false;
     const double a1 = s1 * inv1, a2 = s2 * inv2, a3 = s3 * inv3;
@@ -341,51 +304,53 @@ __device__ __forceinline__ bool smooth_ds_regrouped(const Principal3 &p, const M
     const double K1 = G2 - (a1 * c1a + a2 * c2b + a3 * c3b);
     const double K2 = G2 - (a1 * c1b + a2 * c2a - a3 * c3b);
     const double K3 = G2 + (a1 * c1b + a2 * c2b - a3 * c3a);
-    double q1[6], q2[6], q3[6], dq[6];
+    const double al = G2 * (1.0 + m.sin_phi), be = -G2 * (1.0 - m.sin_phi), ga = 2.0 * m.lame * m.sin_phi;
+    const double ai = al * inv_den, bi = be * inv_den, gi = ga * inv_den;
+    const double w11 = K1 + K2 - al * ai, w33 = K3 + K2 - be * bi, w13 = K2 - al * bi, w1 = -K2 - al * gi, w3 = -K2 - be * gi,
+                 w0 = K2 + m.lame - ga * gi;
+    double C1[6], C3[6], C0[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-        q1[i] = K1 * P1[i];
-        q2[i] = K2 * P2[i];
-        q3[i] = K3 * P3[i];
-        dq[i] = -Dp[i] * inv_den;
+        C1[i] = w11 * P1[i] + w13 * P3[i] + w1 * vol_iota(i);
+        C3[i] = w13 * P1[i] + w33 * P3[i] + w3 * vol_iota(i);
+        C0[i] = w1 * P1[i] + w3 * P3[i] + w0 * vol_iota(i);
     }
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
 #pragma unroll
         for (int i = 0; i <= j; ++i) {
-            double v = A * square_jac(p.t, i, j) + q1[i] * P1[j] + q2[i] * P2[j] + q3[i] * P3[j] + dq[i] * Dp[j];
+            double v = A * square_jac(p.t, i, j) + P1[i] * C1[j] + P3[i] * C3[j];
+            if (i < 3) v += C0[j];
             if (i == j) v -= half_ident(i) * B;
-            if (j < 3) v += m.lame;
             store_sym(DS, i, j, v);
         }
     }
     return true;
 }
 
-// Edges: left Q = P12, R = P3, e = e3, em = e1 + e2; right Q = P23, R = P1, e = e1, em = e2 + e3;
-// a the branch's (s_R - s_Q) inv and gap its eigenvalue gap.
-__device__ __forceinline__ bool edge_ds_regrouped(const Principal3 &p, const Mat3 &m, const double *Q, const double *R,
-                                                  double a, double em, double e, double gap, const double *Dp,
-                                                  double inv_den, double *DS) {
+// Edges, in the basis (R, t, iota): left R = P3, e = e3, em = e1 + e2; right R = P1, e = e1, em = e2 + e3;
+// Q = iota - R, a the branch's (s_R - s_Q) inv, gap its eigenvalue gap and Dp = be R + ga iota.
+__device__ __forceinline__ bool edge_ds_regrouped(const Principal3 &p, const Mat3 &m, const double *R, double a, double em,
+                                                  double e, double gap, double be, double ga, double inv_den,
+                                                  double *DS) {
     if (!(gap >= kRegroupGap * fmax(fabs(p.e1), fabs(p.e3)))) return false;
     const double kQ = a * em + m.shear, kR = a * (em - 2.0 * e) + 2.0 * m.shear, ae = a * e, aem = a * em;
-    double aq[6], kqq[6], krr[6], aeq[6], dq[6];
+    const double bi = be * inv_den, gi = ga * inv_den;
+    const double wrr = kQ + kR - 2.0 * ae - be * bi, wr = ae - kQ - be * gi, w0 = kQ + m.lame - ga * gi;
+    double CR[6], CT[6], C0[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-        aq[i] = -a * Q[i];
-        kqq[i] = kQ * Q[i];
-        krr[i] = kR * R[i];
-        aeq[i] = ae * Q[i];
-        dq[i] = -Dp[i] * inv_den;
+        CR[i] = wrr * R[i] + a * p.t[i] + wr * vol_iota(i);
+        CT[i] = a * R[i] - a * vol_iota(i);
+        C0[i] = wr * R[i] - a * p.t[i] + w0 * vol_iota(i);
     }
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
 #pragma unroll
         for (int i = 0; i <= j; ++i) {
-            double v = a * square_jac(p.t, i, j) + aq[i] * p.t[j] + p.t[i] * aq[j] + kqq[i] * Q[j] + krr[i] * R[j] +
-                       aeq[i] * R[j] + R[i] * aeq[j] + dq[i] * Dp[j];
+            double v = a * square_jac(p.t, i, j) + R[i] * CR[j] + p.t[i] * CT[j];
+            if (i < 3) v += C0[j];
             if (i == j) v -= half_ident(i) * aem;
-            if (j < 3) v += m.lame;
             store_sym(DS, i, j, v);
         }
     }
@@ -403,30 +368,63 @@ __device__ void finish3(const Principal3 &p, const Decision3 &d, const Mat3 &m, 
         finish_elastic(p.t, I1, m, S, DS);
         return;
     }
-    if (d.branch == kSmooth) {
-        const double lam_s = d.lam;
-        const double inv1 = 1.0 / ((e1 - e2) * (e1 - e3));
-        const double inv2 = 1.0 / ((e2 - e1) * (e2 - e3));
-        const double inv3 = 1.0 / ((e3 - e1) * (e3 - e2));
-        double P1[6], P2[6], P3[6];
-        projection(p, e2 + e3, e2 * e3, inv1, P1);
-        projection(p, e1 + e3, e1 * e3, inv2, P2);
-        projection(p, e1 + e2, e1 * e2, inv3, P3);
-        const double s1 = lame * I1 + 2.0 * shear * e1 - lam_s * (2.0 * lame * sp + 2.0 * shear * (1.0 + sp));
-        const double s2 = lame * I1 + 2.0 * shear * e2 - lam_s * 2.0 * lame * sp;
-        const double s3 = lame * I1 + 2.0 * shear * e3 - lam_s * (2.0 * lame * sp - 2.0 * shear * (1.0 - sp));
+    if (d.branch == kApex) {
+        const double sa = m.c_bar / (2.0 * sin_phi);
 #pragma unroll
-        for (int i = 0; i < 6; ++i) S[i] = s1 * P1[i] + s2 * P2[i] + s3 * P3[i];
+        for (int i = 0; i < 3; ++i) S[i] = sa;
+#pragma unroll
+        for (int i = 3; i < 6; ++i) S[i] = 0.0;
+        if (DS) {
+#pragma unroll
+            for (int k = 0; k < 36; ++k) DS[k] = 0.0;
+        }
+        return;
+    }
+    double sq[6];
+    square3(p.t, sq);
+    const double inv_den = recip_newton(d.den), lam = __dmul_rn(d.num, inv_den);
+    const double li = __dmul_rn(lame, I1), l2s = __dmul_rn(2.0 * lame, sp), p1 = 1.0 + sp, m1 = 1.0 - sp;
+    if (d.branch == kSmooth) {
+        // the three 1 / ((e_k - e_l)(e_k - e_m)) from one reciprocal where the product of the gaps is far from
+        // FP64's ends
+        const double g12 = e1 - e2, g13 = e1 - e3, g23 = e2 - e3, g = g12 * g13 * g23;
+        double inv1, inv2, inv3;
+        if (g > 1e-250) {
+            const double ig = recip_newton(g);
+            inv1 = g23 * ig;
+            inv2 = -(g13 * ig);
+            inv3 = g12 * ig;
+        } else {
+            inv1 = 1.0 / (g12 * g13);
+            inv2 = -1.0 / (g12 * g23);
+            inv3 = 1.0 / (g13 * g23);
+        }
+        double P1[6], P3[6];
+        projection(p.t, sq, e2 + e3, __dmul_rn(e2, e3), inv1, P1);
+        projection(p.t, sq, e1 + e2, __dmul_rn(e1, e2), inv3, P3);
+        const double s1 = fma(-lam, fma(2.0 * shear, p1, l2s), fma(2.0 * shear, e1, li));
+        const double s2 = fma(-lam, l2s, fma(2.0 * shear, e2, li));
+        const double s3 = fma(-lam, fma(-2.0 * shear, m1, l2s), fma(2.0 * shear, e3, li));
+        const bool wide = fmin(g12, g23) >= kRegroupGap * fmax(fabs(e1), fabs(e3));
+        if (wide) {  // P2 = iota - P1 - P3
+#pragma unroll
+            for (int i = 0; i < 6; ++i) S[i] = fma(s1 - s2, P1[i], fma(s3 - s2, P3[i], s2 * vol_iota(i)));
+            if (!COMP && DS && smooth_ds_regrouped(p, m, P1, P3, inv1, inv2, inv3, s1, s2, s3, inv_den, DS)) return;
+        }
+        if (wide && !DS) return;
+        double P2[6];
+        projection(p.t, sq, e1 + e3, __dmul_rn(e1, e3), inv2, P2);
+        if (!wide) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) S[i] = fma(s1, P1[i], fma(s2, P2[i], s3 * P3[i]));
+        }
         if (DS) {
             double Dp[6];
 #pragma unroll
             for (int i = 0; i < 6; ++i)
                 Dp[i] = 2.0 * shear * ((1.0 + sin_phi) * P1[i] - (1.0 - sin_phi) * P3[i]) + 2.0 * lame * sin_phi * vol_iota(i);
-            const double inv_den = 1.0 / d.den;
             if constexpr (COMP) {
                 if (smooth_ds_compensated(p, m, P1, P2, P3, inv1, inv2, inv3, s1, s2, s3, Dp, inv_den, DS)) return;
-            } else {
-                if (smooth_ds_regrouped(p, m, P1, P2, P3, inv1, inv2, inv3, s1, s2, s3, Dp, inv_den, DS)) return;
             }
             const double em23 = e2 + e3, em13 = e1 + e3, em12 = e1 + e2;
             const double c1a = 2.0 * e1 - e2 - e3, c1b = e2 - e3;
@@ -451,27 +449,26 @@ __device__ void finish3(const Principal3 &p, const Decision3 &d, const Mat3 &m, 
         return;
     }
     if (d.branch == kLeft) {
-        const double lam_l = d.lam;
-        const double inv3 = 1.0 / ((e3 - e1) * (e3 - e2));
+        const double inv3 = recip_newton((e3 - e1) * (e3 - e2));
         double P3[6], P12[6];
-        projection(p, e1 + e2, e1 * e2, inv3, P3);
+        projection(p.t, sq, e1 + e2, __dmul_rn(e1, e2), inv3, P3);
 #pragma unroll
         for (int i = 0; i < 6; ++i) P12[i] = vol_iota(i) - P3[i];
-        const double s1 = lame * I1 + shear * (e1 + e2) - lam_l * (2.0 * lame * sp + shear * (1.0 + sp));
-        const double s3 = lame * I1 + 2.0 * shear * e3 - lam_l * (2.0 * lame * sp - 2.0 * shear * (1.0 - sp));
+        const double s1 = fma(-lam, fma(shear, p1, l2s), fma(shear, e1 + e2, li));
+        const double s3 = fma(-lam, fma(-2.0 * shear, m1, l2s), fma(2.0 * shear, e3, li));
 #pragma unroll
-        for (int i = 0; i < 6; ++i) S[i] = s1 * P12[i] + s3 * P3[i];
+        for (int i = 0; i < 6; ++i) S[i] = fma(s3 - s1, P3[i], s1 * vol_iota(i));
         if (DS) {
+            if (!COMP && edge_ds_regrouped(p, m, P3, (s3 - s1) * inv3, e1 + e2, e3, e2 - e3, -shear * (3.0 - sin_phi),
+                                           shear * (1.0 + sin_phi) + 2.0 * lame * sin_phi, inv_den, DS))
+                return;
             double Dp[6];
 #pragma unroll
             for (int i = 0; i < 6; ++i)
                 Dp[i] = shear * ((1.0 + sin_phi) * P12[i] - 2.0 * (1.0 - sin_phi) * P3[i]) + 2.0 * lame * sin_phi * vol_iota(i);
             const double em12 = e1 + e2;
-            const double inv_den = 1.0 / d.den;
             if constexpr (COMP) {
                 if (edge_ds_compensated(p, m, P12, P3, (s3 - s1) * inv3, em12, e3, e2 - e3, Dp, inv_den, DS)) return;
-            } else {
-                if (edge_ds_regrouped(p, m, P12, P3, (s3 - s1) * inv3, em12, e3, e2 - e3, Dp, inv_den, DS)) return;
             }
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
@@ -490,27 +487,26 @@ __device__ void finish3(const Principal3 &p, const Decision3 &d, const Mat3 &m, 
         return;
     }
     if (d.branch == kRight) {
-        const double lam_r = d.lam;
-        const double inv1 = 1.0 / ((e1 - e2) * (e1 - e3));
+        const double inv1 = recip_newton((e1 - e2) * (e1 - e3));
         double P1[6], P23[6];
-        projection(p, e2 + e3, e2 * e3, inv1, P1);
+        projection(p.t, sq, e2 + e3, __dmul_rn(e2, e3), inv1, P1);
 #pragma unroll
         for (int i = 0; i < 6; ++i) P23[i] = vol_iota(i) - P1[i];
-        const double s1 = lame * I1 + 2.0 * shear * e1 - lam_r * (2.0 * lame * sp + 2.0 * shear * (1.0 + sp));
-        const double s3 = lame * I1 + shear * (e2 + e3) - lam_r * (2.0 * lame * sp - shear * (1.0 - sp));
+        const double s1 = fma(-lam, fma(2.0 * shear, p1, l2s), fma(2.0 * shear, e1, li));
+        const double s3 = fma(-lam, fma(-shear, m1, l2s), fma(shear, e2 + e3, li));
 #pragma unroll
-        for (int i = 0; i < 6; ++i) S[i] = s1 * P1[i] + s3 * P23[i];
+        for (int i = 0; i < 6; ++i) S[i] = fma(s1 - s3, P1[i], s3 * vol_iota(i));
         if (DS) {
+            if (!COMP && edge_ds_regrouped(p, m, P1, (s1 - s3) * inv1, e2 + e3, e1, e1 - e2, shear * (3.0 + sin_phi),
+                                           2.0 * lame * sin_phi - shear * (1.0 - sin_phi), inv_den, DS))
+                return;
             double Dp[6];
 #pragma unroll
             for (int i = 0; i < 6; ++i)
                 Dp[i] = shear * (2.0 * (1.0 + sin_phi) * P1[i] - (1.0 - sin_phi) * P23[i]) + 2.0 * lame * sin_phi * vol_iota(i);
             const double em23 = e2 + e3;
-            const double inv_den = 1.0 / d.den;
             if constexpr (COMP) {
                 if (edge_ds_compensated(p, m, P23, P1, (s1 - s3) * inv1, em23, e1, e1 - e2, Dp, inv_den, DS)) return;
-            } else {
-                if (edge_ds_regrouped(p, m, P23, P1, (s1 - s3) * inv1, em23, e1, e1 - e2, Dp, inv_den, DS)) return;
             }
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
@@ -527,15 +523,6 @@ __device__ void finish3(const Principal3 &p, const Decision3 &d, const Mat3 &m, 
             }
         }
         return;
-    }
-    const double sa = m.c_bar / (2.0 * sin_phi);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) S[i] = sa;
-#pragma unroll
-    for (int i = 3; i < 6; ++i) S[i] = 0.0;
-    if (DS) {
-#pragma unroll
-        for (int k = 0; k < 36; ++k) DS[k] = 0.0;
     }
 }
 
@@ -622,27 +609,24 @@ __global__ void __launch_bounds__(128) mc3d_kernel(const double *__restrict__ E,
 //      (a dozen FP64 instructions), the others are appended to list L (counter 0, region 0).
 //   B: over L, the FP64 eigen-decomposition and branch decision (dense warps); elastic and apex
 //      points are finished here; a smooth / left-edge / right-edge point leaves its decision record
-//      (principal values, t, t*t, I1, multiplier, denominator: 18 doubles) in the first entries of
+//      (principal values, t, I1, the multiplier's numerator and denominator: 12 doubles) in the first entries of
 //      its own DS row, which pass C overwrites, and is appended to its branch's list (smooth:
 //      region 1 from the front; left: region 2 from the front; right: region 2 from the back;
 //      counters 1, 2, 3).
 //   C: one branch per blockIdx.y: the stress and consistent tangent from the record, so every
 //      warp runs one branch's code and nothing is computed twice.
 // Every result equals the single-pass kernel's (the same operations on the same values).
-constexpr int kRecord = 18;
+constexpr int kRecord = 12;
 __device__ __forceinline__ void store_record(double *DS, long long p, const Principal3 &pr, const Decision3 &d) {
     double r[kRecord];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        r[i] = pr.t[i];
-        r[6 + i] = pr.sq[i];
-    }
-    r[12] = pr.I1;
-    r[13] = pr.e1;
-    r[14] = pr.e2;
-    r[15] = pr.e3;
-    r[16] = d.lam;
-    r[17] = d.den;
+    for (int i = 0; i < 6; ++i) r[i] = pr.t[i];
+    r[6] = pr.I1;
+    r[7] = pr.e1;
+    r[8] = pr.e2;
+    r[9] = pr.e3;
+    r[10] = d.num;
+    r[11] = d.den;
     double2 *D2 = reinterpret_cast<double2 *>(DS + 36 * p);
 #pragma unroll
     for (int k = 0; k < kRecord / 2; ++k) D2[k] = make_double2(r[2 * k], r[2 * k + 1]);
@@ -657,16 +641,13 @@ __device__ __forceinline__ void load_record(const double *DS, long long p, Princ
         r[2 * k + 1] = v.y;
     }
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        pr.t[i] = r[i];
-        pr.sq[i] = r[6 + i];
-    }
-    pr.I1 = r[12];
-    pr.e1 = r[13];
-    pr.e2 = r[14];
-    pr.e3 = r[15];
-    d.lam = r[16];
-    d.den = r[17];
+    for (int i = 0; i < 6; ++i) pr.t[i] = r[i];
+    pr.I1 = r[6];
+    pr.e1 = r[7];
+    pr.e2 = r[8];
+    pr.e3 = r[9];
+    d.num = r[10];
+    d.den = r[11];
 }
 
 // warp-aggregated append of the lanes with want == true to list[...] through counter *ctr;
@@ -735,8 +716,9 @@ __global__ void __launch_bounds__(128) mc3d_bin_kernel(const double *__restrict_
     if (listed) scratch[4 + slot] = p;
 }
 
-// five CTAs per SM (at most 102 registers; 96 used without spills): the pass is FP64-bound with long
-// dependent chains per point, and more resident warps hide more of their latency
+// Five CTAs per SM (at most 102 registers): the pass is bound by its 120 FP64 operations a point, in long chains,
+// and more resident warps hide more of their latency.  With an acos, the series and divisions it took 302 us of a
+// mesh with 3.0 M points, 365 k of them plastic; with the Newton steps 196.
 __global__ void __launch_bounds__(128, 5) mc3d_decide_kernel(const double *__restrict__ E,
                                                           const double *__restrict__ c_bar,
                                                           const double *__restrict__ sin_phi,
@@ -790,7 +772,7 @@ __global__ void __launch_bounds__(128, 5) mc3d_decide_kernel(const double *__res
 }
 
 // Stress only: the listed points decided and finished (the single pass paid an eigen-decomposition in nearly
-// every warp for the tenth of the points that need one: 296 us for 1.1 M points; screen and list 37 + 100).
+// every warp for the tenth of the points that need one: 296 us for 1.1 M points; screen and list 108 together).
 __global__ void __launch_bounds__(128, 5) mc3d_stress_list_kernel(const double *__restrict__ E,
                                                                   const double *__restrict__ c_bar,
                                                                   const double *__restrict__ sin_phi,
@@ -815,7 +797,9 @@ __global__ void __launch_bounds__(128, 5) mc3d_stress_list_kernel(const double *
     }
 }
 
-// three CTAs per SM (168 registers): the lists are short and each point a long dependent chain
+// Three CTAs per SM (168 registers): the lists are short and each point a long dependent chain, bound by its FP64
+// operations (82 % of the pipe's cycles).  Tangents as quadratic forms in (P1, P3, iota) or (R, t, iota) and one
+// reciprocal for the three gaps: 224 -> 206 us for 365 k points.
 template <bool COMP>
 __global__ void __launch_bounds__(128, 3) mc3d_finish_kernel(const double *__restrict__ c_bar,
                                                           const double *__restrict__ sin_phi,

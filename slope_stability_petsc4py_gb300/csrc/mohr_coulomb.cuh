@@ -9,31 +9,117 @@ struct Mat3 {
     double c_bar, sin_phi, shear, lame;
 };
 
-// sin and cos of a Lode angle theta in [0, pi/3] from their Taylor series, Horner in theta^2: the
-// first omitted terms, theta^19 / 19! and theta^20 / 20!, are below 2e-17 there, and without a
-// branch every lane of a warp runs the same instructions (a general sincos reduces its argument by
-// quadrants, and pi/4 < pi/3).  Within one ulp of the correctly rounded values on [0, pi/3].
-__device__ __forceinline__ void sincos_lode(double theta, double &s, double &c) {
-    const double z = theta * theta;
-    double ps = 1.0 / 355687428096000.0;  // 1/17!
-    ps = fma(ps, z, -1.0 / 1307674368000.0);
-    ps = fma(ps, z, 1.0 / 6227020800.0);
-    ps = fma(ps, z, -1.0 / 39916800.0);
-    ps = fma(ps, z, 1.0 / 362880.0);
-    ps = fma(ps, z, -1.0 / 5040.0);
-    ps = fma(ps, z, 1.0 / 120.0);
-    ps = fma(ps, z, -1.0 / 6.0);
-    s = fma(theta * z, ps, theta);
-    double pc = -1.0 / 6402373705728000.0;  // -1/18!
-    pc = fma(pc, z, 1.0 / 20922789888000.0);
-    pc = fma(pc, z, -1.0 / 87178291200.0);
-    pc = fma(pc, z, 1.0 / 479001600.0);
-    pc = fma(pc, z, -1.0 / 3628800.0);
-    pc = fma(pc, z, 1.0 / 40320.0);
-    pc = fma(pc, z, -1.0 / 720.0);
-    pc = fma(pc, z, 1.0 / 24.0);
-    pc = fma(pc, z, -0.5);
-    c = fma(z, pc, 1.0);
+// Roots and reciprocals in FP64 by Newton steps from an FP32 start: the FP64 pipe does 1.6 operations a clock on an
+// SM, and what bounds the return mapping is their number.  A square root and its reciprocal together take six, a
+// reciprocal three (a division of the compiler's takes about eight, measured as time); errors below 1.5 ulp.
+// Arguments outside FP32's comfortable range (zero, negative, not finite) take the routines.
+__device__ __forceinline__ bool f32_range(double x) {
+    const int e = (__double2hiint(x) >> 20) - 1023;
+    return e > -110 && e < 110;
+}
+// root = sqrt(x), inv = 1 / sqrt(x): with e = 1 - x v^2, v <- v (1 + e / 2 + 3 e^2 / 8)
+__device__ __forceinline__ void roots_newton(double x, double &root, double &inv) {
+    if (!f32_range(x)) {
+        root = sqrt(x);
+        inv = 1.0 / root;
+        return;
+    }
+    const double v = f32_widen(rsqrtf(df_from_f64(x).hi));
+    const double g = x * v, e = fma(-g, v, 1.0), c = e * fma(0.375, e, 0.5);
+    root = fma(g, c, g);
+    inv = fma(v, c, v);
+}
+__device__ __forceinline__ double recip_newton(double x) {
+    if (!f32_range(fabs(x))) return 1.0 / x;
+    const double r = f32_widen(1.0f / df_from_f64(x).hi);
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// Invariants of the deviator of the symmetric tensor t = [11, 22, 33, 12, 23, 13]: Q = J2 / 3, R = -J3 / 2.
+struct Deviator {
+    double I1, third, Q, R;
+};
+__device__ __forceinline__ Deviator deviator_invariants(const double *t) {
+    Deviator d;
+    d.I1 = t[0] + t[1] + t[2];
+    d.third = d.I1 * (1.0 / 3.0);
+    const double a = t[0] - d.third, b = t[1] - d.third, c = t[2] - d.third;
+    const double sq = fma(a, a, fma(b, b, c * c)), sh = fma(t[3], t[3], fma(t[4], t[4], t[5] * t[5]));
+    d.Q = fma(sq, 1.0 / 6.0, sh * (1.0 / 3.0));
+    const double bc = fma(b, c, -(t[4] * t[4])), m1 = fma(t[3], c, -(t[4] * t[5])), m2 = fma(t[3], t[4], -(t[5] * b));
+    d.R = -0.5 * fma(a, bc, fma(-t[3], m1, t[5] * m2));
+    return d;
+}
+
+// Ordered principal values third + rq (cos(a) + sqrt(3) sin(a)), third + rq (cos(a) - sqrt(3) sin(a)),
+// third - 2 rq cos(a) for the Lode angle a = acos(c) / 3 (c clamped to [-1, 1]).  With phi = acos(|c|) / 3 in
+// [0, pi/6], y = cos(phi) is the root of 4 y^3 - 3 y = |c| in [0.86, 1], where its slope is at least 6, so an FP32
+// estimate and two Newton steps give it: ten multiply-adds against the forty of an FP64 acos and series for sine
+// and cosine.  The steps are on w = 1 - y, which keeps its own digits near an edge:
+// w (9 - 12 w + 4 w^2) = 1 - |c|, sin(phi)^2 = w (2 - w).  c < 0 is a = pi/3 - phi: the values' signs and order
+// reversed.  Returns 1 or 2 where e1, e2 or e2, e3 are a close pair (phi < 2^-7.5, their gap below a fiftieth of
+// rq), else 0.
+__device__ __forceinline__ int lode_values(double c, double rq, double third, double &e1, double &e2, double &e3) {
+    const bool reversed = __double2hiint(c) < 0;
+    c = fabs(c);
+    const bool repeated = __double2hiint(c) >= 0x3FF00000;  // |c| >= 1, or NaN
+    const float y0 = __cosf(acosf(repeated ? 1.0f : df_from_f64(c).hi) * (1.0f / 3.0f));
+    const double slope = f32_widen(1.0f / fmaf(12.0f * y0, y0, -3.0f)), c1 = 1.0 - c;
+    double w = f32_widen(1.0f - y0);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) w = fma(fma(-fma(fma(4.0, w, -12.0), w, 9.0), w, c1), slope, w);
+    if (repeated) w = 0.0;
+    const double s2 = fma(-w, w, w + w);
+    double z = 0.0;
+    if (__double2hiint(s2) > 0) {  // sin(phi) by Newton steps on z^2 = s2
+        const float r = sqrtf(df_from_f64(s2).hi);
+        const double h = f32_widen(0.5f / r);
+        z = f32_widen(r);
+        z = fma(fma(-z, z, s2), h, z);
+        z = fma(fma(-z, z, s2), h, z);
+    }
+    const double y = reversed ? w - 1.0 : 1.0 - w;
+    const double a = rq * y, b = rq * (1.7320508075688772 * z);
+    const double ta = third + a, hi = ta + b, lo = ta - b, single = fma(-2.0, a, third);
+    e1 = reversed ? single : hi;
+    e2 = reversed ? hi : lo;
+    e3 = reversed ? lo : single;
+    return __double2hiint(s2) >= 0x3F000000 ? 0 : 1 + reversed;
+}
+
+// t t (the squared tensor) as [11, 22, 33, 12, 23, 13].  Contractions are written out here and on the way to the
+// stresses, so that every kernel that shares this code has the same bits.
+__device__ __forceinline__ void square3(const double *t, double *sq) {
+    sq[0] = fma(t[0], t[0], fma(t[3], t[3], t[5] * t[5]));
+    sq[1] = fma(t[1], t[1], fma(t[3], t[3], t[4] * t[4]));
+    sq[2] = fma(t[2], t[2], fma(t[4], t[4], t[5] * t[5]));
+    sq[3] = fma(t[3], t[0] + t[1], t[4] * t[5]);
+    sq[4] = fma(t[4], t[1] + t[2], t[3] * t[5]);
+    sq[5] = fma(t[5], t[0] + t[2], t[3] * t[4]);
+}
+
+// The close pair (hi, lo) of t's principal values again, from its third one: an ulp of the invariants moves the pair
+// by ulp / (gap / rq), and the tangent divides by the gap twice more.  With the pair at m +- b and the third at
+// m - 3a, N = t - m has the values +-b and -3a, N (N + 3a) has b (b + 3a), b (b - 3a) and 0, and its squared
+// Frobenius norm F = b^2 (18 a^2 + 2 b^2) gives b to a few ulps of the largest value.
+__device__ __forceinline__ void refine_pair(const double *t, double third, double single, double &hi, double &lo) {
+    const double a = 0.5 * (third - single), m = third + a, a3 = 3.0 * a;
+    double n[6], sq[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) n[i] = i < 3 ? t[i] - m : t[i];
+    square3(n, sq);
+    double f = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const double v = fma(a3, n[i], sq[i]);
+        f = fma(i < 3 ? v : 2.0 * v, v, f);
+    }
+    const double b0 = 0.5 * (hi - lo);
+    double b, inv;
+    roots_newton(f * recip_newton(fma(2.0 * b0, b0, 18.0 * a * a)), b, inv);
+    hi = m + b;
+    lo = m - b;
 }
 
 // Elastic screen from invariants, before any eigen-decomposition, in FP32.  With principal trial

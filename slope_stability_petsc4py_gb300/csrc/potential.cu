@@ -50,26 +50,26 @@ __device__ __forceinline__ int mc_potential(double e1, double e2, double e3, dou
         psi = vol + G * (e1 * e1 + e2 * e2 + e3 * e3);
         return 0;
     }
-    // each bound where its branch is tested: an FP64 division costs as much as five multiply-adds here
-    const double g_sl = (e1 - e2) / np_maximum(1.0e-15, 1.0 + s);
-    const double g_sr = (e2 - e3) / np_maximum(1.0e-15, 1.0 - s);
+    // the bounds g = a / p (p > 0) cross-multiplied: an FP64 division costs as much as eight multiply-adds here
+    const double a_sl = e1 - e2, p_sl = np_maximum(1.0e-15, 1.0 + s);
+    const double a_sr = e2 - e3, p_sr = np_maximum(1.0e-15, 1.0 - s);
     const double l_s = f_tr / safe_denominator(d_s);
-    if (l_s <= g_sl && l_s <= g_sr) {  // lambda_s <= np.minimum(g_sl, g_sr), NaN-failing
+    if (l_s * p_sl <= a_sl && l_s * p_sr <= a_sr) {  // lambda_s <= np.minimum(g_sl, g_sr), NaN-failing
         psi = vol + G * (e1 * e1 + e2 * e2 + e3 * e3) - 0.5 * d_s * (l_s * l_s);
         return 1;
     }
     const double lin = 2.0 * L * s * tr - c;
-    if (g_sl < g_sr) {
+    if (a_sl * p_sr < a_sr * p_sl) {
         const double l_l = (G * ((1.0 + s) * (e1 + e2) - 2.0 * (1.0 - s) * e3) + lin) / safe_denominator(d_l);
-        if (l_l >= g_sl && l_l <= (e1 + e2 - 2.0 * e3) / np_maximum(1.0e-15, 3.0 - s)) {
+        if (l_l * p_sl >= a_sl && l_l * np_maximum(1.0e-15, 3.0 - s) <= e1 + e2 - 2.0 * e3) {
             const double h = e1 + e2;
             psi = vol + G * (e3 * e3 + 0.5 * (h * h)) - 0.5 * d_l * (l_l * l_l);
             return 2;
         }
     }
-    if (g_sl > g_sr) {
+    if (a_sl * p_sr > a_sr * p_sl) {
         const double l_r = (G * (2.0 * (1.0 + s) * e1 - (1.0 - s) * (e2 + e3)) + lin) / safe_denominator(d_r);
-        if (l_r >= g_sr && l_r <= (2.0 * e1 - e2 - e3) / np_maximum(1.0e-15, 3.0 + s)) {
+        if (l_r * p_sr >= a_sr && l_r * np_maximum(1.0e-15, 3.0 + s) <= 2.0 * e1 - e2 - e3) {
             const double h = e2 + e3;
             psi = vol + G * (e1 * e1 + 0.5 * (h * h)) - 0.5 * d_r * (l_r * l_r);
             return 3;
@@ -86,28 +86,14 @@ __device__ __forceinline__ int point_potential(const double *__restrict__ E, dou
                                                double L, double &psi) {
     const double s2 = s * s;
     if (DIM == 3) {
-        const double e11 = E[0], e22 = E[1], e33 = E[2], r3 = E[3], r4 = E[4], r5 = E[5];
-        const double I1 = e11 + e22 + e33;
-        const double I2 = e11 * e22 + e11 * e33 + e22 * e33 - r3 * r3 - r4 * r4 - r5 * r5;
-        const double I3 = e11 * e22 * e33 - e33 * r3 * r3 - e22 * r4 * r4 - e11 * r5 * r5 + 2.0 * r3 * r4 * r5;
-        // divisions by constants as products with the rounded reciprocals, sqrt(Q^3) as sqrt(Q) Q (an ulp)
-        const double Q = np_maximum(0.0, (I1 * I1 - 3.0 * I2) * (1.0 / 9.0));
-        const double R = (-2.0 * (I1 * I1 * I1) + 9.0 * I1 * I2 - 27.0 * I3) * (1.0 / 54.0);
-        const double rq = sqrt(Q);
-        double theta = 0.0;
-        if (Q > 0.0) {
-            double t = R / np_maximum(1.0e-15, rq * Q);
-            t = t < -1.0 ? -1.0 : (t > 1.0 ? 1.0 : t);
-            theta = acos(t) * (1.0 / 3.0);
-        }
-        const double third = I1 * (1.0 / 3.0);
-        // cos(theta +- 2 pi / 3) from one sine and cosine
-        double st, ct;
-        ssp::sincos_lode(theta, st, ct);
-        const double rs = 1.7320508075688772 * st;
-        const double e1 = rq * (ct + rs) + third;
-        const double e2 = rq * (ct - rs) + third;
-        const double e3 = -2.0 * rq * ct + third;
+        const double t[6] = {E[0], E[1], E[2], E[3], E[5], E[4]};
+        const ssp::Deviator d = ssp::deviator_invariants(t);
+        double rq, v, e1, e2, e3;
+        ssp::roots_newton(d.Q, rq, v);
+        // R / max(1e-15, sqrt(Q^3)), and an angle of 0 where Q is 0
+        const double c3 = v * v * v;
+        ssp::lode_values(d.Q > 0.0 ? d.R * (c3 > 1.0e15 ? 1.0e15 : c3) : 1.0, rq, d.third, e1, e2, e3);
+        const double I1 = d.I1;
         const double d_s = 4.0 * L * s2 + 4.0 * G * (1.0 + s2);
         const double d_l = 4.0 * L * s2 + G * (1.0 + s) * (1.0 + s) + 2.0 * G * (1.0 - s) * (1.0 - s);
         const double d_r = 4.0 * L * s2 + 2.0 * G * (1.0 + s) * (1.0 + s) + G * (1.0 - s) * (1.0 - s);
@@ -147,9 +133,9 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
 
 // 3D: the FP32 elastic screen of the return mapping (screen_elastic, whose bound holds for every Lode angle)
 // settles the points it proves elastic from two invariants: e1^2 + e2^2 + e3^2 = I1^2 - 2 I2, the sum of the
-// squared tensor entries.  The others queue up in shared memory, 32 to a warp, and take the eigenvalues'
-// acos and square root as full warps: with a tenth of the points listed nearly every warp paid for them
-// (613 us for 1.1 M points, now 160).  A warp's queue fills in point order, so the sums are the same in
+// squared tensor entries.  The others queue up in shared memory, 32 to a warp, and take the eigenvalues
+// as full warps: with a tenth of the points listed nearly every warp paid for them (613 us for 1.1 M points, now
+// 131).  A warp's queue fills in point order, so the sums are the same in
 // every run.
 template <int DIM>
 __global__ void __launch_bounds__(kBlock, 5) potential_kernel(const double *__restrict__ E, const double *__restrict__ c_bar,
