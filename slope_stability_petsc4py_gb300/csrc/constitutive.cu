@@ -118,14 +118,15 @@ __device__ __forceinline__ Decision3 decide3(const Principal3 &p, const Mat3 &m)
     return {kApex, 0.0, 1.0};
 }
 
-// Elastic branch: S = lambda tr(E) I + 2 G t (t = E with halved shears), DS = the elastic matrix.
-__device__ __forceinline__ void finish_elastic(const double *t, double I1, const Mat3 &m, double *S, double *DS) {
+// Elastic branch: S = lambda tr(E) I + 2 G t (t = E with halved shears, so G E for the shears), DS = the elastic
+// matrix.
+__device__ __forceinline__ void finish_elastic(const double *E, double I1, const Mat3 &m, double *S, double *DS) {
     const double shear = m.shear, lame = m.lame;
     const double lI1 = lame * I1, s2 = 2.0 * shear;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) S[i] = lI1 + s2 * t[i];
+    for (int i = 0; i < 3; ++i) S[i] = fma(s2, E[i], lI1);
 #pragma unroll
-    for (int i = 3; i < 6; ++i) S[i] = s2 * t[i];
+    for (int i = 3; i < 6; ++i) S[i] = shear * E[i];
     if (DS) {
 #pragma unroll
         for (int k = 0; k < 36; ++k) DS[k] = 0.0;
@@ -138,13 +139,6 @@ __device__ __forceinline__ void finish_elastic(const double *t, double I1, const
         store_sym(DS, 0, 2, lame);
         store_sym(DS, 1, 2, lame);
     }
-}
-
-// t (shears halved) and I1 of the trial strain, in FP64, as principal3 forms them.
-__device__ __forceinline__ void elastic_trial(const double *E, double *t, double &I1) {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) t[i] = half_ident(i) * E[i];
-    I1 = t[0] + t[1] + t[2];
 }
 
 // ---- consistent tangent of the plastic branches in double-float arithmetic (the mixed form)
@@ -365,7 +359,8 @@ __device__ void finish3(const Principal3 &p, const Decision3 &d, const Mat3 &m, 
     const double sp = m.sin_phi, sin_phi = m.sin_phi, shear = m.shear, lame = m.lame;
     const double e1 = p.e1, e2 = p.e2, e3 = p.e3, I1 = p.I1;
     if (d.branch == kElastic) {
-        finish_elastic(p.t, I1, m, S, DS);
+        const double E[6] = {p.t[0], p.t[1], p.t[2], 2.0 * p.t[3], 2.0 * p.t[4], 2.0 * p.t[5]};
+        finish_elastic(E, I1, m, S, DS);
         return;
     }
     if (d.branch == kApex) {
@@ -530,10 +525,8 @@ __device__ void finish3(const Principal3 &p, const Decision3 &d, const Mat3 &m, 
 __device__ int mc3d_point(const double *E, double c_bar, double sin_phi, double shear, double lame, double *S,
                           double *DS) {
     const Mat3 m{c_bar, sin_phi, shear, lame};
-    if (screen_elastic(E, m)) {
-        double t[6], I1;
-        elastic_trial(E, t, I1);
-        finish_elastic(t, I1, m, S, DS);
+    if (screen_elastic<false>(E, m)) {
+        finish_elastic(E, E[0] + E[1] + E[2], m, S, DS);
         return kElastic;
     }
     Principal3 p;
@@ -687,10 +680,9 @@ __global__ void __launch_bounds__(128) mc3d_bin_kernel(const double *__restrict_
         double e[6];
         load6(E, p, e);
         const Mat3 m{c_bar[p], sin_phi[p], shear[p], lame[p]};
-        if (screen_elastic(e, m)) {
-            double t[6], I1, s[6], ds[36];
-            elastic_trial(e, t, I1);
-            finish_elastic(t, I1, m, s, WRITE_EL ? ds : nullptr);
+        if (screen_elastic<false>(e, m)) {
+            double s[6], ds[36];
+            finish_elastic(e, e[0] + e[1] + e[2], m, s, WRITE_EL ? ds : nullptr);
             store6(S, p, s);
             if (WRITE_EL) {
 #pragma unroll

@@ -188,8 +188,9 @@ __global__ void __launch_bounds__(kBlock, 5) potential_kernel(const double *__re
             double e[6];
             load(p, e);
             const ssp::Mat3 m{c_bar[p], sin_phi[p], shear[p], lame[p]};
-            const double t[6] = {e[0], e[1], e[2], 2.0 * e[3], 2.0 * e[4], 2.0 * e[5]};  // halved by the screen
-            if (ssp::screen_elastic(t, m)) {
+            // as tensor entries (12), (13), (23), halved by the screen
+            const double t[6] = {e[0], e[1], e[2], 2.0 * e[3], 2.0 * e[5], 2.0 * e[4]};
+            if (ssp::screen_elastic<true>(t, m)) {
                 const double tr = e[0] + e[1] + e[2];
                 const double sq = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + 2.0 * (e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
                 settle(p, 0.5 * m.lame * tr * tr + m.shear * sq, 0);
