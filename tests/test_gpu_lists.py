@@ -73,3 +73,25 @@ def test_gather_plastic_rows(cuda_device, n, entries):
     assert np.array_equal(b.cpu().numpy(), branch[pos])
     want = np.where((branch[pos] != 0)[:, None], ds[pos], -7.0)
     assert np.array_equal(rows.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("share", [1, 8])
+@pytest.mark.parametrize("n_rows,longest", [(1, 1), (31, 300), (33, 7), (1000, 90), (517, 700), (40000, 3)])
+def test_copy_marked_rows(cuda_device, n_rows, longest, share):
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+
+    rng = np.random.default_rng(n_rows)
+    lengths = rng.integers(0, longest + 1, n_rows)
+    indptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    src = torch.as_tensor(rng.standard_normal(int(indptr[-1]) + 1), device="cuda")[1:] if share == 1 else \
+        torch.as_tensor(rng.standard_normal(int(indptr[-1])), device="cuda")  # an odd start: 8-byte copies
+    for mark in (np.ones(n_rows), np.zeros(n_rows), rng.uniform(size=n_rows) < 0.5, np.arange(n_rows) % 32 == 31):
+        mark = mark.astype(np.uint8)
+        dst = torch.full_like(src, -7.0)
+        dev = [torch.as_tensor(a, device="cuda") for a in (indptr, mark)]
+        _lib.call("ssp_copy_rows_device_share", _lib.ptr(src), *(_lib.ptr(a) for a in dev), n_rows, int(src.numel()),
+                  _lib.ptr(dst), share, _lib.stream_handle())
+        on = np.repeat(mark != 0, lengths)
+        assert np.array_equal(dst.cpu().numpy(), np.where(on, src.cpu().numpy(), -7.0))
