@@ -13,14 +13,15 @@
 // at its 144-byte stride) feed 81 IMADs.  Two nodes a per thread halve the loads but need 168 registers: 11
 // warps an SM instead of 20, and 520 us against 425 on the P4 correction (before H was rounded by its largest).  Symmetric tangents take the pairs on
 // and above the diagonal (P2: 55, two warps; P4: 630, twenty warps), others all.
-//   1. gradients to 56 or 57 bits and D (correction: w-less DS - D_el by 60-bit subtraction) to 58, by the element's
-//      largest; w D rounded to 56
+//   1. gradients to 56 or 57 bits by their largest (P4: by the node's largest) and D (correction: w-less DS - D_el by 60-bit
+//      subtraction) to 58 by the element's; w D rounded to 56
 //   2. H[q][b][d][m] = sum_r D[m][row(d, r)] g_b,r for every point at once, kept as limbs
 //   3. K[(a,c),(b,d)] = sum_q sum_r g_a,r H[q][b][d][row(c, r)]; 72 terms at most: limbs of 28 bits, the lower
 //      one signed, so that the dropped products have no bias and both accumulators stay below 2^63
 //   4. the sums, at 57 bits or so, become FP64 and are reduced into the CSR values
-// The entries are as near the exact sums as FP64's (a model of these integers: 3e-17 against 1.3e-16 for P2
-// in the 2-norm, P4 6e-17 against 2.4e-16).
+// The entries are nearer the exact sums than FP64's (measured over distorted elements in the 2-norm: P2 0.8e-16 to
+// 1.0e-16 against 1.6e-16 to 2.6e-16, P4 2.0e-16 to 2.3e-16 against 2.8e-16 to 3.4e-16).  P4's nodes differ by an
+// order of magnitude in their gradients; with one exponent for all of an element's its tangent was at 4.0e-16.
 // An element whose inputs are not all finite takes the same sums in FP64.
 #include "fixed.cuh"
 #include "ssp_internal.cuh"
@@ -29,7 +30,7 @@ namespace ssp {
 namespace {
 
 constexpr int kLimb = 28;
-// Factors of 56 bits (P2's gradients 57), H's by the element's largest: 72 terms of H times g (P2 33) stay below
+// Factors of 56 bits (P2's gradients 57), H's by the element's or P4 node's largest: 72 terms of H times g (P2 33) stay below
 // 2^63 in both accumulators.
 
 struct Args {
@@ -61,6 +62,7 @@ struct Smem {
     int2 wl[NQ];
     unsigned long long mags[32];
     int exps[3][32];
+    int eg[NP], hb[NP];  // P4: a node's largest gradient exponent and bits of H
     int sq[NQ];
     int nq;
 };
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
     using Sh = Shape<NP, NQ, SYM>;
     constexpr int kThreads = Sh::kThreads, kWarps = kThreads / 32, kNld = 3 * NP;
     constexpr int kBitsG = NQ * 3 <= 36 ? 57 : 56;
+    constexpr bool kByNode = NP > 10;
     constexpr int kGradRounds = (NQ * NP + kThreads - 1) / kThreads, kDRounds = (NQ * 36 + kThreads - 1) / kThreads;
     extern __shared__ __align__(16) unsigned char fx_raw[];
     Smem<NP, NQ> &S = *reinterpret_cast<Smem<NP, NQ> *>(fx_raw);
@@ -150,6 +153,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
             if (on) S.sq[__popc(mask & ((1u << lane) - 1u))] = lane;
             if (lane == 0) S.nq = __popc(mask);
         }
+        if (kByNode && tid < NP) S.eg[tid] = S.hb[tid] = 0;
         for (int i = tid; i * 32 < kNld * kNld; i += kThreads)  // the map, needed last
             asm volatile("prefetch.global.L2 [%0];" ::"l"(em + i * 32));
         __syncthreads();
@@ -186,7 +190,11 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
             }
         }
 #pragma unroll
-        for (int u = 0; u < kGradRounds; ++u) ex_g = max(ex_g, max(fx_exponent(gv[u][0]), max(fx_exponent(gv[u][1]), fx_exponent(gv[u][2]))));
+        for (int u = 0; u < kGradRounds; ++u) {
+            const int i = tid + u * kThreads, ex = max(fx_exponent(gv[u][0]), max(fx_exponent(gv[u][1]), fx_exponent(gv[u][2])));
+            if (kByNode && i < nq * NP) atomicMax(&S.eg[i % NP], ex);
+            ex_g = max(ex_g, ex);
+        }
 #pragma unroll
         for (int u = 0; u < kDRounds; ++u) ex_d = max(ex_d, fx_exponent(dv[u]));
         ex_d = max(ex_d, max(fx_exponent(g_pt), fx_exponent(l_pt)));
@@ -206,7 +214,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
             if (i < nq * NP) {
                 const int k = i / NP;
 #pragma unroll
-                for (int r = 0; r < 3; ++r) S.g[k][i - k * NP][r] = fx_split<kLimb>(fx_round<60 - kBitsG>(fx_from_f64(gv[u][r], e_g, 60)));
+                for (int r = 0; r < 3; ++r) S.g[k][i - k * NP][r] = fx_split<kLimb>(fx_round<60 - kBitsG>(fx_from_f64(gv[u][r], kByNode ? S.eg[i - k * NP] : e_g, 60)));
             }
         }
         if (tid < nq) {
@@ -249,6 +257,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
         for (int i = tid; i < nq * kNld; i += kThreads) {
             const int k = i / kNld, be = i - k * kNld, n = be / 3, d = be - 3 * n;
             int2 gr[3];
+            if (kByNode) mag = 0;
 #pragma unroll
             for (int r = 0; r < 3; ++r) gr[r] = S.g[k][n][r];
             int4 *out = reinterpret_cast<int4 *>(&S.H[k][n][6 * d]);
@@ -268,12 +277,14 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
                 out[m] = make_int4(static_cast<int>(hs), static_cast<int>(hs >> 32), static_cast<int>(ht),
                                    static_cast<int>(ht >> 32));
             }
+            if (kByNode) atomicMax(&S.hb[n], 64 - __clzll(static_cast<long long>(mag)));
         }
-        block_or(mag);
+        if (!kByNode) block_or(mag);
         __syncthreads();
-        const unsigned room_h = fx_room(64 - __clzll(static_cast<long long>(warps_or())));
+        const int h_bits = kByNode ? 0 : 64 - __clzll(static_cast<long long>(warps_or()));
         for (int i = tid; i < nq * NP * 9; i += kThreads) {
             int4 *p = reinterpret_cast<int4 *>(&S.H[0][0][0]) + i;
+            const unsigned room_h = fx_room(kByNode ? S.hb[i / 9 % NP] : h_bits);
             const int4 x = *p;
             const long long hs = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.y)) << 32 |
                                                         static_cast<unsigned>(x.x)),
@@ -284,9 +295,8 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
         }
         __syncthreads();
         // total = hh 2^56 + mid 2^28
-        const int unit_g = fx_unit(e_g, kBitsG);
         const int unit_wd = fx_unit(e_w, 58) + fx_unit(e_d, 60) + fx_top_unit<58>(room) + kFxDrop + 2;
-        const int unit_k = unit_wd + unit_g + 2 * kLimb + fx_top_unit<56>(room_h) + unit_g + 2 * kLimb;
+        const int unit_e = unit_wd + 4 * kLimb + 2 * fx_unit(0, kBitsG) + (kByNode ? 0 : 2 * e_g + fx_top_unit<56>(fx_room(h_bits)));
         const unsigned nnz32 = static_cast<unsigned>(A.nnz < 0x7FFFFFFFll ? A.nnz : 0x7FFFFFFFll);
         auto emit = [&](int32_t p, double v) {
             if (static_cast<unsigned>(p) < nnz32) red_add(A.values + p, v);
@@ -322,6 +332,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
                         for (int r = 0; r < 3; ++r) acc[c][d].add_prod(ga[r], h[kRow[c][r]]);
                 }
             }
+            const int unit_k = kByNode ? unit_e + S.eg[a] + S.eg[b] + fx_top_unit<56>(fx_room(S.hb[b])) : unit_e;
             const int32_t *up = em + 3 * a * kNld + 3 * b, *low = em + 3 * b * kNld + 3 * a;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
