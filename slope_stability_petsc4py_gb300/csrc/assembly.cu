@@ -384,11 +384,12 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
                 else dS[m - 1][c] = fx_split<kLambdaLimb>(Sm[c] - S0[c]);
             }
         }
-        // the coordinates sum to one: E(q) = S_0 + sum_{m>=1} lambda_qm (S_m - S_0)
+        // the coordinates sum to one: E(q) = S_0 + sum_{m>=1} lambda_qm (S_m - S_0), with two bits more than the
+        // product sums' unit (S is below 2^60)
         const int unit_S = fx_unit(e_u, 60) - s + 8 + fx_unit(e_j, 58) + kFxDrop, shift_0 = fx_unit(e_lam, 58) + 2 * kLambdaLimb;
-        const int unit_E = unit_S + shift_0;
+        const int unit_E = unit_S + shift_0 - 2;  // shift_0 >= 2
 #pragma unroll
-        for (int c = 0; c < 6; ++c) S0[c] >>= min(shift_0, 63);
+        for (int c = 0; c < 6; ++c) S0[c] >>= min(shift_0 - 2, 63);
 #pragma unroll 1
         for (int q = 0; q < n_q; ++q) {
             const int2 l1 = s_lam[3 * q], l2 = s_lam[3 * q + 1], l3 = s_lam[3 * q + 2];
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
                 FxSum t(dS[0][c], l1);
                 t.add_prod(dS[1][c], l2);
                 t.add_prod(dS[2][c], l3);
-                v[c] = fx_to_f64(t.value<kLambdaLimb>() + S0[c], unit_E);
+                v[c] = fx_to_f64(t.value_up<kLambdaLimb, 2>() + S0[c], unit_E);
             }
             double2 *o = reinterpret_cast<double2 *>(out + 6 * q);
             o[0] = make_double2(v[0], v[1]);

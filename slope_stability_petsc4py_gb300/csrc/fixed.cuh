@@ -119,6 +119,9 @@ struct FxSum {
     }
     template <int LIMB = kFxLimb>
     __device__ __forceinline__ long long value() const { return hh + fx_round<LIMB>(mid); }
+    // the same with UP bits more, where hh has them to spare
+    template <int LIMB, int UP>
+    __device__ __forceinline__ long long value_up() const { return (hh << UP) + fx_round<LIMB - UP>(mid); }
 };
 
 }  // namespace ssp
