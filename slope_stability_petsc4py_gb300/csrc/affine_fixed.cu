@@ -2,8 +2,9 @@
 // strain3_affine_kernel and force3_affine_kernel (assembly.cu), whose FP64 form took 197 and 160 us on 10,374
 // elements at that pipe's rate (now 66 and 81).  Each is a product with the reference element's gradient table, the same for
 // every element (strain: 34 nodes x 9 products a point, force: 24 points x 9 a node), so a block converts the
-// table once, keeps it in shared memory and strides over groups of elements.  Products of 55-bit values in
-// limbs of 28 bits, the lower one signed (up to 120 terms without bias or overflow; a total's hh 2^56 + mid 2^28 is kept from 2^54 up); one exponent per element for each input.
+// table once, keeps it in shared memory and strides over groups of elements.  Products of values of 55 bits
+// (strain: 56) in limbs of 28, the lower one signed: up to 120 terms without bias or overflow; a total's
+// hh 2^56 + mid 2^28 is kept from 2^54 up where it has the room.  One exponent per element for each input.
 // An element whose inputs are not all finite takes the FP64 sums.
 #include "fixed.cuh"
 #include "ssp_internal.cuh"
@@ -12,9 +13,10 @@ namespace ssp {
 namespace {
 
 constexpr int kStrainThreads = 192, kForceThreads = 352;  // P4: 8 elements of 24 points, 10 of 35 nodes
-constexpr int kBits = 55;
+constexpr int kBits = 55, kStrainBits = 56;
 
 // the table's exponent (every thread of the block), its limbs into s_ghat; syncs
+template <int BITS>
 __device__ __forceinline__ int load_table(const double *ghat, int n, int2 *s_ghat, int *s_exp) {
     if (threadIdx.x == 0) *s_exp = 0;
     __syncthreads();
@@ -25,7 +27,7 @@ __device__ __forceinline__ int load_table(const double *ghat, int n, int2 *s_gha
     __syncthreads();
     e = *s_exp;
     if (e < 2047)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) s_ghat[i] = fx_split<28>(fx_round<60 - kBits>(fx_from_f64(ghat[i], e, 60)));
+        for (int i = threadIdx.x; i < n; i += blockDim.x) s_ghat[i] = fx_split<28>(fx_round<60 - BITS>(fx_from_f64(ghat[i], e, 60)));
     return e;
 }
 
@@ -44,7 +46,7 @@ __global__ void __launch_bounds__(kStrainThreads, 3) strain3_affine_fixed_kernel
     ElementUnits *s_e = reinterpret_cast<ElementUnits *>(s_j + group * 9);
     int *s_exp = reinterpret_cast<int *>(s_e + group);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int e_t = load_table(ghat, n_table, s_ghat, s_exp);
+    const int e_t = load_table<kStrainBits>(ghat, n_table, s_ghat, s_exp);
     const int n_groups = (n_elem + group - 1) / group;
     for (int gi = blockIdx.x; gi < n_groups; gi += gridDim.x) {
         const long long e0 = (long long)gi * group;
@@ -92,11 +94,11 @@ __global__ void __launch_bounds__(kStrainThreads, 3) strain3_affine_fixed_kernel
                     const int2 x = s_d[k * nld + i];
                     const long long d = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.y)) << 32 |
                                                                static_cast<unsigned>(x.x));
-                    s_d[k * nld + i] = fx_split<28>(fx_round<62 - kBits>(fx_scale(d, room)));
+                    s_d[k * nld + i] = fx_split<28>(fx_round<62 - kStrainBits>(fx_scale(d, room)));
                 }
                 if (lane < 9) s_j[k * 9 + lane] = fx_split(fx_from_f64(jv, e_j, 58));
                 if (lane == 0)
-                    s_e[k] = {fx_unit(e_u, 60) + fx_top_unit<kBits>(room) + fx_unit(e_t, kBits) + 54 + fx_unit(e_j, 58) + kFxDrop, 1};
+                    s_e[k] = {fx_unit(e_u, 60) + fx_top_unit<kStrainBits>(room) + fx_unit(e_t, kStrainBits) + 56 + fx_unit(e_j, 58) + kFxDrop, 1};
             } else if (lane == 0) {
                 s_e[k] = {0, 0};
             }
@@ -119,8 +121,13 @@ __global__ void __launch_bounds__(kStrainThreads, 3) strain3_affine_fixed_kernel
                 long long v[9];
                 unsigned long long mag = 0;
 #pragma unroll
+                for (int x = 0; x < 9; ++x) mag |= fx_mag(G[x / 3][x % 3].hh);
+                const bool small = __clzll(static_cast<long long>(mag)) >= 4;  // two bits to spare
+                mag = 0;
+#pragma unroll
                 for (int x = 0; x < 9; ++x) {
-                    v[x] = (G[x / 3][x % 3].hh << 2) + fx_round<26>(G[x / 3][x % 3].mid);
+                    const FxSum &g = G[x / 3][x % 3];
+                    v[x] = small ? g.value_up<28, 2>() : g.value<28>();
                     mag |= fx_mag(v[x]);
                 }
                 const int lz = min(__clzll(static_cast<long long>(mag)), 63) - 6;  // to 58 bits
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(kStrainThreads, 3) strain3_affine_fixed_kernel
                     Gl[x / 3][x % 3] = fx_split((v[x] << up) >> down);
                     J[x / 3][x % 3] = s_j[k * 9 + x];
                 }
-                const int unit = s_e[k].unit - up + down;
+                const int unit = s_e[k].unit - (small ? 2 : 0) - up + down;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     FxSum n(Gl[c][0], J[0][c]);  // (G J^{-1})_cc
@@ -188,7 +195,7 @@ __global__ void __launch_bounds__(kForceThreads, 2) force3_affine_fixed_kernel(
     int *s_ex = reinterpret_cast<int *>(s_mag + group);                    // [group][3]: stress, weight, J^{-1}
     int *s_exp = s_ex + group * 3;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int e_t = load_table(ghat, n_table, s_ghat, s_exp);
+    const int e_t = load_table<kBits>(ghat, n_table, s_ghat, s_exp);
     const int n_groups = (n_elem + group - 1) / group;
     for (int gi = blockIdx.x; gi < n_groups; gi += gridDim.x) {
         const long long e0 = (long long)gi * group;
