@@ -89,12 +89,12 @@ __global__ void __launch_bounds__(kStrainThreads, 3) strain3_affine_fixed_kernel
                     mag |= fx_mag(d);
                     s_d[k * nld + i] = make_int2(static_cast<int>(d), static_cast<int>(d >> 32));
                 }
-                const unsigned room = fx_room(fx_warp_bits(mag));
+                const int room = fx_room(fx_warp_bits(mag));
                 for (int i = lane; i < nld; i += 32) {
                     const int2 x = s_d[k * nld + i];
                     const long long d = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.y)) << 32 |
                                                                static_cast<unsigned>(x.x));
-                    s_d[k * nld + i] = fx_split<28>(fx_round<62 - kStrainBits>(fx_scale(d, room)));
+                    s_d[k * nld + i] = fx_round_split<28, 62 - kStrainBits>(fx_scale(d, room));
                 }
                 if (lane < 9) s_j[k * 9 + lane] = fx_split(fx_from_f64(jv, e_j, 58));
                 if (lane == 0)
@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(kForceThreads, 2) force3_affine_fixed_kernel(
         for (int i = threadIdx.x; i < here * n_q * 9; i += kForceThreads) {
             const int k = i / (9 * n_q);
             if (!finite(k)) continue;
-            const unsigned room = fx_room(64 - __clzll(static_cast<long long>(s_mag[k])));
-            s_T[i] = fx_split<28>(fx_round<62 - kBits>(fx_scale(reinterpret_cast<long long *>(s_T)[i], room)));
+            const int room = fx_room(64 - __clzll(static_cast<long long>(s_mag[k])));
+            s_T[i] = fx_round_split<28, 62 - kBits>(fx_scale(reinterpret_cast<long long *>(s_T)[i], room));
         }
         __syncthreads();
         for (int i = threadIdx.x; i < here * n_p; i += kForceThreads) {
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kForceThreads, 2) force3_affine_fixed_kernel(
 #pragma unroll
                         for (int z = 0; z < 3; ++z) acc[a].add_prod(T[3 * a + z], g[z]);
                 }
-                const unsigned room = fx_room(64 - __clzll(static_cast<long long>(s_mag[k])));
+                const int room = fx_room(64 - __clzll(static_cast<long long>(s_mag[k])));
                 const int unit = fx_unit(s_ex[3 * k], 58) + fx_unit(s_ex[3 * k + 1], 58) + kFxDrop + fx_unit(s_ex[3 * k + 2], 58) +
                                  kFxDrop + fx_top_unit<kBits>(room) + fx_unit(e_t, kBits) + 54;
 #pragma unroll

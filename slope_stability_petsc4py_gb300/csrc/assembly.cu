@@ -1629,7 +1629,7 @@ __global__ void __launch_bounds__(32 * kMomWarps, 2) correction_p2_moment_kernel
         const long long vi = fx_from_f64(v_pt, e_v, kBitsRoom);  // 0 beyond lane 8
         long long v0 = -(vi + __shfl_down_sync(0xffffffffu, vi, 3) + __shfl_down_sync(0xffffffffu, vi, 6));
         if (lane >= 3) v0 = 0;
-        const unsigned room_v = fx_room(fx_warp_bits(fx_mag(vi) | fx_mag(v0)));
+        const int room_v = fx_room(fx_warp_bits(fx_mag(vi) | fx_mag(v0)));
         if (lane < 9) W.v[1 + lane / 3][lane % 3] = fx_split_top<kBitsV>(fx_scale(vi, room_v));
         if (lane < 3) W.v[0][lane] = fx_split_top<kBitsV>(fx_scale(v0, room_v));
         // D_el's entry, formed once where the element has one material
@@ -1655,7 +1655,7 @@ __global__ void __launch_bounds__(32 * kMomWarps, 2) correction_p2_moment_kernel
                 mag_d |= fx_mag(dd[kk]);
             }
         }
-        const unsigned room_d = fx_room(fx_warp_bits(mag_d));
+        const int room_d = fx_room(fx_warp_bits(mag_d));
         if (lane < 24) {
 #pragma unroll
             for (int kk = 0; kk < kMaxQ; ++kk)
@@ -1688,7 +1688,7 @@ __global__ void __launch_bounds__(32 * kMomWarps, 2) correction_p2_moment_kernel
 #pragma unroll
             for (int y = 0; y < 4; ++y)
                 if (lane < 30 && 4 * eg + y < 21) mag_m |= fx_mag(m[x][y].value());
-        const unsigned room_m = fx_room(fx_warp_bits(mag_m));
+        const int room_m = fx_room(fx_warp_bits(mag_m));
         __syncwarp();  // the inputs are dead: their storage becomes the moments
 #pragma unroll
         for (int y = 0; y < 4; ++y) {

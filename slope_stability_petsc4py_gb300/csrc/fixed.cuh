@@ -77,23 +77,34 @@ __device__ __forceinline__ int fx_warp_bits(unsigned long long mags) {
     if (hi) return 64 - __clz(hi);
     return 32 - __clz(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(mags)));
 }
-// x 2^s for 0 <= s < 32, s the same for a block (two multiply-adds instead of a 64-bit shift by a variable)
-__device__ __forceinline__ long long fx_scale(long long x, unsigned two_s) {
-    return x * static_cast<long long>(static_cast<unsigned long long>(two_s));
+// x 2^s for 0 <= s < 32: two funnel shifts (a 64-bit shift by a variable also looks at larger s)
+__device__ __forceinline__ long long fx_scale(long long x, int s) {
+    const unsigned lo = static_cast<unsigned>(x), hi = static_cast<unsigned>(static_cast<unsigned long long>(x) >> 32);
+    return static_cast<long long>(static_cast<unsigned long long>(__funnelshift_l(lo, hi, s)) << 32 | (lo << s));
 }
-// the power of two that brings a block of `bits` bits to 62, at most 2^31
-__device__ __forceinline__ unsigned fx_room(int bits) { return 1u << min(31, 62 - bits); }
+// the shift that brings a block of `bits` bits to 62, at most 31
+__device__ __forceinline__ int fx_room(int bits) { return min(31, 62 - bits); }
 // x 2^-s rounded: truncated operands have a bias that every product of a sum repeats (the full P2 contraction
 // with truncated 55-bit factors was 16 times as far from the exact sums as FP64; rounded to 56 it is nearer)
 template <int S>
 __device__ __forceinline__ long long fx_round(long long x) { return (x + (1ll << (S - 1))) >> S; }
-// x of up to 62 bits as limbs of x 2^(BITS - 62), rounded, and the exponent of that unit after fx_scale by two_s
+// fx_split<LIMB>(fx_round<S>(x)), its upper limb from x's upper word alone
+template <int LIMB, int S>
+__device__ __forceinline__ int2 fx_round_split(long long x) {
+    static_assert(LIMB + S > 32, "the rounding of the upper limb is in the upper word");
+    const long long w = x + (1ll << (S - 1));
+    const int wh = static_cast<int>(w >> 32), h = (wh + (1 << (LIMB + S - 33))) >> (LIMB + S - 32);
+    return make_int2(h, static_cast<int>(__funnelshift_r(static_cast<unsigned>(w), static_cast<unsigned>(wh), S) -
+                                         (static_cast<unsigned>(h) << LIMB)));
+}
+// x of up to 62 bits as limbs of x 2^(BITS - 62), rounded, and the exponent of that unit after fx_scale by s
 template <int BITS>
 __device__ __forceinline__ int2 fx_split_top(long long x) {
-    return fx_split(fx_round<62 - BITS>(x));
+    if constexpr (kFxLimb + 62 - BITS > 32) return fx_round_split<kFxLimb, 62 - BITS>(x);
+    else return fx_split(fx_round<62 - BITS>(x));
 }
 template <int BITS>
-__device__ __forceinline__ int fx_top_unit(unsigned two_s) { return (62 - BITS) - (31 - __clz(two_s)); }
+__device__ __forceinline__ int fx_top_unit(int s) { return (62 - BITS) - s; }
 
 // 32 x 32 -> 64-bit product and multiply-add, one IMAD.WIDE each (written out: from the C++ expressions the
 // compiler made about half as many instructions again)

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
         }
         block_or(mag);
         __syncthreads();
-        const unsigned room = fx_room(64 - __clzll(static_cast<long long>(warps_or())));
+        const int room = fx_room(64 - __clzll(static_cast<long long>(warps_or())));
 #pragma unroll
         for (int u = 0; u < kDRounds; ++u) {
             const int i = tid + u * kThreads;
@@ -284,13 +284,13 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
         const int h_bits = kByNode ? 0 : 64 - __clzll(static_cast<long long>(warps_or()));
         for (int i = tid; i < nq * NP * 9; i += kThreads) {
             int4 *p = reinterpret_cast<int4 *>(&S.H[0][0][0]) + i;
-            const unsigned room_h = fx_room(kByNode ? S.hb[i / 9 % NP] : h_bits);
+            const int room_h = fx_room(kByNode ? S.hb[i / 9 % NP] : h_bits);
             const int4 x = *p;
             const long long hs = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.y)) << 32 |
                                                         static_cast<unsigned>(x.x)),
                             ht = static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(x.w)) << 32 |
                                                         static_cast<unsigned>(x.z));
-            const int2 hl = fx_split<kLimb>(fx_round<6>(fx_scale(hs, room_h))), tl = fx_split<kLimb>(fx_round<6>(fx_scale(ht, room_h)));
+            const int2 hl = fx_round_split<kLimb, 6>(fx_scale(hs, room_h)), tl = fx_round_split<kLimb, 6>(fx_scale(ht, room_h));
             *p = make_int4(hl.x, hl.y, tl.x, tl.y);
         }
         __syncthreads();
