@@ -333,16 +333,23 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
                 }
             }
             const int unit_k = kByNode ? unit_e + S.eg[a] + S.eg[b] + fx_top_unit<56>(fx_room(S.hb[b])) : unit_e;
+            // the tile's positions first (and its mirror's): behind a reduction each load would wait by itself
             const int32_t *up = em + 3 * a * kNld + 3 * b, *low = em + 3 * b * kNld + 3 * a;
+            int32_t pu[9], pl[9];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
+            for (int i = 0; i < 9; ++i) {
+                pu[i] = up[i / 3 * kNld + i % 3];
+                pl[i] = SYM && a != b ? low[i % 3 * kNld + i / 3] : -1;
+            }
+            if (SYM && a == b) {  // the upper triangle of a diagonal tile counts twice
+                pl[1] = pu[3], pl[2] = pu[6], pl[5] = pu[7];
+                pu[3] = pu[6] = pu[7] = -1;
+            }
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    if (SYM && a == b && c > d) continue;
-                    const double v = fx_to_f64(acc[c][d].value<kLimb>(), unit_k);
-                    emit(up[c * kNld + d], v);
-                    if (SYM && (a != b || c != d)) emit(low[d * kNld + c], v);
-                }
+            for (int i = 0; i < 9; ++i) {
+                const double v = fx_to_f64(acc[i / 3][i % 3].template value<kLimb>(), unit_k);
+                emit(pu[i], v);
+                if (SYM) emit(pl[i], v);
             }
         }
     }
