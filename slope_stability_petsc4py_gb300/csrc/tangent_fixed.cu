@@ -4,23 +4,23 @@
 //
 // In FP64 these contractions run at that pipe's 1.6 multiply-adds per clock and SM (full P2 contraction of
 // 19,200 elements 1,267 us, P4 correction of 2,150 plastic elements 1,362 us).  Here every product is three
-// 32 x 32 -> 64-bit IMADs and every sum exact until it is converted once: 485 and 455 us, the IMADs some 60 and
-// 45 % of their pipe's time, then the latency of the phases between barriers.  The P2 correction of 27,283
-// plastic elements takes 380 us (641 in FP64); the moment form (assembly.cu) is faster from three points up.
+// 32 x 32 -> 64-bit IMADs and every sum exact until it is converted once: 444 and 370 us, the IMADs 60 to 65 % of
+// their pipe's time, then the conversions and the latency of the phases between barriers.  The moment form of the P2
+// correction (assembly.cu) is faster from three points up.
 //
-// One CTA per element (grid-stride), one node pair of K_e per thread: 3 x 3 entries in 18 64-bit accumulators,
-// whose loads of a point (three gradients of node a, the H column of node b in nine 16-byte loads, conflict-free
+// One CTA per element or part of its points (grid-stride), one node pair of K_e per thread: 3 x 3 entries in 18
+// 64-bit accumulators, whose loads of a point (three gradients of node a, the H column of node b in nine 16-byte loads, conflict-free
 // at its 144-byte stride) feed 81 IMADs.  Two nodes a per thread halve the loads but need 168 registers: 11
-// warps an SM instead of 20, and 520 us against 425 on the P4 correction (before H was rounded by its largest).  Symmetric tangents take the pairs on
-// and above the diagonal (P2: 55, two warps; P4: 630, twenty warps), others all.
-//   1. gradients to 56 or 57 bits by their largest (P4: by the node's largest) and D (correction: w-less DS - D_el by 60-bit
+// warps an SM instead of 20, and a quarter more time on the P4 correction.  Symmetric tangents take the pairs on
+// and above the diagonal (P2: 55, two warps; P4: 630, seven warps in rounds), others all.
+//   1. gradients to 57 bits by their largest (P4: by the node's largest) and D (correction: w-less DS - D_el by 60-bit
 //      subtraction) to 58 by the element's; w D rounded to 56
 //   2. H[q][b][d][m] = sum_r D[m][row(d, r)] g_b,r for every point at once, kept as limbs
-//   3. K[(a,c),(b,d)] = sum_q sum_r g_a,r H[q][b][d][row(c, r)]; 72 terms at most: limbs of 28 bits, the lower
+//   3. K[(a,c),(b,d)] = sum_q sum_r g_a,r H[q][b][d][row(c, r)]; 36 terms at most: limbs of 28 bits, the lower
 //      one signed, so that the dropped products have no bias and both accumulators stay below 2^63
 //   4. the sums, at 57 bits or so, become FP64 and are reduced into the CSR values
 // The entries are nearer the exact sums than FP64's (measured over distorted elements in the 2-norm: P2 0.8e-16 to
-// 1.0e-16 against 1.6e-16 to 2.6e-16, P4 2.0e-16 to 2.3e-16 against 2.8e-16 to 3.4e-16).  P4's nodes differ by an
+// 1.0e-16 against 1.6e-16 to 2.6e-16, P4 1.1e-16 to 1.2e-16 against 2.8e-16 to 3.4e-16).  P4's nodes differ by an
 // order of magnitude in their gradients; with one exponent for all of an element's its tangent was at 4.0e-16.
 // An element whose inputs are not all finite takes the same sums in FP64.
 #include "fixed.cuh"
@@ -30,8 +30,8 @@ namespace ssp {
 namespace {
 
 constexpr int kLimb = 28;
-// Factors of 56 bits (P2's gradients 57), H's by the element's or P4 node's largest: 72 terms of H times g (P2 33) stay below
-// 2^63 in both accumulators.
+// Gradients of 57 bits, H of 56 by the element's or P4 node's largest: 36 terms of H times g stay below 2^63 in both
+// accumulators.
 
 struct Args {
     const double *d1, *d2, *d3, *DS, *w;
@@ -45,14 +45,23 @@ struct Args {
     const int32_t *elist, *elist_count;
 };
 
+// P4: 6.2 KB of shared memory a point of an element and 630 tiles.  A CTA of 12 points (half an element's) leaves room for
+// three of 7 warps an SM, so that one's barriers and conversions hide behind another's products: 370 us for the
+// correction of 2,150 elements against 399 of whole elements, a CTA of 20 warps an SM (two of 10: 379; thirds of
+// 5 or 7 warps: 412, 391).
+constexpr int kP4Threads = 224, kP4Parts = 2;
+
 template <int NP, int NQ, bool SYM>
 struct Shape {
     static constexpr int kTiles = SYM ? NP * (NP + 1) / 2 : NP * NP;
-    // P4's full matrix (1,225 tiles) in two rounds
-    static constexpr int kThreads = kTiles > 1024 ? 640 : (kTiles + 31) / 32 * 32;
-    static constexpr int kMinCtas = kThreads > 128 ? 1 : 640 / kThreads;  // 20 warps an SM (96 registers)
+    // 20 or 21 warps an SM (96 registers); P4's tiles in several rounds
+    static constexpr int kThreads = kTiles > 128 ? kP4Threads : (kTiles + 31) / 32 * 32;
+    static constexpr int kMinCtas = 672 / kThreads;
+    static constexpr int kParts = NQ > 12 ? kP4Parts : 1;  // an element's points, in parts
+    static constexpr int kPoints = (NQ + kParts - 1) / kParts;
 };
 
+// NQ: the points of a part
 template <int NP, int NQ>
 struct Smem {
     int2 g[NQ][NP][3];
@@ -108,11 +117,12 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
     tangent_fixed_kernel(Args A) {
     using Sh = Shape<NP, NQ, SYM>;
     constexpr int kThreads = Sh::kThreads, kWarps = kThreads / 32, kNld = 3 * NP;
-    constexpr int kBitsG = NQ * 3 <= 36 ? 57 : 56;
+    constexpr int kPoints = Sh::kPoints, kBitsG = 57;
+    static_assert(kPoints * 3 <= 36, "63 bits for the sums of a part");
     constexpr bool kByNode = NP > 10;
-    constexpr int kGradRounds = (NQ * NP + kThreads - 1) / kThreads, kDRounds = (NQ * 36 + kThreads - 1) / kThreads;
+    constexpr int kGradRounds = (kPoints * NP + kThreads - 1) / kThreads, kDRounds = (kPoints * 36 + kThreads - 1) / kThreads;
     extern __shared__ __align__(16) unsigned char fx_raw[];
-    Smem<NP, NQ> &S = *reinterpret_cast<Smem<NP, NQ> *>(fx_raw);
+    Smem<NP, kPoints> &S = *reinterpret_cast<Smem<NP, kPoints> *>(fx_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     auto block_max = [&](int which, int v) {  // written before, read after a barrier
@@ -138,8 +148,9 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
     };
 
     const long long n_iter = A.elist ? static_cast<long long>(*A.elist_count) : static_cast<long long>(A.n_elem);
-    for (long long it = blockIdx.x; it < n_iter; it += gridDim.x) {
-        const long long e = A.elist ? A.elist[it] : it;
+    for (long long item = blockIdx.x; item < Sh::kParts * n_iter; item += gridDim.x) {
+        const int part = Sh::kParts > 1 ? static_cast<int>(item / n_iter) : 0;
+        const long long it = item - part * n_iter, e = A.elist ? A.elist[it] : it;
         if (e < 0 || e >= A.n_elem) {  // uniform
             if (tid == 0) flag(SSP_DEV_BAD_INDEX);
             continue;
@@ -150,8 +161,11 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
         if (warp == 0) {
             const bool on = lane < NQ && (!CORR || A.branch[g0 + lane] != 0);
             const unsigned mask = __ballot_sync(0xffffffffu, on);
-            if (on) S.sq[__popc(mask & ((1u << lane) - 1u))] = lane;
-            if (lane == 0) S.nq = __popc(mask);
+            // the element's points in equal parts, no more of them than needed
+            const int all = __popc(mask), parts = (all + kPoints - 1) / kPoints, size = parts > 1 ? (all + parts - 1) / parts : all,
+                      k = __popc(mask & ((1u << lane) - 1u)) - part * size;
+            if (on && k >= 0 && k < size) S.sq[k] = lane;
+            if (lane == 0) S.nq = max(0, min(size, all - part * size));
         }
         if (kByNode && tid < NP) S.eg[tid] = S.hb[tid] = 0;
         for (int i = tid; i * 32 < kNld * kNld; i += kThreads)  // the map, needed last
@@ -359,15 +373,19 @@ template <int NP, int NQ, bool SYM, bool CORR>
 int launch(const Args &a, cudaStream_t st) {
     using Sh = Shape<NP, NQ, SYM>;
     auto kernel = tangent_fixed_kernel<NP, NQ, SYM, CORR>;
-    constexpr int smem = static_cast<int>(sizeof(Smem<NP, NQ>));
+    constexpr int smem = static_cast<int>(sizeof(Smem<NP, Sh::kPoints>));
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return SSP_ERR_CUDA;
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, Sh::kThreads, smem);
     if (per_sm < 1) per_sm = 1;
-    long long grid = (long long)sms * per_sm;
-    if (grid > a.n_elem) grid = a.n_elem;
+    // More CTAs than fit, so that the device hands them out as others end.  P4 corrections: 1 to 24 points an element
+    // (in one go 442 us for 2,150 elements, 8 times 399, 16 times 408); full tangents: no last wave (P2: 477 us in
+    // one go, 8 times 448, 16 times 444).  P2 corrections here have few points and a long list's empty CTAs cost
+    // more: 88 us in one go, 8 times 92.
+    long long grid = (long long)sms * per_sm * (a.elist ? (NP > 10 ? 8 : 1) : 16);
+    if (grid > Sh::kParts * (long long)a.n_elem) grid = Sh::kParts * (long long)a.n_elem;
     kernel<<<static_cast<unsigned>(grid), Sh::kThreads, smem, st>>>(a);
     return launch_status();
 }
