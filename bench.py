@@ -16,7 +16,8 @@ set moves from step to step.
   the host cores, on a bounded sample of the workload (contiguous runs of elements spread over the
   mesh, built as a mesh of their own), the same states.
 * ``roofline`` / ``roofline_fp64``: the dominant kernel's algorithmic bytes over its CUDA-event
-  time against the measured HBM bandwidth, and its FP64 operations against the live FP64 probe;
+  time against the measured HBM bandwidth, and its multiply-adds against the live FP64 probe (above 1
+  where a kernel forms them in fixed point on the integer pipe);
   ``kernel_rooflines`` the same for every step kernel.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--config 3d_p2_large] [--impl reference]
@@ -391,8 +392,8 @@ def algorithmic(name, st):
         return {"bytes": units * per_el, "flops": units * fl_el, "fp64": 2.0 * 22 * st["n_plastic_many"],
                 "units": f"{units:.0f} plastic elements in moment form per launch"}
     if name == "ssp_tangent_plastic_correction_p2_moments":
-        # elements at or above the split: 7,530 FP64 operations per element + 261 per plastic point
-        # (DS - D_el, weighted coordinate products, moments, beta^T M, R, the R sums, K), FMA-equivalent
+        # elements at or above the split: 7,530 operations per element + 261 per plastic point
+        # (DS - D_el, weighted coordinate products, moments, beta^T M, R, the R sums, K), counted as FP64 FMAs
         units = st["n_many_el"]
         return {"bytes": units * per_el, "flops": units * fl_el,
                 "fp64": 2.0 * (7530 * units + 261 * st["n_plastic_many"]),

@@ -227,7 +227,7 @@ __device__ __forceinline__ void sym_matvec(const double *M, const double *v, dou
 
 // Both kernels: one thread per element, one warp per CTA, in 58-bit fixed point (fixed.cuh; one exponent per
 // element for the displacement differences, the gradients, the stresses, ...).  In FP64 they were bound by
-// that pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 48 and 71, bound by the
+// that pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 54 and 78, bound by the
 // latency of 10 to 12 warps an SM of 160 registers and some 4,200 integer instructions an element).  E and the stresses pass
 // through shared memory, so that a warp's 32 elements are one contiguous block of global memory; elements
 // with an input that is not finite take the FP64 form of the same sums.
@@ -1353,7 +1353,8 @@ __global__ void fill_elastic_ds_kernel(const int8_t *__restrict__ branch, const 
 //   sums, K  integer additions; each K entry becomes FP64 once and is scattered to its two places
 // Bound by issue and latency at 16 warps an SM (registers and 13 KB of shared memory a warp): 3,900
 // instructions an element, 29 % of them in T and R, 24 % in K.  On 27,283 plastic elements of a
-// 100,800-element mesh 219 us by ncu where the FP64 form took 434 with its split (264 + 169 us).
+// 100,800-element mesh 219 us by ncu for all of them; 156 for the 17,000 from three points up and 88 for the others
+// in the direct form, where the FP64 forms took 264 + 169.
 constexpr int kMaxQ = 11;
 
 // packed upper-triangle index of (i, j) in an n x n symmetric matrix (row-major upper)

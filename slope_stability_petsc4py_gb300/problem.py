@@ -285,12 +285,13 @@ class ConstitutiveOperator:
         # plain form on straight-sided P2 tetrahedra: elements with at least this many plastic points
         # get their correction in moment form (ssp_tangent_plastic_correction_p2_moments), the others
         # point by point (ssp_tangent_plastic_correction); 0 disables it.  100,800 tetrahedra, 27 thousand
-        # of them plastic: both kernels take 252 us with 2, 248 with 3, 356 with 0.  The mixed form's
+        # of them plastic: a Newton iteration takes 575 us with 2 or 3, 592 with 4, 598 with 5.  The mixed form's
         # moment kernel (FP32 after the FP64 DS - D_el) costs less than its point-by-point kernel from
         # one plastic point up: every plastic element by default.
         self.moment_min_points = 3
         self.moment_min_points_mixed = 1
-        # "plain": FP64 throughout (the drop-in, parity 1e-12 with the reference);
+        # "plain": FP64 inputs, results and return mapping, contractions in FP64 or as exact as it
+        # (58-bit fixed point, csrc/fixed.cuh; the drop-in, parity 1e-12 with the reference);
         # "mixed": the plastic-point tangent products in FP32 (CUDA cores for P1/P2, tensor cores
         # for P4) with H = w D B formed in compensated double-float arithmetic, and the 3D strain and
         # force in compensated double-float arithmetic (~1e-13); the return mapping and every CSR /
