@@ -258,6 +258,8 @@ def prepare_bddc_subdomain_pattern(coord, elem, q_mask, material_identifier, mat
     t2 = perf_counter()
     dev["scatter_map"] = _lib.to_device(np.ascontiguousarray(s["scatter_map"]), t.int32)
     dev["cdiag"] = _lib.to_device(s["constrained_diag_positions"], t.int32)
+    # the subdomain's points in the owned evaluation (empty if prepared without its ordering)
+    dev["overlap_positions"] = _lib.to_device(s["overlap_local_positions"], t.int32)
     dev["elastic_values"] = t.zeros(max(nnz, 1), dtype=f64, device="cuda")[:nnz]
     if n_el:
         _c0, _phi, _psi, shear, bulk, lame, _gamma = heterogenous_materials(

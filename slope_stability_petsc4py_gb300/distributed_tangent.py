@@ -347,6 +347,11 @@ def prepare_owned_tangent_pattern(coord, elem, q_mask, material_identifier, mate
     dev["cdiag"] = _lib.to_device(g["constrained_diag_positions"], t.int32)
     owned_free_rows = np.flatnonzero(owned_free).astype(np.int64)
     dev["owned_free_rows"] = _lib.to_device(owned_free_rows.astype(np.int32), t.int32)
+    # elem_row with a row's place among the owned free rows (every entry of elem_row is a free row or -1).  Made
+    # here like every table that operators share: the synchronisation below orders it before any stream's use
+    place = np.full(n_rows + 1, -1, dtype=np.int32)  # the last one for -1
+    place[owned_free_rows] = np.arange(owned_free_rows.size, dtype=np.int32)
+    dev["elem_free_row"] = _lib.to_device(place[g["elem_row"]], t.int32)
     overlap_global_dofs = (dim * np.repeat(ov_nodes, dim) + np.tile(np.arange(dim), ov_nodes.size)).astype(np.int64)
     _ensure_int32_capacity("global dofs", dim * n_nodes)
     dev["overlap_global_dofs32"] = _lib.to_device(overlap_global_dofs.astype(np.int32), t.int32)
@@ -632,20 +637,6 @@ def _local_field_aos(pattern, field, rows: int):
     return _lib.to_device(np.ascontiguousarray(f.T), t.float64)
 
 
-def _free_element_rows(pattern):
-    """elem_row with an owned row's place among the owned free rows instead of the row (every entry
-    of elem_row is a free row or -1); made once per pattern."""
-    d = pattern.device
-    if "elem_free_row" not in d:
-        t = _lib.torch()
-        n_rows = int(pattern.local_matrix_pattern.shape[0])
-        place = t.full((n_rows + 1,), -1, dtype=t.int32, device="cuda")  # the last one for -1
-        free = d["owned_free_rows"].long()
-        place[free] = t.arange(free.numel(), dtype=t.int32, device="cuda")
-        d["elem_free_row"] = place[d["elem_row"].long()]
-    return d["elem_free_row"]
-
-
 def owned_force_device(pattern, S_aos, *, mixed: bool = False, free: bool = False):
     """Owned internal force B^T (w S) on owned rows (constrained rows = 0), CUDA tensor (n_rows,);
     with free on the owned free rows only.  S_aos: a point's stresses in a row, of which the first
@@ -653,7 +644,7 @@ def owned_force_device(pattern, S_aos, *, mixed: bool = False, free: bool = Fals
     t = _lib.require_cuda()
     d = pattern.device
     if free:
-        rows, n_rows = _free_element_rows(pattern), int(d["owned_free_rows"].numel())
+        rows, n_rows = d["elem_free_row"], int(d["owned_free_rows"].numel())
     else:
         rows, n_rows = d["elem_row"], int(pattern.local_matrix_pattern.shape[0])
     F = t.empty(n_rows, dtype=t.float64, device="cuda")

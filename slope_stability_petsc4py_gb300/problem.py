@@ -900,16 +900,11 @@ class ConstitutiveOperator:
         return pattern
 
     def _bddc_positions(self, pattern):
-        """The subdomain's points in the owned evaluation (int64 and int32, device), or None where the
-        pattern was prepared without them."""
+        """The subdomain's points in the owned evaluation (int32, device), or None where the pattern was
+        prepared without them."""
         if int(pattern.overlap_local_positions.size) != int(pattern.local_int_indices.size):
             return None
-        d = pattern.device
-        if "overlap_positions" not in d:
-            t = _lib.torch()
-            d["overlap_positions"] = t.as_tensor(pattern.overlap_local_positions.astype(np.int64), device="cuda")
-            d["overlap_positions32"] = d["overlap_positions"].to(t.int32)
-        return d["overlap_positions"], d["overlap_positions32"]
+        return pattern.device["overlap_positions"]
 
     def _bddc_local_DS(self):
         """DS rows of the subdomain's points as an AoS CUDA tensor (n_local, n_strain^2): gathered
@@ -921,7 +916,7 @@ class ConstitutiveOperator:
             pos = self._bddc_positions(pattern)
             if pos is None:
                 raise RuntimeError("BDDC overlap-local integration-point map is incomplete")
-            return self._DS_aos.index_select(0, pos[0])
+            return self._DS_aos.index_select(0, pos)
         if self.DS is None:
             raise ValueError("Tangent DS not computed")
         ds = np.asarray(self.DS, dtype=np.float64)[:, pattern.local_int_indices]
@@ -989,8 +984,8 @@ class ConstitutiveOperator:
             d, pos = pattern.device, self._bddc_positions(pattern)
             ok = pos is not None and "shear" in d and "lame" in d
             if ok:
-                ok = bool(t.equal(self._dev["shear"].index_select(0, pos[0]), d["shear"])) and bool(
-                    t.equal(self._dev["lame"].index_select(0, pos[0]), d["lame"]))
+                ok = bool(t.equal(self._dev["shear"].index_select(0, pos), d["shear"])) and bool(
+                    t.equal(self._dev["lame"].index_select(0, pos), d["lame"]))
             self._bddc["predictor_ok"] = ok
         return self._bddc["predictor_ok"]
 
@@ -1022,7 +1017,7 @@ class ConstitutiveOperator:
                                               t.empty(1, dtype=t.int32, device="cuda"))
             elist, ecount = self._bddc["plastic_list"]
             _lib.call("ssp_gather_plastic_rows", _lib.ptr(self._branch), _lib.ptr(self._DS_aos),
-                      _lib.ptr(d["overlap_positions32"]), n, int(self._branch.numel()), pattern.n_strain ** 2,
+                      _lib.ptr(d["overlap_positions"]), n, int(self._branch.numel()), pattern.n_strain ** 2,
                       _lib.ptr(branch), _lib.ptr(ds), st)
             _lib.call("ssp_copy_device", _lib.ptr(d["elastic_values"]), int(values.numel()), _lib.ptr(values), st)
             _lib.call("ssp_plastic_elements", _lib.ptr(branch), n_el, pattern.n_q, _lib.ptr(elist), _lib.ptr(ecount), st)
