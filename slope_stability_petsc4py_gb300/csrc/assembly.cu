@@ -586,7 +586,8 @@ __device__ __noinline__ void force3_p2_nonfinite(const double *jinv, const doubl
         }
         for (int c = 0; c < 3; ++c) {
             const int row = er[3 * a + c];
-            if (row >= 0 && row < n_rows) red_add(F + row, f[c]);
+            if (row >= n_rows) flag(SSP_DEV_BAD_INDEX);
+            else if (row >= 0) red_add(F + row, f[c]);
         }
     }
 }
