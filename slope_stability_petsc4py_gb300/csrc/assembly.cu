@@ -231,36 +231,70 @@ __device__ __forceinline__ void sym_matvec(const double *M, const double *v, dou
 // latency of 10 to 12 warps an SM of 160 registers and some 4,200 integer instructions an element).  E and the stresses pass
 // through shared memory, so that a warp's 32 elements are one contiguous block of global memory; elements
 // with an input that is not finite take the FP64 form of the same sums.
-constexpr int kP2StageMaxQ = 30;  // points per element up to which a warp's block is staged (46 KiB)
+constexpr int kP2StageMaxQ = 30;  // points per element for which a warp's block fits (46 KiB); more take FP64
 
-__device__ __noinline__ void strain3_p2_nonfinite(const double *jinv, const double *bary, const double *u,
-                                                  const int32_t *dl, long long n_u, int n_q, double *out) {
-    for (int q = 0; q < n_q; ++q) {
-        double G[3][3] = {};
-        for (int a = 0; a < 10; ++a) {
-            double g[3];
-            for (int z = 0; z < 3; ++z) {
-                const double g0 = -(jinv[z] + jinv[3 + z] + jinv[6 + z]);
-                if (a < 4) {
-                    g[z] = (4.0 * bary[4 * q + a] - 1.0) * (a == 0 ? g0 : jinv[3 * (a - 1) + z]);
-                } else {
-                    const int i = (a == 5 || a == 7) ? 1 : (a == 8 ? 2 : 0), j = a == 4 ? 1 : (a == 5 || a == 6) ? 2 : 3;
-                    g[z] = 4.0 * (bary[4 * q + i] * jinv[3 * (j - 1) + z] + bary[4 * q + j] * (i == 0 ? g0 : jinv[3 * (i - 1) + z]));
-                }
-            }
-            for (int c = 0; c < 3; ++c) {
-                const int32_t i = dl[3 * a + c];
-                const double v = i < 0 || i >= n_u ? 0.0 : u[i];
-                for (int z = 0; z < 3; ++z) G[c][z] += v * g[z];
+// One element's strains in FP64: out [n_q][6].
+__device__ __noinline__ void strain3_p2_fp64(const double *jinv, const double *bary, const double *u, const int32_t *dl,
+                                             long long n_u, int n_q, double *out) {
+    double un[10][3];
+#pragma unroll
+    for (int a = 0; a < 10; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int32_t i = dl[3 * a + c];
+            if (i < 0 || i >= n_u) {
+                flag(SSP_DEV_BAD_INDEX);
+                un[a][c] = 0.0;
+            } else {
+                un[a][c] = u[i];
             }
         }
-        out[6 * q] = G[0][0];
-        out[6 * q + 1] = G[1][1];
-        out[6 * q + 2] = G[2][2];
-        out[6 * q + 3] = G[0][1] + G[1][0];
-        out[6 * q + 4] = G[1][2] + G[2][1];
-        out[6 * q + 5] = G[0][2] + G[2][0];
+    double gl[3][3];  // ∇λ_1..3
+#pragma unroll
+    for (int k = 0; k < 9; ++k) gl[k / 3][k % 3] = jinv[k];
+    // ∇u = Σ_m λ_m G_m, G_m = Σ_{i=1..3} (A_im − A_0m) ⊗ ∇λ_i, A_ii = 3u_i, A_im = 4u_(edge im) − u_i
+    double S[4][6];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        double A0[3], G[3][3] = {};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) A0[c] = m == 0 ? 3.0 * un[0][c] : 4.0 * un[p2_edge_node(0, m)][c] - un[0][c];
+#pragma unroll
+        for (int i = 1; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double Ai = i == m ? 3.0 * un[i][c] : 4.0 * un[p2_edge_node(i, m)][c] - un[i][c];
+                const double b = Ai - A0[c];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) G[c][k] += b * gl[i - 1][k];
+            }
+        S[m][0] = G[0][0];
+        S[m][1] = G[1][1];
+        S[m][2] = G[2][2];
+        S[m][3] = G[0][1] + G[1][0];
+        S[m][4] = G[1][2] + G[2][1];
+        S[m][5] = G[0][2] + G[2][0];
     }
+    // the coordinates sum to one: E(q) = S_0 + sum_{m>=1} lambda_qm (S_m - S_0)
+#pragma unroll
+    for (int m = 1; m < 4; ++m)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) S[m][c] -= S[0][c];
+    for (int q = 0; q < n_q; ++q) {
+        const double l1 = bary[4 * q + 1], l2 = bary[4 * q + 2], l3 = bary[4 * q + 3];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) out[6 * q + c] = fma(l3, S[3][c], fma(l2, S[2][c], fma(l1, S[1][c], S[0][c])));
+    }
+}
+
+// The FP64 forms for what the fixed-point kernels do not take: more points than a warp's block of E or of the
+// stresses has room for (the sums of that many products would leave fewer than 53 bits, too), or an array off a
+// 16-byte boundary.
+__global__ void __launch_bounds__(64) strain3_p2_fp64_kernel(const double *__restrict__ jinv, const double *__restrict__ bary,
+                                                             const double *__restrict__ u, const int32_t *__restrict__ dof,
+                                                             long long n_u, int n_elem, int n_q, double *__restrict__ E) {
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e < n_elem) strain3_p2_fp64(jinv + e * 9, bary, u, dof + e * 30, n_u, n_q, E + 6 * n_q * e);
 }
 
 // the points' lambda_1..3 as limbs in shared memory, in units of 2^(*e - 1080); *e >= 1022 (values below 1)
@@ -277,7 +311,6 @@ __device__ __forceinline__ void p2_lambda_table(const double *bary, int n_q, int
 
 // Strain.  bary is [n_q][4] (λ0..λ3 of each point).  With d_a = u_a - u_0 every A_im - A_0m is a sum of at
 // most nine d's, so the differences are taken first, exactly, and brought to 58 bits by their largest.
-template <bool STAGED>
 __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double *__restrict__ jinv,
                                                                    const double *__restrict__ bary,
                                                                    const double *__restrict__ u,
@@ -294,13 +327,11 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
     // the warp's dof lids, through the staging area
     const int n_here = static_cast<int>(n_elem - e0 < 32 ? n_elem - e0 : 32);
     int32_t *s_dof = reinterpret_cast<int32_t *>(stage);
-    if (STAGED) {
-        for (int i = lane; i < 30 * n_here; i += 32) s_dof[i] = dof[e0 * 30 + i];
-    }
+    for (int i = lane; i < 30 * n_here; i += 32) s_dof[i] = dof[e0 * 30 + i];
     __syncwarp();
-    const int32_t *dl = STAGED ? s_dof + 30 * lane : dof + e * 30;
+    const int32_t *dl = s_dof + 30 * lane;
     const bool valid = e < n_elem;
-    double *out = STAGED ? stage + 6 * n_q * lane : E + 6 * n_q * e;
+    double *out = stage + 6 * n_q * lane;
     double un[10][3];
     int e_u = 0;
     bool bad = false;
@@ -324,8 +355,7 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
         e_j = max(e_j, fx_exponent(jv[k]));
     }
     const bool finite = e_u < 2047 && e_j < 2047 && e_lam < 2047;
-    if (STAGED) __syncwarp();  // every lane has its lids: the area may become the strains
-    if (valid && !finite) strain3_p2_nonfinite(jinv + e * 9, bary, u, dof + e * 30, n_u, n_q, out);
+    __syncwarp();  // every lane has its lids: the area may become the strains
     if (valid && finite) {
         long long d[10][3];  // u_a - u_0, then times 2^(s - 4): 58 bits
         unsigned long long mag = 0;
@@ -407,12 +437,11 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
             o[2] = make_double2(v[4], v[5]);
         }
     }
-    if (STAGED) {
-        __syncwarp();
-        const double2 *src = reinterpret_cast<const double2 *>(stage);
-        double2 *dst = reinterpret_cast<double2 *>(E + 6 * n_q * e0);
-        for (int i = lane; i < 3 * n_q * n_here; i += 32) dst[i] = src[i];
-    }
+    if (valid && !finite) strain3_p2_fp64(jinv + e * 9, bary, u, dof + e * 30, n_u, n_q, out);
+    __syncwarp();
+    const double2 *src = reinterpret_cast<const double2 *>(stage);
+    double2 *dst = reinterpret_cast<double2 *>(E + 6 * n_q * e0);
+    for (int i = lane; i < 3 * n_q * n_here; i += 32) dst[i] = src[i];
 }
 
 // ---------------------------------------------------------------------------- affine tetrahedra, FP64
@@ -561,35 +590,59 @@ __global__ void __launch_bounds__(kAffineThreads) force3_affine_kernel(const dou
     if (r2 >= 0) red_add(F + r2, a2);
 }
 
-__device__ __noinline__ void force3_p2_nonfinite(const double *jinv, const double *bary, const double *S, const double *w,
-                                                 const int32_t *er, int n_rows, int n_q, double *F) {
-    double M[4][6] = {}, gl[4][3];
-    for (int q = 0; q < n_q; ++q)
-        for (int m = 0; m < 4; ++m)
-            for (int c = 0; c < 6; ++c) M[m][c] += bary[4 * q + m] * (w[q] * S[6 * q + c]);
-    for (int k = 0; k < 3; ++k) {
-        for (int i = 0; i < 3; ++i) gl[1 + i][k] = jinv[3 * i + k];
-        gl[0][k] = -(gl[1][k] + gl[2][k] + gl[3][k]);
-    }
-    for (int a = 0; a < 10; ++a) {
-        double f[3];
-        if (a < 4) {
-            double V[6];
-            for (int c = 0; c < 6; ++c) V[c] = 4.0 * M[a][c] - (M[0][c] + M[1][c] + M[2][c] + M[3][c]);
-            sym_matvec(V, gl[a], f);
-        } else {
-            const int i = (a == 5 || a == 7) ? 1 : (a == 8 ? 2 : 0), j = a == 4 ? 1 : (a == 5 || a == 6) ? 2 : 3;
-            double x[3], y[3];
-            sym_matvec(M[i], gl[j], x);
-            sym_matvec(M[j], gl[i], y);
-            for (int c = 0; c < 3; ++c) f[c] = 4.0 * (x[c] + y[c]);
-        }
-        for (int c = 0; c < 3; ++c) {
-            const int row = er[3 * a + c];
-            if (row >= n_rows) flag(SSP_DEV_BAD_INDEX);
-            else if (row >= 0) red_add(F + row, f[c]);
+// One element's forces in FP64, S [n_q][6], w [n_q]; reductions into F.
+__device__ __noinline__ void force3_p2_fp64(const double *jinv, const double *bary, const double *S, const double *w,
+                                            const int32_t *er, int n_rows, int n_q, double *F) {
+    double M[4][6] = {};
+    for (int q = 0; q < n_q; ++q) {
+        const double wq = w[q];
+        double T[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) T[c] = wq * S[6 * q + c];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const double l = bary[4 * q + m];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) M[m][c] += l * T[c];
         }
     }
+    double gl[4][3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) gl[1 + k / 3][k % 3] = jinv[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) gl[0][k] = -(gl[1][k] + gl[2][k] + gl[3][k]);
+    auto emit = [&](int a, int c, double f) {
+        const int row = er[3 * a + c];
+        if (row >= n_rows) flag(SSP_DEV_BAD_INDEX);
+        else if (row >= 0) red_add(F + row, f);
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // vertices: (4 M_i − Σ_m M_m) ∇λ_i
+        double V[6], f[3];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) V[c] = 4.0 * M[i][c] - (M[0][c] + M[1][c] + M[2][c] + M[3][c]);
+        sym_matvec(V, gl[i], f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) emit(i, c, f[c]);
+    }
+    constexpr int kEi[6] = {0, 1, 0, 1, 2, 0}, kEj[6] = {1, 2, 2, 3, 3, 3};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {  // edges: 4 (M_i ∇λ_j + M_j ∇λ_i)
+        const int i = kEi[k], j = kEj[k];
+        double x[3], y[3];
+        sym_matvec(M[i], gl[j], x);
+        sym_matvec(M[j], gl[i], y);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) emit(p2_edge_node(i, j), c, 4.0 * (x[c] + y[c]));
+    }
+}
+
+__global__ void __launch_bounds__(64) force3_p2_fp64_kernel(const double *__restrict__ jinv, const double *__restrict__ bary,
+                                                            const double *__restrict__ S, const double *__restrict__ w,
+                                                            const int32_t *__restrict__ elem_row, int n_rows, int n_elem,
+                                                            int n_q, double *__restrict__ F) {
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e < n_elem) force3_p2_fp64(jinv + e * 9, bary, S + 6 * n_q * e, w + e * n_q, elem_row + e * 30, n_rows, n_q, F);
 }
 
 // (M v)[c] for M symmetric as [11,22,33,12,23,13], added to a sum
@@ -601,7 +654,6 @@ __device__ __forceinline__ void fx_sym_row(FxSum &s, const int2 *M, const int2 *
 
 // Force; elem_row as in force_element_kernel; reductions into F.  The moment of lambda_0 is the sum of w sigma
 // less the other three.
-template <bool STAGED>
 __global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *__restrict__ jinv,
                                                                   const double *__restrict__ bary,
                                                                   const double *__restrict__ S,
@@ -614,18 +666,16 @@ __global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *
     const int lane = threadIdx.x;
     const long long e0 = blockIdx.x * 32ll, e = e0 + lane;
     const int n_here = static_cast<int>(n_elem - e0 < 32 ? n_elem - e0 : 32);
-    if (STAGED) {
-        const char *src = reinterpret_cast<const char *>(S + 6 * n_q * e0);
-        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(stage));
-        for (int i = lane; i < 3 * n_q * n_here; i += 32)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
-    }
+    const char *src = reinterpret_cast<const char *>(S + 6 * n_q * e0);
+    const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(stage));
+    for (int i = lane; i < 3 * n_q * n_here; i += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
     int e_lam;
     p2_lambda_table<kFxLimb>(bary, n_q, s_lam, &e_lam);
-    if (STAGED) asm volatile("cp.async.wait_all;\n" ::: "memory");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncwarp();
     if (e >= n_elem) return;
-    const double *Se = STAGED ? stage + 6 * n_q * lane : S + 6 * n_q * e;
+    const double *Se = stage + 6 * n_q * lane;
     const double *we = w + e * n_q;
     int e_s = 0, e_w = 0, e_j = 0;
 #pragma unroll 1
@@ -639,7 +689,7 @@ __global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *
     for (int k = 0; k < 9; ++k) e_j = max(e_j, fx_exponent(jinv[e * 9 + k]));
     const int32_t *er = elem_row + e * 30;
     if (max(max(e_s, e_w), max(e_j, e_lam)) == 2047) {
-        force3_p2_nonfinite(jinv + e * 9, bary, Se, we, er, n_rows, n_q, F);
+        force3_p2_fp64(jinv + e * 9, bary, Se, we, er, n_rows, n_q, F);
         return;
     }
     // the sums of n_q products, and of four moments, stay below 2^63
@@ -2441,13 +2491,13 @@ int ssp_assemble_overlap_strain_3d_p2_affine(const double *jinv, const double *b
     if ((long long)n_elem * n_q != n_int) return SSP_ERR_INVALID;
     if (n_elem == 0) return SSP_OK;
     if (!jinv || !bary || !u_overlap || !elem_dof_lids || !out_values) return SSP_ERR_INVALID;
-    const size_t table = (24 * (size_t)n_q + 15) & ~size_t(15);
-    if (n_q <= kP2StageMaxQ && table + 32 * 48 * (size_t)n_q >= 3840 + table)
-        strain3_p2_affine_kernel<true><<<grid_for(n_elem, 32), 32, table + 32 * 48 * (size_t)n_q, as_stream(stream)>>>(
+    const size_t table = (24 * (size_t)n_q + 15) & ~size_t(15), lids = 32 * 30 * sizeof(int32_t), block = 32 * 48 * (size_t)n_q;
+    if (n_q <= kP2StageMaxQ && (reinterpret_cast<uintptr_t>(out_values) & 15u) == 0)
+        strain3_p2_affine_kernel<<<grid_for(n_elem, 32), 32, table + (block > lids ? block : lids), as_stream(stream)>>>(
             jinv, bary, u_overlap, elem_dof_lids, n_u, n_elem, n_q, out_values);
     else
-        strain3_p2_affine_kernel<false><<<grid_for(n_elem, 32), 32, table, as_stream(stream)>>>(
-            jinv, bary, u_overlap, elem_dof_lids, n_u, n_elem, n_q, out_values);
+        strain3_p2_fp64_kernel<<<grid_for(n_elem, 64), 64, 0, as_stream(stream)>>>(jinv, bary, u_overlap, elem_dof_lids, n_u,
+                                                                                   n_elem, n_q, out_values);
     return launch_status();
 }
 
@@ -2462,11 +2512,11 @@ int ssp_assemble_force_element_p2_affine(const double *jinv, const double *bary,
     if (!jinv || !bary || !stress || !weight || !elem_row) return SSP_ERR_INVALID;
     const size_t table = (24 * (size_t)n_q + 15) & ~size_t(15);
     if (n_q <= kP2StageMaxQ && (reinterpret_cast<uintptr_t>(stress) & 15u) == 0)
-        force3_p2_affine_kernel<true><<<grid_for(n_elem, 32), 32, table + 32 * 48 * (size_t)n_q, st>>>(
+        force3_p2_affine_kernel<<<grid_for(n_elem, 32), 32, table + 32 * 48 * (size_t)n_q, st>>>(
             jinv, bary, stress, weight, elem_row, n_rows, n_elem, n_q, out_values);
     else
-        force3_p2_affine_kernel<false><<<grid_for(n_elem, 32), 32, table, st>>>(jinv, bary, stress, weight, elem_row, n_rows,
-                                                                                n_elem, n_q, out_values);
+        force3_p2_fp64_kernel<<<grid_for(n_elem, 64), 64, 0, st>>>(jinv, bary, stress, weight, elem_row, n_rows, n_elem, n_q,
+                                                                   out_values);
     return launch_status();
 }
 

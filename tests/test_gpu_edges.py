@@ -73,3 +73,63 @@ def test_bad_row_of_a_force_is_reported(et, finite):
     rows[1, k] = n_rows
     force(rows)
     assert _lib.device_status(clear=True) == BAD_INDEX
+
+
+def _p2_gradients(jinv, lam):
+    """(n_el, n_q, 10, 3) gradients of straight-sided P2 tetrahedra at barycentric points lam (n_q, 4)."""
+    gl = np.concatenate([-jinv.sum(axis=1, keepdims=True), jinv], axis=1)
+    g = np.empty((jinv.shape[0], lam.shape[0], 10, 3), dtype=jinv.dtype)
+    for a in range(4):
+        g[:, :, a] = (4 * lam[None, :, a, None] - 1) * gl[:, None, a]
+    for a, (i, j) in zip(range(4, 10), ((0, 1), (1, 2), (0, 2), (1, 3), (2, 3), (0, 3))):
+        g[:, :, a] = 4 * (lam[None, :, i, None] * gl[:, None, j] + lam[None, :, j, None] * gl[:, None, i])
+    return g
+
+
+@pytest.mark.parametrize("n_q,odd", [(1, False), (11, True), (30, False), (31, False), (2049, False), (2100, True)])
+def test_p2_strain_and_force_point_counts_and_alignment(n_q, odd):
+    """Any number of points per element, and E and the stresses at any multiple of eight bytes.  Tolerance as in
+    the tests of the fixed-point kernels, 1e-13 of the largest value for sums of 30 terms (the strain), and
+    sqrt(n_q) times that for the force's sums over the points."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.distributed_tangent import _p2_affine_inputs
+
+    pat = _pattern("P2", (3, 2, 1))
+    d = _p2_affine_inputs(pat)
+    rng = np.random.default_rng(n_q)
+    n_el, n_rows = int(pat.overlap_elements.size), int(pat.local_matrix_pattern.shape[0])
+    lam = rng.dirichlet(np.ones(4), n_q)
+    g = _p2_gradients(d["jinv"].cpu().numpy().reshape(n_el, 3, 3), lam)
+    dof = pat.overlap_element_dof_lids
+    u = rng.standard_normal(int(pat.overlap_global_dofs.size))
+    bary, ud = _dev(lam), _dev(u)
+
+    def room(n):
+        return torch.full((n + 1,), -7.0, dtype=torch.float64, device="cuda")[1:] if odd else \
+            torch.full((n,), -7.0, dtype=torch.float64, device="cuda")
+
+    E = room(n_el * n_q * 6)
+    assert E.data_ptr() % 16 == (8 if odd else 0)
+    _lib.call("ssp_assemble_overlap_strain_3d_p2_affine", _lib.ptr(d["jinv"]), _lib.ptr(bary), _lib.ptr(ud), u.size,
+              _lib.ptr(d["dof_lids"]), n_el * n_q, n_el, n_q, _lib.ptr(E), _lib.stream_handle())
+    ue = u[dof].reshape(n_el, 10, 3)
+    H = np.einsum("eac,eqaz->eqcz", ue, g)
+    want = np.stack([H[..., 0, 0], H[..., 1, 1], H[..., 2, 2], H[..., 0, 1] + H[..., 1, 0], H[..., 1, 2] + H[..., 2, 1],
+                     H[..., 0, 2] + H[..., 2, 0]], -1)
+    assert rel_err(E.cpu().numpy(), want.reshape(-1)) <= 1e-13
+    S = room(n_el * n_q * 6)
+    S_host = rng.standard_normal((n_el * n_q, 6))
+    S.copy_(torch.as_tensor(S_host.reshape(-1)))
+    w = rng.uniform(0.0, 1.0, n_el * n_q)
+    wd, F = _dev(w), torch.empty(n_rows, dtype=torch.float64, device="cuda")
+    _lib.call("ssp_assemble_force_element_p2_affine", _lib.ptr(d["jinv"]), _lib.ptr(bary), _lib.ptr(S), _lib.ptr(wd),
+              _lib.ptr(d["elem_row"]), n_el, n_q, n_rows, _lib.ptr(F), _lib.stream_handle())
+    ws = (w[:, None] * S_host).reshape(n_el, n_q, 6)
+    bt = ((0, 3, 5), (3, 1, 4), (5, 4, 2))
+    rows = d["elem_row"].cpu().numpy().reshape(n_el, 10, 3)
+    f = np.stack([sum(np.einsum("eqa,eq->ea", g[..., z], ws[..., bt[c][z]]) for z in range(3)) for c in range(3)], -1)
+    want = np.zeros(n_rows)
+    np.add.at(want, rows[rows >= 0], f[rows >= 0])
+    assert rel_err(F.cpu().numpy(), want) <= 1e-13 * max(1.0, n_q / 11.0) ** 0.5
