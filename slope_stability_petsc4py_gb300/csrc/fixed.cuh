@@ -25,22 +25,21 @@ namespace ssp {
 constexpr int kFxLimb = 29;
 constexpr int kFxDrop = 2 * kFxLimb;  // a product sum's unit is 2^58 times the product of its factors' units
 
-// biased exponent of x (2047: infinity or nan)
+// biased exponent of x (2047: infinity or nan; 0: subnormal or zero, whose unit is exponent 1's)
 __device__ __forceinline__ int fx_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
 
 // x in units of 2^(e_block - 1022 - bits), truncated: |x| < 2^(e_block - 1022) maps below 2^bits (bits <= 62; at
-// 60 a value is exact down to 2^-7 of the largest).
-// x is finite with an exponent of at most e_block; subnormal values count as zero.
+// 60 a value is exact down to 2^-7 of the largest).  x is finite with an exponent of at most e_block.
 __device__ __forceinline__ long long fx_from_f64(double x, int e_block, int bits) {
     const int hi = __double2hiint(x), e = (hi >> 20) & 0x7FF;
-    const int d = e == 0 ? 63 : min(e_block - e, 63);
+    const int d = min(max(e_block, 1) - max(e, 1), 63);
     const unsigned long long m =
-        (static_cast<unsigned long long>((hi & 0xFFFFF) | 0x100000) << 32) | static_cast<unsigned>(__double2loint(x));
+        (static_cast<unsigned long long>((hi & 0xFFFFF) | (e ? 0x100000 : 0)) << 32) | static_cast<unsigned>(__double2loint(x));
     const long long v = static_cast<long long>((m << (bits - 53)) >> d), sign = hi >> 31;
     return (v ^ sign) - sign;
 }
 // the exponent of fx_from_f64's unit
-__device__ __forceinline__ int fx_unit(int e_block, int bits) { return e_block - 1022 - bits; }
+__device__ __forceinline__ int fx_unit(int e_block, int bits) { return max(e_block, 1) - 1022 - bits; }
 
 // x 2^unit, |x| < 2^63, rounded to nearest (ties away from zero).  unit is the same for a block: only where a
 // result could leave the normal range the general form is taken.  A negative x counts as its one's complement,

@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
         __syncthreads();
         // total = hh 2^56 + mid 2^28
         const int unit_wd = fx_unit(e_w, 58) + fx_unit(e_d, 60) + fx_top_unit<58>(room) + kFxDrop + 2;
-        const int unit_e = unit_wd + 4 * kLimb + 2 * fx_unit(0, kBitsG) + (kByNode ? 0 : 2 * e_g + fx_top_unit<56>(fx_room(h_bits)));
+        const int unit_e = unit_wd + 4 * kLimb + (kByNode ? 0 : 2 * fx_unit(e_g, kBitsG) + fx_top_unit<56>(fx_room(h_bits)));
         const unsigned nnz32 = static_cast<unsigned>(A.nnz < 0x7FFFFFFFll ? A.nnz : 0x7FFFFFFFll);
         auto emit = [&](int32_t p, double v) {
             if (static_cast<unsigned>(p) < nnz32) red_add(A.values + p, v);
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(Shape<NP, NQ, SYM>::kThreads, Shape<NP, NQ, SY
                         for (int r = 0; r < 3; ++r) acc[c][d].add_prod(ga[r], h[kRow[c][r]]);
                 }
             }
-            const int unit_k = kByNode ? unit_e + S.eg[a] + S.eg[b] + fx_top_unit<56>(fx_room(S.hb[b])) : unit_e;
+            const int unit_k = kByNode ? unit_e + fx_unit(S.eg[a], kBitsG) + fx_unit(S.eg[b], kBitsG) + fx_top_unit<56>(fx_room(S.hb[b])) : unit_e;
             // the tile's positions first (and its mirror's): behind a reduction each load would wait by itself
             const int32_t *up = em + 3 * a * kNld + 3 * b, *low = em + 3 * b * kNld + 3 * a;
             int32_t pu[9], pl[9];

@@ -133,3 +133,53 @@ def test_p2_strain_and_force_point_counts_and_alignment(n_q, odd):
     want = np.zeros(n_rows)
     np.add.at(want, rows[rows >= 0], f[rows >= 0])
     assert rel_err(F.cpu().numpy(), want) <= 1e-13 * max(1.0, n_q / 11.0) ** 0.5
+
+
+def test_subnormal_inputs(oracle):
+    """Displacements, stresses and tangents among FP64's subnormal numbers count as what they are.  Tolerance: 1e-13
+    of the largest value as elsewhere, and a quantum of the subnormal range (5e-324) for each of the roundings to it,
+    of which an element's force or tangent has one and an entry a few dozen elements at most."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.distributed_tangent import _affine_fp64_inputs, _p2_affine_inputs
+
+    tiny, step = 2.0**-1030, 2.0**-44  # a quantum of the subnormal range, 2^-1074, scaled up again
+    for et, dims in (("P2", (2, 2, 1)), ("P4", (2, 1, 1))):
+        pat = _pattern(et, dims)
+        d = (_p2_affine_inputs if et == "P2" else _affine_fp64_inputs)(pat)
+        rng = np.random.default_rng(3)
+        n_el, n_q, n_p, n_rows = int(pat.overlap_elements.size), pat.n_q, pat.n_p, int(pat.local_matrix_pattern.shape[0])
+        u = np.round(rng.standard_normal(int(pat.overlap_global_dofs.size)) * 2.0**40) * 2.0**-40  # exact when scaled
+        S = np.round(rng.standard_normal((n_el * n_q, 6)) * 2.0**40) * 2.0**-40
+        A = rng.standard_normal((n_el * n_q, 6, 6))
+        DS = np.round((A + A.transpose(0, 2, 1)) * 2.0**40) * 2.0**-40
+        affine = et == "P4"
+
+        def run(scale):
+            E, F = (torch.zeros(n, dtype=torch.float64, device="cuda") for n in (6 * n_el * n_q, n_rows))
+            K, Km = (torch.zeros(pat.nnz, dtype=torch.float64, device="cuda") for _ in range(2))
+            ud, Sd, Dd = _dev(u * scale), _dev(S * scale), _dev(DS.transpose(0, 2, 1).reshape(-1, 36) * scale)
+            st, table = _lib.stream_handle(), d["ghat" if affine else "bary"]
+            _lib.call("ssp_assemble_overlap_strain_3d" + ("_affine" if affine else "_p2_affine"), _lib.ptr(d["jinv"]),
+                      _lib.ptr(table), _lib.ptr(ud), u.size, _lib.ptr(d["dof_lids"]), n_el * n_q, n_el,
+                      *([n_p] if affine else []), n_q, _lib.ptr(E), st)
+            _lib.call("ssp_assemble_force_element" + ("_affine" if affine else "_p2_affine"), _lib.ptr(d["jinv"]),
+                      _lib.ptr(table), _lib.ptr(Sd), _lib.ptr(d["weight"]), _lib.ptr(d["elem_row"]), n_el,
+                      *([n_p] if affine else []), n_q, n_rows, _lib.ptr(F), st)
+            geo = [_lib.ptr(d[k]) for k in ("dphi1", "dphi2", "dphi3")]
+            _lib.call("ssp_tangent_element", 3, 1, *geo, _lib.ptr(Dd), _lib.ptr(d["weight"]), _lib.ptr(d["scatter_map"]),
+                      n_el, n_p, n_q, pat.nnz, _lib.ptr(K), 0, st)
+            if et == "P2":
+                zero = torch.zeros(n_el * n_q, dtype=torch.float64, device="cuda")
+                branch = torch.ones(n_el * n_q, dtype=torch.int8, device="cuda")
+                elist, count = torch.arange(n_el, dtype=torch.int32, device="cuda"), _dev(np.array([n_el], np.int32))
+                _lib.call("ssp_tangent_plastic_correction_p2_moments", _lib.ptr(d["jinv"]), _lib.ptr(table), _lib.ptr(Dd),
+                          _lib.ptr(d["weight"]), _lib.ptr(branch), _lib.ptr(zero), _lib.ptr(zero), _lib.ptr(d["scatter_map"]),
+                          n_el, n_q, pat.nnz, 1.0, _lib.ptr(Km), _lib.ptr(elist), _lib.ptr(count), st)
+            return [x.cpu().numpy() for x in (E, F, K, Km)]
+
+        for got, want in zip(run(tiny), run(1.0)):
+            err = np.abs(got * 2.0**1000 * 2.0**30 - want)
+            assert np.all(err <= 1e-13 * np.abs(want).max() + 64 * step)
+            assert got.any() or not want.any()
