@@ -225,10 +225,12 @@ __device__ __forceinline__ void sym_matvec(const double *M, const double *v, dou
     out[2] = M[5] * v[0] + M[4] * v[1] + M[2] * v[2];
 }
 
-// Both kernels: one thread per element, one warp per CTA, in 58-bit fixed point (fixed.cuh; one exponent per
-// element for the displacement differences, the gradients, the stresses, ...).  In FP64 they were bound by
-// that pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 54 and 78, bound by the
-// latency of 10 to 12 warps an SM of 160 registers and some 4,200 integer instructions an element).  E and the stresses pass
+// Both kernels: one thread per element, one warp per CTA, in 58-bit fixed point (fixed.cuh; an element has an
+// exponent for each displacement component, each column of J^{-1} and each stress component, so that small ones
+// beside large ones, or thin elements, keep the bits that they have in FP64).  In FP64 they were bound by that
+// pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 55 and 92, bound by the latency of 12 or
+// 13 warps an SM).  With one exponent for all components and columns and the force's last contraction in integers, too,
+// they took 54 and 80, and a strain or force 1e-8 of the others kept half of its digits.  E and the stresses pass
 // through shared memory, so that a warp's 32 elements are one contiguous block of global memory; elements
 // with an input that is not finite take the FP64 form of the same sums.
 constexpr int kP2StageMaxQ = 30;  // points per element for which a warp's block fits (46 KiB); more take FP64
@@ -310,7 +312,7 @@ __device__ __forceinline__ void p2_lambda_table(const double *bary, int n_q, int
 }
 
 // Strain.  bary is [n_q][4] (λ0..λ3 of each point).  With d_a = u_a - u_0 every A_im - A_0m is a sum of at
-// most nine d's, so the differences are taken first, exactly, and brought to 58 bits by their largest.
+// most nine d's, so the differences are taken first, exactly, and brought to 58 bits by their component's largest.
 __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double *__restrict__ jinv,
                                                                    const double *__restrict__ bary,
                                                                    const double *__restrict__ u,
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
     const bool valid = e < n_elem;
     double *out = stage + 6 * n_q * lane;
     double un[10][3];
-    int e_u = 0;
+    int e_u[3] = {0, 0, 0};
     bool bad = false;
 #pragma unroll
     for (int a = 0; a < 10; ++a) {
@@ -343,40 +345,51 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
             un[a][c] = 0.0;
             if (i < 0 || i >= n_u) bad = true;
             else if (valid) un[a][c] = u[i];
-            e_u = max(e_u, fx_exponent(un[a][c]));
+            e_u[c] = max(e_u[c], fx_exponent(un[a][c]));
         }
     }
     if (bad && valid) flag(SSP_DEV_BAD_INDEX);
     double jv[9];
-    int e_j = 0;
+    int e_j[3] = {0, 0, 0};  // of the columns: d lambda / dx, d lambda / dy, d lambda / dz
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         jv[k] = valid ? jinv[e * 9 + k] : 0.0;
-        e_j = max(e_j, fx_exponent(jv[k]));
+        e_j[k % 3] = max(e_j[k % 3], fx_exponent(jv[k]));
     }
-    const bool finite = e_u < 2047 && e_j < 2047 && e_lam < 2047;
+    const bool finite = max(max(max(e_u[0], e_u[1]), max(e_u[2], e_lam)), max(max(e_j[0], e_j[1]), e_j[2])) < 2047;
     __syncwarp();  // every lane has its lids: the area may become the strains
     if (valid && finite) {
         long long d[10][3];  // u_a - u_0, then times 2^(s - 4): 58 bits
-        unsigned long long mag = 0;
+        int unit_d[3];       // of a component's b below
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const long long u0 = fx_from_f64(un[0][c], e_u, 60);
+            unsigned long long mag = 0;
+            const long long u0 = fx_from_f64(un[0][c], e_u[c], 60);
             d[0][c] = 0;
 #pragma unroll
             for (int a = 1; a < 10; ++a) {
-                d[a][c] = fx_from_f64(un[a][c], e_u, 60) - u0;
+                d[a][c] = fx_from_f64(un[a][c], e_u[c], 60) - u0;
                 mag |= fx_mag(d[a][c]);
             }
+            const int s = min(__clzll(static_cast<long long>(mag)) - 2, 58);  // to 62 bits
+#pragma unroll
+            for (int a = 1; a < 10; ++a) d[a][c] = (d[a][c] << s) >> 4;
+            unit_d[c] = mag ? fx_unit(e_u[c], 60) - s + 8 : -16384;  // no weight to a component that is constant
         }
-        const int s = min(__clzll(static_cast<long long>(mag)) - 2, 58);  // to 62 bits
-#pragma unroll
-        for (int a = 1; a < 10; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) d[a][c] = (d[a][c] << s) >> 4;
         int2 gl[3][3];  // ∇λ_1..3
 #pragma unroll
-        for (int k = 0; k < 9; ++k) gl[k / 3][k % 3] = fx_split(fx_from_f64(jv[k], e_j, 58));
+        for (int k = 0; k < 9; ++k) gl[k / 3][k % 3] = fx_split(fx_from_f64(jv[k], e_j[k % 3], 58));
+        // the strains' units; the two halves of a shear have their own, and the smaller unit's is shifted to the other's
+        int unit_S[6], shift_x[3], shift_y[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int x = c == 2 ? 0 : c, y = c == 0 ? 1 : 2;  // (0,1), (1,2), (0,2)
+            const int ux = unit_d[x] + fx_unit(e_j[y], 58), uy = unit_d[y] + fx_unit(e_j[x], 58);
+            unit_S[c] = unit_d[c] + fx_unit(e_j[c], 58) + kFxDrop;
+            unit_S[3 + c] = max(ux, uy) + kFxDrop;
+            shift_x[c] = min(max(uy - ux, 0), 63);
+            shift_y[c] = min(max(ux - uy, 0), 63);
+        }
         // ∇u = Σ_m λ_m G_m, G_m = Σ_{i=1..3} (A_im − A_0m) ⊗ ∇λ_i, A_ii = 3u_i, A_im = 4u_(edge im) − u_i
         long long S0[6];
         int2 dS[3][6];
@@ -398,15 +411,14 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
                 n.add_prod(b[1][c], gl[1][c]);
                 n.add_prod(b[2][c], gl[2][c]);
                 Sm[c] = n.value();
-                const int x = c == 2 ? 0 : c, y = c == 0 ? 1 : 2;  // (0,1), (1,2), (0,2)
-                FxSum t(b[0][x], gl[0][y]);  // G_xy + G_yx
-                t.add_prod(b[0][y], gl[0][x]);
+                const int x = c == 2 ? 0 : c, y = c == 0 ? 1 : 2;
+                FxSum tx(b[0][x], gl[0][y]), ty(b[0][y], gl[0][x]);  // G_xy, G_yx
 #pragma unroll
                 for (int i = 1; i < 3; ++i) {
-                    t.add_prod(b[i][x], gl[i][y]);
-                    t.add_prod(b[i][y], gl[i][x]);
+                    tx.add_prod(b[i][x], gl[i][y]);
+                    ty.add_prod(b[i][y], gl[i][x]);
                 }
-                Sm[3 + c] = t.value();
+                Sm[3 + c] = (tx.value() >> shift_x[c]) + (ty.value() >> shift_y[c]);
             }
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
@@ -416,8 +428,7 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
         }
         // the coordinates sum to one: E(q) = S_0 + sum_{m>=1} lambda_qm (S_m - S_0), with two bits more than the
         // product sums' unit (S is below 2^60)
-        const int unit_S = fx_unit(e_u, 60) - s + 8 + fx_unit(e_j, 58) + kFxDrop, shift_0 = fx_unit(e_lam, 58) + 2 * kLambdaLimb;
-        const int unit_E = unit_S + shift_0 - 2;  // shift_0 >= 2
+        const int shift_0 = fx_unit(e_lam, 58) + 2 * kLambdaLimb;  // at least 2
 #pragma unroll
         for (int c = 0; c < 6; ++c) S0[c] >>= min(shift_0 - 2, 63);
 #pragma unroll 1
@@ -429,7 +440,7 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
                 FxSum t(dS[0][c], l1);
                 t.add_prod(dS[1][c], l2);
                 t.add_prod(dS[2][c], l3);
-                v[c] = fx_to_f64(t.value_up<kLambdaLimb, 2>() + S0[c], unit_E);
+                v[c] = fx_to_f64(t.value_up<kLambdaLimb, 2>() + S0[c], unit_S[c] + shift_0 - 2);
             }
             double2 *o = reinterpret_cast<double2 *>(out + 6 * q);
             o[0] = make_double2(v[0], v[1]);
@@ -454,7 +465,7 @@ __global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double 
 
 // Elements of more than four nodes take the fixed-point kernels (affine_fixed.cu) where their sums have room;
 // P1's 45 multiply-adds a point are no work to convert for.
-constexpr int kAffineSmallNodes = 4, kAffineMaxTerms = 120;
+constexpr int kAffineSmallNodes = 4;
 
 // Strain: grad u = G J^{-1}, G_ik = sum_{a>=1} (u_a - u_0)_i ghat_a,k(q) (the element's rigid
 // translation removed first, as the mixed form does); E the engineering strains of grad u.
@@ -590,7 +601,48 @@ __global__ void __launch_bounds__(kAffineThreads) force3_affine_kernel(const dou
     if (r2 >= 0) red_add(F + r2, a2);
 }
 
-// One element's forces in FP64, S [n_q][6], w [n_q]; reductions into F.
+// The forces of four times an element's moments M_m = sum_q lambda_m w sigma; reductions into F.  The rows are loaded
+// first: behind a reduction each load would wait by itself.
+__device__ __forceinline__ void p2_force_of_moments(const double (&M4)[4][6], const double *jinv, const int32_t *er, int n_rows,
+                                                    double *F) {
+    int32_t row[30];
+#pragma unroll
+    for (int i = 0; i < 30; ++i) row[i] = er[i];
+    double gl[4][3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) gl[1 + k / 3][k % 3] = jinv[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) gl[0][k] = -(gl[1][k] + gl[2][k] + gl[3][k]);
+    auto emit = [&](int a, int c, double f) {
+        const int r = row[3 * a + c];
+        if (r >= n_rows) flag(SSP_DEV_BAD_INDEX);
+        else if (r >= 0) red_add(F + r, f);
+    };
+    double Mt[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) Mt[c] = M4[0][c] + M4[1][c] + M4[2][c] + M4[3][c];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // vertices: (4 M_i − Σ_m M_m) ∇λ_i
+        double V[6], f[3];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) V[c] = fma(-0.25, Mt[c], M4[i][c]);
+        sym_matvec(V, gl[i], f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) emit(i, c, f[c]);
+    }
+    constexpr int kEi[6] = {0, 1, 0, 1, 2, 0}, kEj[6] = {1, 2, 2, 3, 3, 3};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {  // edges: 4 (M_i ∇λ_j + M_j ∇λ_i)
+        const int i = kEi[k], j = kEj[k];
+        double x[3], y[3];
+        sym_matvec(M4[i], gl[j], x);
+        sym_matvec(M4[j], gl[i], y);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) emit(p2_edge_node(i, j), c, x[c] + y[c]);
+    }
+}
+
+// One element's forces in FP64, S [n_q][6], w [n_q].
 __device__ __noinline__ void force3_p2_fp64(const double *jinv, const double *bary, const double *S, const double *w,
                                             const int32_t *er, int n_rows, int n_q, double *F) {
     double M[4][6] = {};
@@ -606,35 +658,9 @@ __device__ __noinline__ void force3_p2_fp64(const double *jinv, const double *ba
             for (int c = 0; c < 6; ++c) M[m][c] += l * T[c];
         }
     }
-    double gl[4][3];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) gl[1 + k / 3][k % 3] = jinv[k];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) gl[0][k] = -(gl[1][k] + gl[2][k] + gl[3][k]);
-    auto emit = [&](int a, int c, double f) {
-        const int row = er[3 * a + c];
-        if (row >= n_rows) flag(SSP_DEV_BAD_INDEX);
-        else if (row >= 0) red_add(F + row, f);
-    };
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {  // vertices: (4 M_i − Σ_m M_m) ∇λ_i
-        double V[6], f[3];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) V[c] = 4.0 * M[i][c] - (M[0][c] + M[1][c] + M[2][c] + M[3][c]);
-        sym_matvec(V, gl[i], f);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) emit(i, c, f[c]);
-    }
-    constexpr int kEi[6] = {0, 1, 0, 1, 2, 0}, kEj[6] = {1, 2, 2, 3, 3, 3};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {  // edges: 4 (M_i ∇λ_j + M_j ∇λ_i)
-        const int i = kEi[k], j = kEj[k];
-        double x[3], y[3];
-        sym_matvec(M[i], gl[j], x);
-        sym_matvec(M[j], gl[i], y);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) emit(p2_edge_node(i, j), c, 4.0 * (x[c] + y[c]));
-    }
+    for (int k = 0; k < 24; ++k) M[k / 6][k % 6] *= 4.0;
+    p2_force_of_moments(M, jinv, er, n_rows, F);
 }
 
 __global__ void __launch_bounds__(64) force3_p2_fp64_kernel(const double *__restrict__ jinv, const double *__restrict__ bary,
@@ -645,16 +671,10 @@ __global__ void __launch_bounds__(64) force3_p2_fp64_kernel(const double *__rest
     if (e < n_elem) force3_p2_fp64(jinv + e * 9, bary, S + 6 * n_q * e, w + e * n_q, elem_row + e * 30, n_rows, n_q, F);
 }
 
-// (M v)[c] for M symmetric as [11,22,33,12,23,13], added to a sum
-__device__ __forceinline__ void fx_sym_row(FxSum &s, const int2 *M, const int2 *v, int c) {
-    constexpr int kRow[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
-#pragma unroll
-    for (int z = 0; z < 3; ++z) s.add_prod(M[kRow[c][z]], v[z]);
-}
-
 // Force; elem_row as in force_element_kernel; reductions into F.  The moment of lambda_0 is the sum of w sigma
-// less the other three.
-__global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *__restrict__ jinv,
+// less the other three.  The moments, exact to 58 bits of a stress component's largest, are contracted with the gradients
+// in FP64: 200 operations an element.
+__global__ void __launch_bounds__(32, 13) force3_p2_affine_kernel(const double *__restrict__ jinv,
                                                                   const double *__restrict__ bary,
                                                                   const double *__restrict__ S,
                                                                   const double *__restrict__ w,
@@ -677,18 +697,20 @@ __global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *
     if (e >= n_elem) return;
     const double *Se = stage + 6 * n_q * lane;
     const double *we = w + e * n_q;
-    int e_s = 0, e_w = 0, e_j = 0;
+    int e_s[6] = {0, 0, 0, 0, 0, 0}, e_w = 0;
 #pragma unroll 1
     for (int q = 0; q < n_q; ++q) {
         e_w = max(e_w, fx_exponent(we[q]));
         const double2 *s2 = reinterpret_cast<const double2 *>(Se + 6 * q);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) e_s = max(e_s, max(fx_exponent(s2[k].x), fx_exponent(s2[k].y)));
+        for (int k = 0; k < 3; ++k) {
+            const double2 v = s2[k];
+            e_s[2 * k] = max(e_s[2 * k], fx_exponent(v.x));
+            e_s[2 * k + 1] = max(e_s[2 * k + 1], fx_exponent(v.y));
+        }
     }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) e_j = max(e_j, fx_exponent(jinv[e * 9 + k]));
     const int32_t *er = elem_row + e * 30;
-    if (max(max(e_s, e_w), max(e_j, e_lam)) == 2047) {
+    if (max(max(max(e_s[0], e_s[1]), max(e_s[2], e_s[3])), max(max(e_s[4], e_s[5]), max(e_w, e_lam))) == 2047) {
         force3_p2_fp64(jinv + e * 9, bary, Se, we, er, n_rows, n_q, F);
         return;
     }
@@ -709,7 +731,7 @@ __global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int c = 2 * k + h;
-                const long long T = FxSum(wq, fx_split(fx_from_f64(h == 0 ? sv.x : sv.y, e_s, bits_s))).value();
+                const long long T = FxSum(wq, fx_split(fx_from_f64(h == 0 ? sv.x : sv.y, e_s[c], bits_s))).value();
                 Mt[c] += T;
                 const int2 Tl = fx_split(T);
 #pragma unroll
@@ -717,82 +739,21 @@ __global__ void __launch_bounds__(32, 12) force3_p2_affine_kernel(const double *
             }
         }
     }
-    // all in units of Mt's, brought to 58 bits by the largest
-    const int shift_l = min(e_lam - 1022, 63);
-    long long M[4][6];
-    unsigned long long mag = 0;
+    const int shift_l = min(e_lam - 1022, 63);  // all in units of Mt's
+    double M[4][6];
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-        const long long sum = Mt[c] >> shift_l;
-        M[0][c] = sum;
+        const int unit = fx_unit(e_s[c], bits_s) + fx_unit(e_w, 58) + kFxDrop + shift_l + 2;  // 4 M
+        long long m0 = Mt[c] >> shift_l;
 #pragma unroll
         for (int m = 1; m < 4; ++m) {
-            M[m][c] = Ms[m - 1][c].value();
-            M[0][c] -= M[m][c];
-            mag |= fx_mag(M[m][c]);
+            const long long v = Ms[m - 1][c].value();
+            m0 -= v;
+            M[m][c] = fx_to_f64(v, unit);
         }
-        Mt[c] = sum;
-        mag |= fx_mag(M[0][c]) | fx_mag(sum);
+        M[0][c] = fx_to_f64(m0, unit);
     }
-    const int lz = min(__clzll(static_cast<long long>(mag)), 63) - 6;  // to 58 bits (the sums may have 62)
-    const int up = max(lz, 0), down = max(-lz, 0);
-    int2 Ml[4][6], v[4][3];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        Mt[c] = (Mt[c] << up) >> down;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            M[m][c] = (M[m][c] << up) >> down;
-            Ml[m][c] = fx_split(M[m][c]);
-        }
-    }
-    // grad lambda_0..3: the high limb of grad lambda_0 has up to 31 bits
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        long long v0 = 0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const long long x = fx_from_f64(jinv[e * 9 + 3 * i + k], e_j, 58);
-            v0 -= x;
-            v[1 + i][k] = fx_split(x);
-        }
-        v[0][k] = fx_split(v0);
-    }
-    const int unit_M = fx_unit(e_s, bits_s) + fx_unit(e_w, 58) + kFxDrop + shift_l - up + down;
-    const int unit_f = unit_M + fx_unit(e_j, 58) + kFxDrop;
-    auto emit = [&](int a, int c, const FxSum &f, int unit) {
-        const int row = er[3 * a + c];
-        if (row < 0) return;
-        if (row >= n_rows) {
-            flag(SSP_DEV_BAD_INDEX);
-            return;
-        }
-        red_add(F + row, fx_to_f64(f.value(), unit));
-    };
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {  // vertices: (4 M_i − Σ_m M_m) ∇λ_i, the bracket below 2^61, by 8
-        int2 V[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) V[c] = fx_split((4 * M[i][c] - Mt[c]) >> 3);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            FxSum f;
-            fx_sym_row(f, V, v[i], c);
-            emit(i, c, f, unit_f + 3);
-        }
-    }
-    constexpr int kEi[6] = {0, 1, 0, 1, 2, 0}, kEj[6] = {1, 2, 2, 3, 3, 3};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {  // edges: 4 (M_i ∇λ_j + M_j ∇λ_i)
-        const int i = kEi[k], j = kEj[k];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            FxSum f;
-            fx_sym_row(f, Ml[i], v[j], c);
-            fx_sym_row(f, Ml[j], v[i], c);
-            emit(p2_edge_node(i, j), c, f, unit_f + 2);
-        }
-    }
+    p2_force_of_moments(M, jinv + e * 9, er, n_rows, F);
 }
 
 // ---------------------------------------------------------------------------- tangent (rows)
@@ -2530,7 +2491,7 @@ int ssp_assemble_overlap_strain_3d_affine(const double *jinv, const double *ghat
     // the table plus the displacements of the at most 128 / n_q + 2 elements a block's points cover
     const size_t smem = sizeof(double) * (3 * (size_t)n_p * n_q + 3 * (size_t)n_p * (kAffineThreads / n_q + 2));
     if (smem > 48 * 1024) return SSP_ERR_UNSUPPORTED;
-    if (n_p > kAffineSmallNodes && n_p <= kAffineMaxTerms)
+    if (n_p > kAffineSmallNodes && n_p <= kAffineMaxNodes)
         return strain3_affine_fixed(jinv, ghat, u_overlap, elem_dof_lids, n_u, n_elem, n_p, n_q, out_values,
                                     as_stream(stream));
     strain3_affine_kernel<<<grid_for(n_int, kAffineThreads), kAffineThreads, smem, as_stream(stream)>>>(
@@ -2550,7 +2511,7 @@ int ssp_assemble_force_element_affine(const double *jinv, const double *ghat, co
     if (n_rows > 0 && cudaMemsetAsync(out_values, 0, sizeof(double) * n_rows, st) != cudaSuccess) return SSP_ERR_CUDA;
     if (n_elem == 0) return SSP_OK;
     if (!jinv || !ghat || !stress || !weight || !elem_row) return SSP_ERR_INVALID;
-    if (n_p > kAffineSmallNodes && 3 * n_q <= kAffineMaxTerms && (reinterpret_cast<uintptr_t>(stress) & 15u) == 0)
+    if (n_p > kAffineSmallNodes && n_q <= kAffineMaxPoints && (reinterpret_cast<uintptr_t>(stress) & 15u) == 0)
         return force3_affine_fixed(jinv, ghat, weight, stress, elem_row, n_rows, n_elem, n_p, n_q, out_values, st);
     const long long n = (long long)n_elem * n_p;
     force3_affine_kernel<<<grid_for(n, kAffineThreads), kAffineThreads, smem, st>>>(jinv, ghat, weight, stress,

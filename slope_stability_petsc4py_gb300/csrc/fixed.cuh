@@ -8,10 +8,17 @@
 // of its largest; a value is a 64-bit integer in units of the block's last place.  Operands of a product
 // are split into two limbs, x = h 2^29 + l with a signed lower limb; a sum of products keeps the h h and the
 // h l + l h parts in two 64-bit accumulators and drops l l (a quarter of a unit of the result per term, of either
-// sign, so that long sums have no bias).  With |x| < 2^58 there is room for 15 terms, with 55 bits and limbs of
-// 28 for 120, with 56 for 72.  Every stage is brought back to 58 bits by the block's largest
+// sign, so that long sums have no bias).  n products of a-bit and b-bit factors in units of 2^(2 LIMB) stay below 2^63
+// for n < 2^(63 + 2 LIMB - a - b): 31 terms of two 58-bit factors (limbs of 29), 127 of two of 56 bits, 63 of 57 and 56
+// (limbs of 28).  Every stage is brought back to 58 bits by the block's largest
 // value (fx_warp_bits, fx_room): without that the losses of the stages add up (three of them left 40 bits of
-// the P2 moment form).  Errors are relative to the largest value of a block, as norms see them.
+// the P2 moment form).
+//
+// Errors are relative to the largest value of a block.  What FP64 keeps apart, displacement components,
+// directions of thin elements, stress components, is therefore a block each in the strains and forces, whose components
+// are as exact as FP64's one by one.  The tangents' blocks are an element's gradients (P4: a node's) and its
+// tangents: an element matrix is as exact as FP64's relative to its largest entry, not entry by entry (a
+// thousand times thinner than wide, the entries that couple the wide directions have ten bits less).
 //
 // Conversions from and to FP64 are integer operations, too: the hardware's 64-bit conversions run at 1.9 per
 // clock and SM at best, and a warp waited some 50 to 60 clocks of the FP64 pipe for each.

@@ -69,7 +69,9 @@ int binned_decide_finish(const double *E, const double *c_bar, const double *sin
                          long long list_stride, bool compensated_ds, cudaStream_t st);
 
 // Strain and force of straight-sided tetrahedra through J^{-1} and the gradient table, in fixed point
-// (affine_fixed.cu); arguments as the ssp_*_affine entries, checked there.  force adds into F.
+// (affine_fixed.cu); arguments as the ssp_*_affine entries, checked there, and at most so many nodes (strain) or
+// points (force).  force adds into F.
+constexpr int kAffineMaxNodes = 120, kAffineMaxPoints = 40;
 int strain3_affine_fixed(const double *jinv, const double *ghat, const double *u, const int32_t *dof, int n_u, int n_elem,
                          int n_p, int n_q, double *E, cudaStream_t st);
 int force3_affine_fixed(const double *jinv, const double *ghat, const double *w, const double *S, const int32_t *elem_row,

@@ -68,3 +68,89 @@ def test_bddc_regularised_matrix(cuda_device, et, dims, seed):
         np.add.at(want, at[at >= 0], Ke[at >= 0])
     want[pat.constrained_diag_positions] = 1.0
     assert _distance(K, want) <= 2e-16
+
+
+def _components(et, shrink, small):
+    """A pattern whose cells are thinned by the powers of ten `shrink` along x, y, z, displacements whose components
+    and stresses whose rows and columns are scaled by `small`."""
+    from slope_stability_petsc4py_gb300 import ConstitutiveOperator, synthetic
+
+    mats = synthetic.MaterialSet.homogeneous()
+    mesh = synthetic.slope_mesh_3d(*((4, 2, 2) if et == "P2" else (2, 1, 2)), elem_type=et)
+    coord = mesh.coord * 10.0 ** np.asarray(shrink, dtype=np.float64)[:, None]
+    specs = [dict(c0=float(mats.c0[0]), phi=float(mats.phi[0]), psi=float(mats.psi[0]), young=float(mats.young[0]),
+                  poisson=float(mats.poisson[0]), gamma_sat=20.0, gamma_unsat=20.0)]
+    pat = ConstitutiveOperator.from_mesh(coord, mesh.elem, mesh.q_mask, mesh.material_id, specs,
+                                         elem_type=et).owned_tangent_pattern
+    rng = np.random.default_rng(5)
+    scale = np.asarray(small)
+    u = (0.3 + rng.standard_normal((int(pat.overlap_nodes.size), 3))) * scale
+    S = rng.standard_normal((pat.n_local_int, 6)) * np.array([scale[a] * scale[b] for a, b in
+                                                              ((0, 0), (1, 1), (2, 2), (0, 1), (1, 2), (0, 2))])
+    return pat, u.reshape(-1), S
+
+
+@pytest.mark.parametrize("et", ["P2", "P4"])
+@pytest.mark.parametrize("shrink,small", [((0, 0, 0), (1.0, 1.0, 1.0)), ((0, 0, 0), (1.0, 1e-8, 1.0)),
+                                          ((0, 0, -3), (1.0, 1.0, 0.0)), ((0, -3, 0), (1.0, 1e-8, 1e-4)),
+                                          ((-6, 0, 0), (0.0, 1.0, 1e-12))])
+def test_strain_and_force_component_by_component(cuda_device, et, shrink, small):
+    """Each strain component and force component to a few ulps of its own terms, whatever the others are.
+
+    An element's terms: for a strain row at a point the sum of |u_a - u_0| |grad phi_a| over its products, for a force
+    component the sum of w |sigma| |grad phi_a|, both the largest over the element (one exponent holds its points and
+    nodes).  FP64 sums are within some sqrt(30) x 2^-53 of that, the fixed-point ones (2^-56 an operand, of the
+    largest difference and table entry, which are up to eight times a term) within about as much: 2^-50."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.distributed_tangent import _affine_fp64_inputs, _p2_affine_inputs
+    from slope_stability_petsc4py_gb300.fem import quadrature, reference_gradients
+
+    pat, u, S = _components(et, shrink, small)
+    d = (_p2_affine_inputs if et == "P2" else _affine_fp64_inputs)(pat)
+    assert d is not None
+    n_el, n_q, n_p = int(pat.overlap_elements.size), pat.n_q, pat.n_p
+    n_rows = int(pat.local_matrix_pattern.shape[0])
+    jinv = d["jinv"].cpu().numpy().reshape(n_el, 3, 3).astype(LD)
+    if et == "P2":  # the kernels' own inputs: barycentric coordinates
+        lam = d["bary"].cpu().numpy().astype(LD)
+        gl = np.concatenate([-jinv.sum(axis=1, keepdims=True), jinv], axis=1)
+        g = np.empty((n_el, n_q, 10, 3), LD)
+        for a in range(4):
+            g[:, :, a] = (4 * lam[None, :, a, None] - 1) * gl[:, None, a]
+        for a, (i, j) in zip(range(4, 10), ((0, 1), (1, 2), (0, 2), (1, 3), (2, 3), (0, 3))):
+            g[:, :, a] = 4 * (lam[None, :, i, None] * gl[:, None, j] + lam[None, :, j, None] * gl[:, None, i])
+    else:
+        gh = np.transpose(reference_gradients(3, et), (2, 1, 0)).astype(LD)  # (n_q, n_p, 3)
+        g = sum(gh[None, :, :, k, None] * jinv[:, None, None, k, :] for k in range(3))
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a), device="cuda")  # noqa: E731
+    E, F = (torch.zeros(n, dtype=torch.float64, device="cuda") for n in (6 * n_el * n_q, n_rows))
+    ud, Sd = dev(u), dev(S)
+    st, more = _lib.stream_handle(), [] if et == "P2" else [n_p]
+    kind, table = ("_p2_affine", d["bary"]) if et == "P2" else ("_affine", d["ghat"])
+    _lib.call("ssp_assemble_overlap_strain_3d" + kind, _lib.ptr(d["jinv"]), _lib.ptr(table), _lib.ptr(ud), u.size,
+              _lib.ptr(d["dof_lids"]), n_el * n_q, n_el, *more, n_q, _lib.ptr(E), st)
+    _lib.call("ssp_assemble_force_element" + kind, _lib.ptr(d["jinv"]), _lib.ptr(table), _lib.ptr(Sd), _lib.ptr(d["weight"]),
+              _lib.ptr(d["elem_row"]), n_el, *more, n_q, n_rows, _lib.ptr(F), st)
+    E, F = E.cpu().numpy().reshape(n_el, n_q, 6).astype(LD), F.cpu().numpy().astype(LD)
+    ue = u[pat.overlap_element_dof_lids].reshape(n_el, n_p, 3).astype(LD)
+    ue = ue - ue[:, :1]
+    H, M = (np.stack([[sum(x[:, None, a, c] * y[:, :, a, z] for a in range(n_p)) for z in range(3)] for c in range(3)])
+            for x, y in ((ue, g), (np.abs(ue), np.abs(g))))  # [c][z][e][q]
+    for row, (x, y) in enumerate(((0, 0), (1, 1), (2, 2), (0, 1), (1, 2), (0, 2))):
+        want, terms = (H[x, x], M[x, x]) if x == y else (H[x, y] + H[y, x], M[x, y] + M[y, x])
+        size = terms.max(axis=1, keepdims=True)
+        assert np.all(np.abs(E[:, :, row] - want) <= 2.0**-50 * size), (row, float((np.abs(E[:, :, row] - want) / np.maximum(size, 1e-300)).max()))
+    ws = pat.overlap_assembly_weight.reshape(n_el, n_q, 1).astype(LD) * S.reshape(n_el, n_q, 6).astype(LD)
+    rows = d["elem_row"].cpu().numpy().reshape(n_el, n_p, 3)
+    for c in range(3):
+        f, terms = (sum((y[:, :, :, z] * x[:, :, None, BT[c][z]]).sum(axis=1) for z in range(3))
+                    for x, y in ((ws, g), (np.abs(ws), np.abs(g))))  # (n_el, n_p)
+        want, size = np.zeros(n_rows, LD), np.zeros(n_rows, LD)
+        r = rows[:, :, c]
+        np.add.at(want, r[r >= 0], f[r >= 0])
+        np.add.at(size, r[r >= 0], np.broadcast_to(terms.max(axis=1, keepdims=True), r.shape)[r >= 0])
+        mine = np.unique(r[r >= 0])
+        err = np.abs(F[mine] - want[mine])
+        assert np.all(err <= 2.0**-50 * size[mine]), (c, float((err / np.maximum(size[mine], 1e-300)).max()))
