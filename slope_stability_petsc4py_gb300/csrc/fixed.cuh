@@ -18,7 +18,7 @@
 // directions of thin elements, stress components, is therefore a block each in the strains and forces, whose components
 // are as exact as FP64's one by one.  The tangents' blocks are an element's gradients (P4: a node's) and its
 // tangents: an element matrix is as exact as FP64's relative to its largest entry, not entry by entry (a
-// thousand times thinner than wide, the entries that couple the wide directions have ten bits less).
+// thousand times thinner than wide, gradients along the wide directions have ten of their 57 bits less).
 //
 // Conversions from and to FP64 are integer operations, too: the hardware's 64-bit conversions run at 1.9 per
 // clock and SM at best, and a warp waited some 50 to 60 clocks of the FP64 pipe for each.

@@ -154,3 +154,82 @@ def test_strain_and_force_component_by_component(cuda_device, et, shrink, small)
         mine = np.unique(r[r >= 0])
         err = np.abs(F[mine] - want[mine])
         assert np.all(err <= 2.0**-50 * size[mine]), (c, float((err / np.maximum(size[mine], 1e-300)).max()))
+
+
+@pytest.mark.parametrize("thin", [1.0, 1e-3])
+@pytest.mark.parametrize("et,kind", [("P2", "symmetric"), ("P2", "full"), ("P2", "correction"), ("P2", "moments"),
+                                     ("P4", "symmetric"), ("P4", "full"), ("P4", "correction")])
+def test_element_matrices_in_the_norm(cuda_device, et, kind, thin):
+    """Element matrices of distorted, and of 1:1000, elements in the 2-norm.  Gradients, w D and H are within
+    2^-57 or 2^-56 of their largest, an entry is rounded to FP64 once, and DS - D_el may cancel two bits: 2^-55 for each
+    of three stages and 2^-53 / sqrt(3) are 1.5e-16 together; 3e-16 leaves a factor two for entries below
+    the largest.  (FP64 sums are 1.6e-16 to 4.4e-16 away.)"""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import _lib
+    from slope_stability_petsc4py_gb300.fem import quadrature, reference_gradients
+
+    rng = np.random.default_rng(7)
+    n_el, n_p, n_q = (60, 10, 11) if et == "P2" else (8, 35, 24)
+    n_ld = 3 * n_p
+    nnz = n_el * n_ld * n_ld
+    J = (np.eye(3) + 0.4 * rng.uniform(-1, 1, (n_el, 3, 3))) * rng.uniform(0.1, 5, (n_el, 1, 1))
+    J[:, 2] *= thin  # dx_i / dxi_j
+    jinv = np.linalg.inv(J)  # [k][i]: dxi_k / dx_i
+    if kind == "moments":
+        xi, _w = quadrature(3, et)
+        bary = np.vstack([1 - xi.sum(0), xi]).T
+        jl, lam = jinv.astype(LD), bary.astype(LD)
+        gl = np.concatenate([-jl.sum(1, keepdims=True), jl], 1)
+        g = np.empty((n_el, n_q, 10, 3), LD)
+        for a in range(4):
+            g[:, :, a] = (4 * lam[None, :, a, None] - 1) * gl[:, None, a]
+        for a, (i, j) in zip(range(4, 10), ((0, 1), (1, 2), (0, 2), (1, 3), (2, 3), (0, 3))):
+            g[:, :, a] = 4 * (lam[None, :, i, None] * gl[:, None, j] + lam[None, :, j, None] * gl[:, None, i])
+    else:
+        g = np.einsum("eki,kaq->eqai", jinv, np.asarray(reference_gradients(3, et)))
+    G = np.repeat(rng.uniform(5e3, 2e4, (n_el, 1)), n_q, axis=1)
+    L = 1.5 * G
+    D_el = np.zeros((n_el, n_q, 6, 6), LD)
+    D_el[..., :3, :3] = L[..., None, None]
+    for i in range(6):
+        D_el[..., i, i] += (2 if i < 3 else 1) * G
+    V = rng.standard_normal((n_el, n_q, 6, 3))
+    DS = D_el.astype(np.float64) - 0.1 * G[..., None, None] * np.einsum("eqik,eqjk->eqij", V, V)
+    if kind == "full":
+        DS = DS + 0.2 * G[..., None, None] * rng.standard_normal(DS.shape)
+    w = rng.uniform(0.5, 1, (n_el, 1)) * rng.uniform(0.05, 0.2, (1, n_q))
+    branch = (rng.uniform(size=(n_el, n_q)) < 0.7).astype(np.int8)
+    branch[:, 0] = 1
+    D = DS.astype(LD)
+    if kind in ("correction", "moments"):
+        D = (D - D_el) * (branch != 0)[..., None, None]
+    want = np.zeros((n_el, n_ld, n_ld), LD)
+    for e in range(n_el):
+        B = np.zeros((n_q, 6, n_ld), LD)
+        for c in range(3):
+            for z in range(3):
+                B[:, BT[c][z], c::3] = g[e, :, :, z]
+        want[e] = sum(B[q].T @ ((LD(w[e, q]) * D[e, q]) @ B[q]) for q in range(n_q))
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a), device="cuda")  # noqa: E731
+    ds, wd, b, sh, la = (dev(a) for a in (DS.swapaxes(-1, -2).reshape(-1, 36), w.reshape(-1), branch.reshape(-1),
+                                          G.reshape(-1), L.reshape(-1)))
+    emap, elist = torch.arange(nnz, dtype=torch.int32, device="cuda"), torch.arange(n_el, dtype=torch.int32, device="cuda")
+    count = dev(np.array([n_el], np.int32))
+    K = torch.zeros(nnz, dtype=torch.float64, device="cuda")
+    st = _lib.stream_handle()
+    if kind == "moments":
+        ji, ba = dev(jinv.reshape(n_el, 9)), dev(bary)
+        _lib.call("ssp_tangent_plastic_correction_p2_moments", _lib.ptr(ji), _lib.ptr(ba), _lib.ptr(ds), _lib.ptr(wd),
+                  _lib.ptr(b), _lib.ptr(sh), _lib.ptr(la), _lib.ptr(emap), n_el, n_q, nnz, 1.0, _lib.ptr(K), _lib.ptr(elist),
+                  _lib.ptr(count), st)
+    else:
+        geo = [dev(g[..., z].reshape(-1, n_p)) for z in range(3)]
+        if kind == "correction":
+            _lib.call("ssp_tangent_plastic_correction", 3, *(_lib.ptr(x) for x in geo), _lib.ptr(ds), _lib.ptr(wd), _lib.ptr(b),
+                      _lib.ptr(sh), _lib.ptr(la), _lib.ptr(emap), n_el, n_p, n_q, nnz, 1.0, _lib.ptr(K), _lib.ptr(elist),
+                      _lib.ptr(count), st)
+        else:
+            _lib.call("ssp_tangent_element", 3, int(kind == "symmetric"), *(_lib.ptr(x) for x in geo), _lib.ptr(ds),
+                      _lib.ptr(wd), _lib.ptr(emap), n_el, n_p, n_q, nnz, _lib.ptr(K), 0, st)
+    assert _distance(K.cpu().numpy().reshape(want.shape), want) <= 3e-16
