@@ -115,6 +115,7 @@ __device__ __forceinline__ void refine_pair(const double *t, double third, doubl
         const double v = fma(a3, n[i], sq[i]);
         f = fma(i < 3 ? v : 2.0 * v, v, f);
     }
+    if (!(f < 1e300)) return;  // strains from 1e75 up: the pair as it was
     const double b0 = 0.5 * (hi - lo);
     double b, inv;
     roots_newton(f * recip_newton(fma(2.0 * b0, b0, 18.0 * a * a)), b, inv);
