@@ -52,13 +52,19 @@ except Exception:  # pragma: no cover
 _OWNED_MODES = {"overlap", "unique_exchange", "unique", "unique_gather", "no_overlap", "partitioned"}
 # (dim, nodes per element) with a mixed-precision plastic-correction kernel (CUDA-core warp kernel
 # for the triangles and P1/P2 tets, tcgen05 tensor-core kernel for P4 tets)
-# points from which stress-only evaluations screen first and decide a dense list (two launches and a memset
-# more; one pass below, where a launch costs more than the eigen-decompositions it saves)
-SCREENED_STRESS_POINTS = 16384
-# CSR values from which their starting values are staged on a second stream: its events and stream switches
-# cost the host about 40 us a step, the rows of a smaller pattern less than that to copy in line
+# Points from which stress-only evaluations screen first and decide a dense list (two launches and a memset more;
+# one pass below, where a launch costs more than the eigen-decompositions it saves).  Evaluations in turn, one pass
+# against screened: 42 and 47 us at 26,730 points, 42 and 49 at 52,272, 52 and 48 at 118,272, 68 and 62 at 264,000.
+SCREENED_STRESS_POINTS = 98_304
+# CSR values from which their starting values are staged on a second stream: its events and stream switches cost the
+# host 30 to 50 us a step, the rows of a smaller pattern less than that to copy in line.  Device outputs, iterations in
+# turn, in line against staged: 166 and 177 us at 2.8 M values (P2 tetrahedra), 193 and 172 at 3.9 M (P4 triangles), 219
+# and 183 at 6.1 M, 527 and 490 at 33 M; one iteration at a time they are equal from 6 to 16 M.  With host outputs the
+# copy to the host bounds the step, and in line stays ahead (401 and 436 at 6.1 M) up to some 20 M.
 STAGED_NNZ = 4_000_000
-# CSR values below which the host mirror is refreshed in full on the current stream (2 MB: 12 us of the link)
+# CSR values below which the host mirror is refreshed in full on the current stream: an iteration of 260 us against
+# 312 with the side stream at 0.27 M values (2 MB: 12 us of the link).  In line stays ahead up to 1.3 M (349 and
+# 355), but more than a tenth of the step is then a copy that the side stream would hide behind the force.
 IN_LINE_HOST_VALUES = 262_144
 MIXED_TANGENT_ELEMENTS = {(2, 3), (2, 6), (2, 15), (3, 4), (3, 10), (3, 35)}
 
