@@ -1,6 +1,6 @@
 // Strain and internal force of straight-sided P4 tetrahedra in fixed point (fixed.cuh): the sums of
 // strain3_affine_kernel and force3_affine_kernel (assembly.cu), whose FP64 form took 197 and 160 us on 10,374
-// elements at that pipe's rate (now 78 and 84).  Each is a product with the reference element's gradient table, the same for
+// elements at that pipe's rate (now 70 and 84).  Each is a product with the reference element's gradient table, the same for
 // every element (strain: 34 nodes x 9 products a point, force: 24 points x 9 a node), so a block converts the
 // table once, keeps it in shared memory and strides over groups of elements.  Products of values of 56 bits in limbs of
 // 28, the lower one signed: every sum exact.  What a thread does once a point, the products with
@@ -39,7 +39,7 @@ struct ElementUnits {
     int unit[3], finite;
 };
 
-__global__ void __launch_bounds__(kStrainThreads, 3) strain3_affine_fixed_kernel(
+__global__ void __launch_bounds__(kStrainThreads, 4) strain3_affine_fixed_kernel(
     const double *__restrict__ jinv, const double *__restrict__ ghat, const double *__restrict__ u,
     const int32_t *__restrict__ dof, long long n_u, int n_elem, int n_p, int n_q, int group, double *__restrict__ E) {
     extern __shared__ __align__(16) unsigned char raw[];

@@ -228,8 +228,8 @@ __device__ __forceinline__ void sym_matvec(const double *M, const double *v, dou
 // Both kernels: one thread per element, one warp per CTA, in 58-bit fixed point (fixed.cuh; an element has an
 // exponent for each displacement component, each column of J^{-1} and each stress component, so that small ones
 // beside large ones, or thin elements, keep the bits that they have in FP64).  In FP64 they were bound by that
-// pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 55 and 92, bound by the latency of 12 or
-// 13 warps an SM).  With one exponent for all components and columns and the force's last contraction in integers, too,
+// pipe (95 and 123 us on 100,800 elements, where the bytes take 11 and 12; now 53 and 92, bound by the latency of 13
+// warps an SM).  With one exponent for all components and columns and the force's last contraction in integers, too,
 // they took 54 and 80, and a strain or force 1e-8 of the others kept half of its digits.  E and the stresses pass
 // through shared memory, so that a warp's 32 elements are one contiguous block of global memory; elements
 // with an input that is not finite take the FP64 form of the same sums.
@@ -313,7 +313,7 @@ __device__ __forceinline__ void p2_lambda_table(const double *bary, int n_q, int
 
 // Strain.  bary is [n_q][4] (λ0..λ3 of each point).  With d_a = u_a - u_0 every A_im - A_0m is a sum of at
 // most nine d's, so the differences are taken first, exactly, and brought to 58 bits by their component's largest.
-__global__ void __launch_bounds__(32, 10) strain3_p2_affine_kernel(const double *__restrict__ jinv,
+__global__ void __launch_bounds__(32, 13) strain3_p2_affine_kernel(const double *__restrict__ jinv,
                                                                    const double *__restrict__ bary,
                                                                    const double *__restrict__ u,
                                                                    const int32_t *__restrict__ dof, long long n_u,
