@@ -50,8 +50,6 @@ except Exception:  # pragma: no cover
     PETSc = None
 
 _OWNED_MODES = {"overlap", "unique_exchange", "unique", "unique_gather", "no_overlap", "partitioned"}
-# (dim, nodes per element) with a mixed-precision plastic-correction kernel (CUDA-core warp kernel
-# for the triangles and P1/P2 tets, tcgen05 tensor-core kernel for P4 tets)
 # Points from which stress-only evaluations screen first and decide a dense list (two launches and a memset more;
 # one pass below, where a launch costs more than the eigen-decompositions it saves).  Evaluations in turn, one pass
 # against screened: 42 and 47 us at 26,730 points, 42 and 49 at 52,272, 52 and 48 at 118,272, 68 and 62 at 264,000.
@@ -66,6 +64,10 @@ STAGED_NNZ = 4_000_000
 # 312 with the side stream at 0.27 M values (2 MB: 12 us of the link).  In line stays ahead up to 1.3 M (349 and
 # 355), but more than a tenth of the step is then a copy that the side stream would hide behind the force.
 IN_LINE_HOST_VALUES = 262_144
+# (dim, nodes per element) whose element tangents are formed in fixed point (csrc/tangent_fixed.cu)
+FIXED_POINT_TANGENT_ELEMENTS = {(3, 10), (3, 35)}
+# (dim, nodes per element) with a mixed-precision plastic-correction kernel (CUDA-core warp kernel
+# for the triangles and P1/P2 tets, tcgen05 tensor-core kernel for P4 tets)
 MIXED_TANGENT_ELEMENTS = {(2, 3), (2, 6), (2, 15), (3, 4), (3, 10), (3, 35)}
 
 
@@ -291,7 +293,7 @@ class ConstitutiveOperator:
         # plain form on straight-sided P2 tetrahedra: elements with at least this many plastic points
         # get their correction in moment form (ssp_tangent_plastic_correction_p2_moments), the others
         # point by point (ssp_tangent_plastic_correction); 0 disables it.  100,800 tetrahedra, 27 thousand
-        # of them plastic: a Newton iteration takes 575 us with 2 or 3, 592 with 4, 598 with 5.  The mixed form's
+        # of them plastic: a Newton iteration takes 598 us with 2, 593 with 3, 606 with 4 or 5, 696 with 0.  The mixed form's
         # moment kernel (FP32 after the FP64 DS - D_el) costs less than its point-by-point kernel from
         # one plastic point up: every plastic element by default.
         self.moment_min_points = 3
@@ -981,9 +983,15 @@ class ConstitutiveOperator:
 
     def _bddc_predictor_ok(self, pattern) -> bool:
         """Whether the subdomain tangent may start from the pattern's elastic values: the subdomain's
-        DS rows come from this operator's own evaluation (symmetric, branch codes known) and the
-        pattern's elastic moduli are the operator's at the same points (checked once per pattern)."""
-        if self._branch is None or not self._ds_symmetric or self._DS_aos is None:
+        DS rows come from this operator's own evaluation (symmetric, branch codes known), the
+        pattern's elastic moduli are the operator's at the same points (checked once per pattern), and
+        the corrections are formed in fixed point (P2 and P4 tetrahedra).  A plastic element's elastic
+        part and its correction are both rounded; with FP64 corrections the matrix is then farther from exact
+        sums than the full contraction's (units of 1e-16, full and predictor: P1, P2 and P4 triangles 0.86 and
+        0.98, 1.10 and 1.20, 2.2 and 2.7, P1 tetrahedra 1.3 and 1.5), with fixed-point ones it is not (P2 1.2 and
+        1.2, P4 2.2 and 1.3, where the full contraction is FP64's)."""
+        if self._branch is None or not self._ds_symmetric or self._DS_aos is None or \
+                (pattern.dim, pattern.n_p) not in FIXED_POINT_TANGENT_ELEMENTS:
             return False
         if "predictor_ok" not in self._bddc:
             t = _lib.torch()

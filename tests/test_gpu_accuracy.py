@@ -233,3 +233,46 @@ def test_element_matrices_in_the_norm(cuda_device, et, kind, thin):
             _lib.call("ssp_tangent_element", 3, int(kind == "symmetric"), *(_lib.ptr(x) for x in geo), _lib.ptr(ds),
                       _lib.ptr(wd), _lib.ptr(emap), n_el, n_p, n_q, nnz, _lib.ptr(K), 0, st)
     assert _distance(K.cpu().numpy().reshape(want.shape), want) <= 3e-16
+
+
+@pytest.mark.parametrize("dim,et,dims", [(2, "P1", (40, 30)), (2, "P4", (12, 8)), (3, "P1", (8, 4, 5))])
+def test_bddc_matrix_of_fp64_elements(cuda_device, dim, et, dims):
+    """Elements whose tangents are FP64 sums: the subdomain matrix is as near the exact sums as the full contraction
+    of every point, whose reductions land in another order (up to a twentieth of the distance from run to run: a tenth)."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import ConstitutiveOperator, _lib, prepare_bddc_subdomain_pattern, synthetic
+    from slope_stability_petsc4py_gb300.bddc import bddc_tangent_values_device
+
+    mats = synthetic.MaterialSet.layered(4, seed=1)
+    mesh = (synthetic.slope_mesh_3d if dim == 3 else synthetic.slope_mesh_2d)(*dims, elem_type=et, n_layers=4)
+    specs = [dict(c0=float(mats.c0[i]), phi=float(mats.phi[i]), psi=float(mats.psi[i]), young=float(mats.young[i]),
+                  poisson=float(mats.poisson[i]), gamma_sat=20.0, gamma_unsat=20.0) for i in range(mats.c0.size)]
+    op = ConstitutiveOperator.from_mesh(mesh.coord, mesh.elem, mesh.q_mask, mesh.material_id, specs, elem_type=et)
+    op.host_outputs = False
+    op.set_bddc_subdomain_pattern(prepare_bddc_subdomain_pattern(
+        mesh.coord, mesh.elem, mesh.q_mask, mesh.material_id, specs, (0, mesh.n_nodes // 2), elem_type=et,
+        overlap_local_int_indices=op.owned_tangent_pattern.local_int_indices, adjacency_source="none"))
+    op.reduction(1.1)
+    op.constitutive_problem_stress_tangent(synthetic.displacement_field(mesh, mats, 0.004, seed=1))
+    K = op.build_bddc_tangent_matrix().values.cpu().numpy()
+    assert 0.02 < float((op._branch != 0).double().mean()) < 0.9
+    pat, ns = op.bddc_subdomain_pattern, 6 if dim == 3 else 3
+    n_q, n_p = pat.n_q, pat.n_p
+    rows = np.ascontiguousarray(np.asarray(op._owned_local_DS).T[pat.overlap_local_positions])
+    full = bddc_tangent_values_device(pat, torch.as_tensor(rows, device="cuda")).cpu().numpy()
+    DS = rows.reshape(-1, n_q, ns, ns).transpose(0, 1, 3, 2).astype(LD)
+    g = np.stack([np.asarray(x).reshape(-1, n_q, n_p) for x in (pat.dphi1, pat.dphi2, pat.dphi3)[:dim]], -1)
+    w = np.asarray(pat.local_assembly_weight).reshape(-1, n_q).astype(LD)
+    bt = BT if dim == 3 else ((0, 2), (2, 1))
+    want = np.zeros(pat.nnz, LD)
+    for e in range(g.shape[0]):
+        B = np.zeros((n_q, ns, dim * n_p), LD)
+        for c in range(dim):
+            for z in range(dim):
+                B[:, bt[c][z], c::dim] = g[e, :, :, z]
+        Ke = sum(B[q].T @ ((w[e, q] * DS[e, q]) @ B[q]) for q in range(n_q)).reshape(-1)
+        at = pat.scatter_map[e].reshape(-1)
+        np.add.at(want, at[at >= 0], Ke[at >= 0])
+    want[pat.constrained_diag_positions] = 1.0
+    assert _distance(K, want) <= 1.1 * _distance(full, want)
