@@ -58,8 +58,8 @@ SAMPLE_POINTS, SAMPLE_POINTS_1T = 4_000_000, 250_000
 # profiles/dram_traffic_3d_p2_large.md), keyed by workload and entry point; reported as roofline.traffic
 # with that source when the bench's dominant kernel is one of them
 NCU_TRAFFIC = {"3d_p2_large": {
-    "ssp_tangent_plastic_correction_p2_moments": (2994.5e6 + 1058.4e6,
-                                                  "ncu capture 2026-12-04, profiles/dram_traffic_3d_p2_large.md"),
+    "ssp_tangent_plastic_correction_p2_moments": (3562.2e6 + 1242.6e6,
+                                                  "ncu capture 2026-12-05, profiles/dram_traffic_3d_p2_large.md"),
     "ssp_tangent_plastic_correction_p2_moments_mixed": (4694.0e6 + 1440.7e6,
                                                         "ncu capture 2026-12-04, profiles/dram_traffic_3d_p2_large.md"),
 }}
@@ -588,7 +588,8 @@ def measure_graph_replay(torch, lib, op, states_dev, args):
 def measure_bddc(torch, lib, op, w, states_dev, args):
     """BDDC subdomain tangent (prepare_bddc_subdomain_pattern on the lower half of the node range),
     one regularised subdomain build per Newton iteration after the owned evaluation: elastic
-    predictor + plastic corrections (FP64 and mixed), and the full contraction of every point."""
+    predictor + plastic corrections (P2 and P4 tetrahedra; after either form's evaluation), and the full
+    contraction of every point."""
     from slope_stability_petsc4py_gb300 import prepare_bddc_subdomain_pattern
 
     mesh = w.mesh
