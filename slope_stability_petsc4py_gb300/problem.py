@@ -109,10 +109,12 @@ class OwnedCSRMatrix:
         stream's events and switches cost the host more than the copy takes."""
         t = _lib.torch()
         if self.values.numel() < IN_LINE_HOST_VALUES:
+            cur = t.cuda.current_stream()
             self._host.copy_(self.values, non_blocking=True)
             if self._copied is None:
                 self._copied = t.cuda.Event()
-            self._copied.record()
+            self._copied.record(cur)
+            self.values.record_stream(cur)  # not freed for another stream's use while the copy reads them
             self.mirror = mirror
             self._last_rows = None
             return self

@@ -75,3 +75,32 @@ def test_first_forces_of_two_operators_on_two_streams(cuda_device):
         assert float((f - want).abs().max() / want.abs().max()) <= 1e-14
     for k in K:
         assert float((k - K_want).abs().max() / K_want.abs().max()) <= 1e-14
+
+
+@pytest.mark.parametrize("dims", [(3, 2, 2), (8, 5, 7)])
+def test_host_copy_holds_the_values_on_its_stream(cuda_device, monkeypatch, dims):
+    """The CSR values stay allocated until their copy to the host has read them, whichever stream it runs on (few
+    values: the caller's, many: a side stream)."""
+    import torch
+
+    from slope_stability_petsc4py_gb300 import problem
+
+    _mesh, U, op, _sub = _slope(dims=dims)
+    few = op.owned_tangent_pattern.nnz < problem.IN_LINE_HOST_VALUES
+    assert few == (dims == (3, 2, 2))
+    _F, K = op.build_F_K_regularized_all_free(1.1, U, 0.1)
+    torch.cuda.synchronize()
+    seen, real = [], torch.Tensor.record_stream
+
+    def record(self, stream):
+        if self.data_ptr() == K.values.data_ptr():
+            seen.append(stream.cuda_stream)
+        return real(self, stream)
+
+    monkeypatch.setattr(torch.Tensor, "record_stream", record)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        K.sync_host()
+        assert seen == [s.cuda_stream if few else K._copy_stream.cuda_stream]
+        host = K.getValuesCSR()[2]
+    assert np.array_equal(host, K.values.cpu().numpy())
