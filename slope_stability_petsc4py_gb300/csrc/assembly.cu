@@ -843,7 +843,8 @@ __device__ __forceinline__ double elastic_d(int i, int j, double G, double lam) 
     return 0.0;
 }
 
-// One CTA per element (grid-stride).  K_e = sum_q B_q^T (w_q D_q) B_q is formed in two
+// One CTA (a warp) per element, grid-stride: P1 tetrahedra and P1, P2 triangles, whose entries are too few for
+// more.  K_e = sum_q B_q^T (w_q D_q) B_q is formed in two
 // stages per quadrature point through shared memory:
 //   H[alpha][m] = (B^T (w D))[alpha][m]      (n_ld x n_s, split over the CTA)
 //   K[alpha][beta] += sum_m H[alpha][m] B[m][beta]   (each thread owns fixed entries in registers)
@@ -856,7 +857,7 @@ __device__ __forceinline__ double elastic_d(int i, int j, double G, double lam) 
 // full tangent with the FP64 work of the plastic points only: for an elastic point DS_q equals
 // D_el,q exactly, so its term vanishes.
 template <int DIM, int NP, int NQ, int THREADS, bool SYM, bool CORR>
-__global__ void __launch_bounds__(THREADS, SYM ? 2 : 1) tangent_element_kernel(ElemArgs A) {
+__global__ void __launch_bounds__(THREADS) tangent_element_kernel(ElemArgs A) {
     constexpr int NS = DIM == 3 ? 6 : 3;
     constexpr int NLD = DIM * NP;
     constexpr int NENT = SYM ? NLD * (NLD + 1) / 2 : NLD * NLD;
@@ -866,8 +867,7 @@ __global__ void __launch_bounds__(THREADS, SYM ? 2 : 1) tangent_element_kernel(E
     __shared__ double sD[NQ][NS * NS];
     __shared__ double sH[NLD * NS];
     // SYM: entry id -> alpha | beta << 8 of the row-major upper triangle, 0xFFFF past the last entry
-    // (in shared memory rather than registers, so two CTAs fit an SM); the full matrix decodes
-    // id = alpha NLD + beta directly
+    // (decoded once a CTA); the full matrix decodes id = alpha NLD + beta directly
     __shared__ uint16_t scode[SYM ? PER * THREADS : 1];
     __shared__ int sq[NQ];
     __shared__ int snq;
@@ -1027,8 +1027,8 @@ template <int DIM, int NP, int NQ, int WARPS, bool SYM, bool CORR, bool MIXED>
 __global__ void __launch_bounds__(32 * WARPS, MIXED ? 5 : 4) tangent_element_warp_kernel(ElemArgs A) {
     constexpr int NS = DIM == 3 ? 6 : 3;
     constexpr int NLD = DIM * NP;
-    // FP64 form (bound by the FP64 pipe): each lane owns PER scattered entries of K_e, which keeps
-    // 97 % of the lanes' FP64 slots busy.  Mixed form (bound by issue): each lane owns whole
+    // FP64 form (P4 triangles; bound by the FP64 pipe): each lane owns PER scattered entries of K_e, which
+    // keeps 97 % of the lanes' FP64 slots busy.  Mixed form (bound by issue): each lane owns whole
     // node-pair blocks (a, b) of DIM x DIM entries (a <= b when SYM), so it reads one row of H per
     // block row and one gradient per direction and reuses them across the block's entries.
     constexpr int NENT = SYM ? NLD * (NLD + 1) / 2 : NLD * NLD;

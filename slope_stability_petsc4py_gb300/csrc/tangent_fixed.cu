@@ -19,8 +19,8 @@
 //   3. K[(a,c),(b,d)] = sum_q sum_r g_a,r H[q][b][d][row(c, r)]; 36 terms at most: limbs of 28 bits, the lower
 //      one signed, so that the dropped products have no bias and both accumulators stay below 2^63
 //   4. the sums, at 57 bits or so, become FP64 and are reduced into the CSR values
-// The entries are nearer the exact sums than FP64's (measured over distorted elements in the 2-norm: P2 0.8e-16 to
-// 1.0e-16 against 1.6e-16 to 2.6e-16, P4 1.1e-16 to 1.2e-16 against 2.8e-16 to 3.4e-16).  P4's nodes differ by an
+// Element matrices are nearer the exact sums than FP64's, in the norm (over distorted elements P2 0.8e-16 to
+// 1.3e-16 against 1.6e-16 to 3.6e-16, P4 1.0e-16 to 1.1e-16 against 2.4e-16 to 3.0e-16).  P4's nodes differ by an
 // order of magnitude in their gradients; with one exponent for all of an element's its tangent was at 4.0e-16.
 // An element whose inputs are not all finite takes the same sums in FP64.
 #include "fixed.cuh"
